@@ -57,7 +57,9 @@ struct SrcPair {
 // limbs below ncm come from the inputs, the others from the extension. The
 // products are Montgomery reductions (value * 2^-64 mod q_j, in [0, 2q_j));
 // the inverse NTT that consumes them scales by N^-1 * 2^64 instead of N^-1,
-// so its output is the canonical INTT of the exact products.
+// so its output is the canonical INTT of the exact products. FOLD kernels take
+// plain products instead, folded at 2^k: seven wide multiplies against nine
+// and two narrow ones.
 struct SrcTensor {
   static constexpr bool kMontgomery = true;
   static constexpr bool kStaged = true;
@@ -72,6 +74,12 @@ struct SrcTensor {
   __device__ __forceinline__ uint64_t op(uint32_t b, uint32_t w, uint32_t limb, uint32_t i) const {
     return row(b, w, limb)[i];
   }
+  // A product (or the sum of two), reduced for the transform that takes it.
+  template <bool FOLD>
+  __device__ __forceinline__ static uint64_t reduced(uint64_t hi, uint64_t lo, const DevPrime& pr) {
+    if constexpr (FOLD) return fold_wide_product(hi, lo, pr);
+    else return mont_reduce(hi, lo, pr);
+  }
   // Staged load for the inverse NTT (k_ntt_inv): the operand rows stream
   // into shared memory with asynchronous copies, so every load of the phase
   // is in flight at once instead of what the registers can hold. A square
@@ -79,7 +87,7 @@ struct SrcTensor {
   // the cross term (l0 r1 + l1 r0) a quarter block of its four, so that its
   // two products are summed exactly (below 2 q_j^2 < q_j 2^64) and reduced
   // once, as the unstaged path does.
-  template <int LOGN, int T, int E>
+  template <int LOGN, int T, int E, bool FOLD>
   __device__ __forceinline__ void stage(const NttJob& j, const DevPrime& pr, uint32_t base, uint64_t* sm,
                                         uint32_t tid, uint64_t* x) const {
     constexpr uint32_t HALF = 1u << (LOGN - 1), QTR = HALF / 2;
@@ -99,7 +107,7 @@ struct SrcTensor {
         for (int e = 0; e < E / 2; e++) {
           const uint32_t idx = tid + e * T;
           const uint64_t u = sm[idx], v = sm[HALF + idx];
-          x[h * (E / 2) + e] = mont_reduce(__umul64hi(u, v), u * v, pr);
+          x[h * (E / 2) + e] = reduced<FOLD>(__umul64hi(u, v), u * v, pr);
         }
         __syncthreads();
       }
@@ -125,7 +133,7 @@ struct SrcTensor {
         uint64_t hi = 0, lo = 0;
         mac128(hi, lo, sm[idx], sm[QTR + idx]);
         mac128(hi, lo, sm[2 * QTR + idx], sm[3 * QTR + idx]);
-        x[qt * (E / 4) + e] = mont_reduce(hi, lo, pr);
+        x[qt * (E / 4) + e] = reduced<FOLD>(hi, lo, pr);
       }
       __syncthreads();
     }
@@ -141,11 +149,12 @@ struct SrcTensor {
       prefetch_l2(row(b, 3, j.limb) + i);
     }
   }
-  __device__ __forceinline__ uint64_t operator()(const NttJob& j, const DevPrime& pr, uint32_t i) const {
+  template <bool FOLD>
+  __device__ __forceinline__ uint64_t product(const NttJob& j, const DevPrime& pr, uint32_t i) const {
     const uint32_t b = j.poly / 3, part = j.poly % 3;
     if (part != 1) {
       const uint64_t x = op(b, part >> 1, j.limb, i), y = op(b, 2 + (part >> 1), j.limb, i);
-      return mont_reduce(__umul64hi(x, y), x * y, pr);
+      return reduced<FOLD>(__umul64hi(x, y), x * y, pr);
     }
     const uint64_t a0 = op(b, 0, j.limb, i), a1 = op(b, 1, j.limb, i);
     const uint64_t b0 = op(b, 2, j.limb, i), b1 = op(b, 3, j.limb, i);
@@ -153,7 +162,7 @@ struct SrcTensor {
     uint64_t hi = 0, lo = 0;
     mac128(hi, lo, a0, b1);
     mac128(hi, lo, a1, b0);
-    return mont_reduce(hi, lo, pr);
+    return reduced<FOLD>(hi, lo, pr);
   }
 };
 
@@ -161,7 +170,8 @@ struct SrcTensor {
 struct SrcPolyMont {
   static constexpr bool kMontgomery = true;
   PolyRef r;
-  __device__ __forceinline__ uint64_t operator()(const NttJob& j, const DevPrime&, uint32_t i) const {
+  template <bool FOLD>
+  __device__ __forceinline__ uint64_t product(const NttJob& j, const DevPrime&, uint32_t i) const {
     return r.at(j.poly, j.limb)[i];
   }
   __device__ __forceinline__ void prefetch(const NttJob& j, uint32_t i) const { prefetch_l2(r.at(j.poly, j.limb) + i); }
@@ -169,6 +179,7 @@ struct SrcPolyMont {
 
 // The tensor products of SrcTensor as an element-wise kernel: one thread per
 // (product polynomial, limb, coefficient).
+template <bool FOLD>
 __global__ void k_tensor(const DevPrime* primes, SrcTensor t, PolyRef out, uint32_t limbs, uint32_t logn,
                          uint64_t total) {
   const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -181,7 +192,7 @@ __global__ void k_tensor(const DevPrime* primes, SrcTensor t, PolyRef out, uint3
   j.beta = 0;
   j.aux = 0;
   const DevPrime pr = primes[j.limb];
-  out.at(j.poly, j.limb)[i] = t(j, pr, i);
+  out.at(j.poly, j.limb)[i] = t.product<FOLD>(j, pr, i);
 }
 
 // Digit i of c2 (power basis, mod q_i) lazily reduced modulo key limb j
@@ -190,12 +201,16 @@ __global__ void k_tensor(const DevPrime* primes, SrcTensor t, PolyRef out, uint3
 // lies in the forward NTT's input range [0, 4 q_j) and needs no reduction
 // (the transform is the same modulo q_j).
 struct SrcDigit {
+  static constexpr bool kAnyWord = true;
   PolyRef digits;  // poly b * ndig + i -> row (b, i): stored as poly b, limb i
   uint32_t ndig;
   uint32_t raw;
-  __device__ __forceinline__ uint64_t operator()(const NttJob& j, const DevPrime& pr, uint32_t i) const {
+  __device__ __forceinline__ uint64_t word(const NttJob& j, const DevPrime&, uint32_t i) const {
     const uint32_t b = j.poly / ndig, d = j.poly % ndig;
-    const uint64_t x = digits.at(b, d)[i];
+    return digits.at(b, d)[i];
+  }
+  __device__ __forceinline__ uint64_t operator()(const NttJob& j, const DevPrime& pr, uint32_t i) const {
+    const uint64_t x = word(j, pr, i);
     return raw ? x : reduce64_lazy(x, pr);
   }
 
@@ -208,12 +223,15 @@ struct SrcDigit {
 // row (key_switching_key.rs:300-314), lazily reduced into the key modulus
 // (rq/mod.rs:525-528): polynomial b * nd + d reads row b.
 struct SrcDecompDigit {
+  static constexpr bool kAnyWord = true;
   PolyRef rows;  // poly b, limb 0
   uint32_t nd, log_base;
-  __device__ __forceinline__ uint64_t operator()(const NttJob& j, const DevPrime& pr, uint32_t i) const {
+  __device__ __forceinline__ uint64_t word(const NttJob& j, const DevPrime&, uint32_t i) const {
     const uint32_t b = j.poly / nd, d = j.poly % nd;
-    const uint64_t x = (rows.at(b, 0)[i] >> (d * log_base)) & ((1ull << log_base) - 1);
-    return reduce64_lazy(x, pr);
+    return (rows.at(b, 0)[i] >> (d * log_base)) & ((1ull << log_base) - 1);
+  }
+  __device__ __forceinline__ uint64_t operator()(const NttJob& j, const DevPrime& pr, uint32_t i) const {
+    return reduce64_lazy(word(j, pr, i), pr);
   }
   __device__ __forceinline__ void prefetch(const NttJob& j, uint32_t i) const {
     prefetch_l2(rows.at(j.poly / nd, 0) + i);
@@ -255,7 +273,7 @@ struct SrcSubst {
   __device__ __forceinline__ uint64_t operator()(const NttJob& j, const DevPrime&, uint32_t i) const {
     return in.at(j.poly, j.limb)[gather_index(i, e, logn)];
   }
-  template <int LOGN, int T, int E>
+  template <int LOGN, int T, int E, bool FOLD>
   __device__ __forceinline__ void stage(const NttJob& j, const DevPrime&, uint32_t base, uint64_t* sm, uint32_t tid,
                                         uint64_t* x) const {
     stage_gather<LOGN, T, E>(in.at(j.poly, j.limb), e, logn, base, sm, tid, x);
@@ -268,9 +286,14 @@ struct SrcSubst {
 // (digit d of ciphertext b is polynomial b*L + d, lazily reduced into key
 // limb j), polynomials [B*L, B*L + 2B) are c0 and c1 of each product.
 struct SrcKsF {
+  static constexpr bool kAnyWord = true;
   PolyRef digits;  // c2 rows: poly b, limb d
   PolyRef c01;     // c0 / c1: poly 2b + part
   uint32_t ndig, ndig_polys;
+  __device__ __forceinline__ uint64_t word(const NttJob& j, const DevPrime&, uint32_t i) const {
+    if (j.poly < ndig_polys) return digits.at(j.poly / ndig, j.poly % ndig)[i];
+    return c01.at(j.poly - ndig_polys, j.limb)[i];
+  }
   __device__ __forceinline__ uint64_t operator()(const NttJob& j, const DevPrime& pr, uint32_t i) const {
     if (j.poly < ndig_polys) return reduce64_lazy(digits.at(j.poly / ndig, j.poly % ndig)[i], pr);
     return c01.at(j.poly - ndig_polys, j.limb)[i];
@@ -570,7 +593,7 @@ void ntt_forward_into(uint32_t logn, NttGeom g, uint64_t polys, PolyRef inplace,
   if (bl == 12 && ntt_cluster_enabled(logn) &&
       launch_fwd_cluster<12, true>(g, logn - bl, polys, SrcPoly{inplace}, dst, st))
     return;
-  launch_fwd_top(logn - bl, g, bl, polys, SrcPoly{inplace}, DstPoly{inplace}, st);
+  launch_fwd_top<true>(logn - bl, g, bl, polys, SrcPoly{inplace}, DstPoly{inplace}, st);
   ntt_forward_after_top<true>(logn, g, polys, DstPoly{inplace}, dst, st, bl);
 }
 
@@ -587,7 +610,7 @@ static void finish_switch_down(const Ksk& k, uint64_t* ks, uint64_t* sd, uint64_
   PolyRef sdref = plain_ref(sd, cc.L(), logn);
   ntt_backward(kc, ksref, ksref, 2 * batch, st);
   switch_down_chain(k, ksref, sdref, 2 * batch, st);
-  NttGeom g{cc.primes_dev(), (uint32_t)cc.L(), 0};
+  const NttGeom g = ntt_geom(cc);
   DstAddParts dst{out, out_poly_stride, add0, add0_poly_stride, add0_exponent, add1, add1_poly_stride,
                   (uint32_t)cc.L(), logn};
   ntt_forward_into(logn, g, 2 * batch, sdref, dst, st);
@@ -610,7 +633,7 @@ void key_switch(const Ksk& k, PolyRef digits, uint64_t batch, const uint64_t* ad
   const size_t Lk = kc.L(), nd = k.count, N = kc.N();
   const uint32_t logn = kc.logn;
   PolyRef dref = plain_ref(D, Lk, logn);
-  NttGeom g{kc.primes_dev(), (uint32_t)Lk, 0};
+  const NttGeom g = ntt_geom(kc);
   // Every digit in every key modulus (rq/mod.rs:518-540), reduced output.
   if (k.log_base)
     ntt_forward_any<true>(logn, g, batch * nd, SrcDecompDigit{digits, (uint32_t)nd, k.log_base}, DstPoly{dref}, st);
@@ -680,7 +703,7 @@ void galois_relinearize(const Ksk& gk, uint64_t exponent, const uint64_t* ct, ui
   // substitution is a gather fused into the inverse NTT.
   PolyRef src = sub_ref(const_cast<uint64_t*>(ct), L, c.logn, 2, 1, 1);
   PolyRef dst = plain_ref(digits, L, c.logn);
-  NttGeom g{c.primes_dev(), (uint32_t)L, 0};
+  const NttGeom g = ntt_geom(c);
   ntt_inverse_any(c.logn, g, count, SrcSubst{src, e, c.logn}, DstPoly{dst}, st);
   // galois_key.rs:111-122: key switch, then out0 += substitute(ct[0]).
   key_switch(gk, dst, count, ct, 2 * L * N, e, nullptr, 0, out, 2 * L * N, D, st);
@@ -744,7 +767,7 @@ struct SrcRotSubst {
     const RotDesc& r = d[j.poly];
     return r.ct[((uint64_t)(r.L + j.limb) << logn) + gather_index(i, r.e, logn)];
   }
-  template <int LOGN, int T, int E>
+  template <int LOGN, int T, int E, bool FOLD>
   __device__ __forceinline__ void stage(const NttJob& j, const DevPrime&, uint32_t base, uint64_t* sm, uint32_t tid,
                                         uint64_t* x) const {
     const RotDesc& r = d[j.poly];
@@ -769,13 +792,16 @@ struct DstRotDigits {
 
 // F: digit `aux` of ciphertext `poly` in key limb `limb`.
 struct SrcRotDigit {
+  static constexpr bool kAnyWord = true;
   const RotDesc* d;
   uint32_t logn;
-  __device__ __forceinline__ uint64_t operator()(const NttJob& j, const DevPrime& pr, uint32_t i) const {
+  __device__ __forceinline__ uint64_t word(const NttJob& j, const DevPrime&, uint32_t i) const {
     const RotDesc& r = d[j.poly];
-    if (r.log_base)
-      return reduce64_lazy((r.digits[i] >> (j.aux * r.log_base)) & ((1ull << r.log_base) - 1), pr);
-    return reduce64_lazy(r.digits[((uint64_t)j.aux << logn) + i], pr);
+    if (r.log_base) return (r.digits[i] >> (j.aux * r.log_base)) & ((1ull << r.log_base) - 1);
+    return r.digits[((uint64_t)j.aux << logn) + i];
+  }
+  __device__ __forceinline__ uint64_t operator()(const NttJob& j, const DevPrime& pr, uint32_t i) const {
+    return reduce64_lazy(word(j, pr, i), pr);
   }
   __device__ __forceinline__ void prefetch(const NttJob& j, uint32_t i) const {
     prefetch_l2(d[j.poly].digits + ((uint64_t)j.aux << logn) + i);
@@ -1055,10 +1081,10 @@ static void launch_rot_batch(const RotBatchPlan& pl, cudaStream_t st) {
   const uint4* d_jobs = pl.d_jobs;
   const uint2* d_rows = pl.d_rows;
   // R1: substituted c1 into the power basis.
-  NttGeom g1{top.primes_dev(), 1, 0, d_jobs};
+  const NttGeom g1 = ntt_geom(top, d_jobs);
   ntt_inverse_any(logn, g1, cnt.n_r1, SrcRotSubst{d_desc, logn}, DstRotDigits{d_desc, logn}, st);
   // F: every digit in every key limb.
-  NttGeom g2{top.primes_dev(), 1, 0, d_jobs + cnt.n_r1};
+  const NttGeom g2 = ntt_geom(top, d_jobs + cnt.n_r1);
   ntt_forward_any<true>(logn, g2, cnt.n_f, SrcRotDigit{d_desc, logn}, DstRotD{d_desc, logn}, st);
   // G: inner products and the substituted c0.
   const unsigned gx = (unsigned)((N + 255) / 256);
@@ -1067,7 +1093,7 @@ static void launch_rot_batch(const RotBatchPlan& pl, cudaStream_t st) {
   if (cnt.n_chain == 0) return;
   // Requests with keys below their level: the sums into the power basis, down
   // to the ciphertext context, back to Ntt, plus the substituted c0.
-  NttGeom g3{top.primes_dev(), 1, 0, d_jobs + cnt.n_r1 + cnt.n_f};
+  const NttGeom g3 = ntt_geom(top, d_jobs + cnt.n_r1 + cnt.n_f);
   ntt_inverse_any(logn, g3, cnt.n_inv, RotKs{d_desc, logn}, RotKs{d_desc, logn}, st);
   const uint2* d_chain = d_rows + cnt.n_rows;
   const dim3 gc(gx, (unsigned)cnt.n_chain);
@@ -1075,7 +1101,7 @@ static void launch_rot_batch(const RotBatchPlan& pl, cudaStream_t st) {
   else if (cnt.max_lk <= 16) k_rot_chain<16><<<gc, 256, 0, st>>>(top.primes_dev(), d_desc, d_chain, logn);
   else k_rot_chain<32><<<gc, 256, 0, st>>>(top.primes_dev(), d_desc, d_chain, logn);
   after_launch("k_rot_chain");
-  NttGeom g4{top.primes_dev(), 1, 0, d_jobs + cnt.n_r1 + cnt.n_f + cnt.n_inv};
+  const NttGeom g4 = ntt_geom(top, d_jobs + cnt.n_r1 + cnt.n_f + cnt.n_inv);
   ntt_forward_any<true>(logn, g4, cnt.n_fwd, RotSd{d_desc, logn}, RotSd{d_desc, logn}, st);
   k_rot_add<<<dim3(gx, (unsigned)cnt.n_add), 256, 0, st>>>(top.primes_dev(), d_desc, d_chain + cnt.n_chain, logn);
   after_launch("k_rot_add");
@@ -1226,16 +1252,26 @@ void Multiplicator::multiply(const uint64_t* lhs, const uint64_t* rhs, uint64_t*
     return s1;
   };
 
+  // One arithmetic for every transform (the scaler kernels pass lazy values
+  // from one to the next): the fold form when every modulus involved has it.
+  const bool fold = mc.fold && bc.fold && (!rk || rk->ctx_ksk->fold);
+  auto geom = [&](const Context& c, size_t first, size_t limbs) {
+    NttGeom g = ntt_geom(c, first, limbs);
+    g.fold = fold;
+    return g;
+  };
+  const uint32_t bl_a = plan_a ? plan_a : ntt_block_logn(logn), bl_d = plan_d ? plan_d : ntt_block_logn(logn);
+
   // A: inverse NTT of the four operands (without its strided last stages
   // when B applies them).
   mark(0);
   const uint32_t top_a = top_stages(plan_a, *ext_lhs, ext_rhs.get(), (uint32_t)(M - std::min(ncm_l, ncm_r)));
   {
-    NttGeom g{bc.primes_dev(), (uint32_t)L, 0};
+    const NttGeom g = geom(bc, 0, L);
     if (top_a) ntt_inverse_blocks(logn, g, 4 * count, SrcPair{lref, rref}, DstPoly{pbref}, st, plan_a);
     else ntt_inverse_any(logn, g, 4 * count, SrcPair{lref, rref}, DstPoly{pbref}, st, plan_a);
   }
-  const InverseTop top_a_args{top_a, 0u, bc.primes_dev()};
+  const InverseTop top_a_args{top_a, 0u, bc.primes_dev(), fold && bl_a == 12};
   mark(1);
   // B + C: extension of each operand and forward NTT of the new limbs.
   const bool same_ext = ncm_l == ncm_r && ext_lhs->num == ext_rhs->num && ext_lhs->den == ext_rhs->den;
@@ -1252,7 +1288,7 @@ void Multiplicator::multiply(const uint64_t* lhs, const uint64_t* rhs, uint64_t*
     rns_scale(*s.rns, logn, in, o, (uint32_t)ncm, (uint32_t)(M - ncm), count * take, st,
               top_a ? &top_a_args : nullptr, fuse_c ? &fwd : nullptr);
     if (first == 0) mark(2);
-    NttGeom g{mc.primes_dev() + ncm, (uint32_t)(M - ncm), 0};
+    const NttGeom g = geom(mc, ncm, M - ncm);
     if (fuse_c) ntt_forward_after_top<true>(logn, g, count * take, DstPoly{o}, st, plan_c);
     else ntt_forward_any<true>(logn, g, count * take, SrcPoly{o}, DstPoly{o}, st, plan_c);
   };
@@ -1270,11 +1306,12 @@ void Multiplicator::multiply(const uint64_t* lhs, const uint64_t* rhs, uint64_t*
   PolyRef prodref = plain_ref(prod, M, logn);
   const uint32_t top_d = top_stages(plan_d, *down, nullptr, (uint32_t)L);
   {
-    NttGeom g{mc.primes_dev(), (uint32_t)M, 0};
+    const NttGeom g = geom(mc, 0, M);
     const SrcTensor tensor{lref, rref, extref, (uint32_t)ncm_l, (uint32_t)ncm_r};
     if (tensor_split) {
       const uint64_t total = 3 * count * M << logn;
-      k_tensor<<<nblocks(total, 256), 256, 0, st>>>(mc.primes_dev(), tensor, prodref, (uint32_t)M, logn, total);
+      auto kern = ntt_folds(g, logn, bl_d) ? k_tensor<true> : k_tensor<false>;
+      kern<<<nblocks(total, 256), 256, 0, st>>>(mc.primes_dev(), tensor, prodref, (uint32_t)M, logn, total);
       after_launch("k_tensor");
       if (top_d) ntt_inverse_blocks(logn, g, 3 * count, SrcPolyMont{prodref}, DstPoly{prodref}, st, plan_d);
       else ntt_inverse_any(logn, g, 3 * count, SrcPolyMont{prodref}, DstPoly{prodref}, st, plan_d);
@@ -1288,7 +1325,7 @@ void Multiplicator::multiply(const uint64_t* lhs, const uint64_t* rhs, uint64_t*
   // E: scale down by t/Q into the base context (power basis), applying the
   // strided last stages of D's inverse NTT (Montgomery products) on the way.
   PolyRef dnref = plain_ref(dn, L, logn);
-  const InverseTop top_d_args{top_d, 1u, mc.primes_dev()};
+  const InverseTop top_d_args{top_d, 1u, mc.primes_dev(), fold && bl_d == 12};
   // F's strided first stages run in E's epilogue when F's plan has as many as
   // D's: c0 and c1 get them over their own limbs (left in dn for F's block
   // pass), and c2 is expanded there into the digit rows of every key modulus
@@ -1307,14 +1344,14 @@ void Multiplicator::multiply(const uint64_t* lhs, const uint64_t* rhs, uint64_t*
   rns_scale(*down->rns, logn, prodref, dnref, 0, (uint32_t)L, 3 * count, st, top_d ? &top_d_args : nullptr,
             fuse_f ? &fwd_e : nullptr);
   mark(5);
-  NttGeom gb{bc.primes_dev(), (uint32_t)L, 0};
+  const NttGeom gb = geom(bc, 0, L);
   if (rk) {
     const Context& kc = *rk->ctx_ksk;
     PolyRef dref = plain_ref(D, Lk, logn);
     PolyRef c2 = sub_ref(dn, L, logn, 3, 2, 1);
     PolyRef c01 = sub_ref(dn, L, logn, 3, 0, 2);
     PolyRef oref = plain_ref(dest, L, logn);
-    NttGeom gk{kc.primes_dev(), (uint32_t)Lk, 0};
+    const NttGeom gk = geom(kc, 0, Lk);
     if (ks_decomp) {
       // mul.rs:196-210 with key_switching_key.rs:292-329: c0, c1 into Ntt;
       // G below adds the decomposed key switch of c2.

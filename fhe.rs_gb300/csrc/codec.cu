@@ -46,21 +46,29 @@ std::vector<uint32_t> index_map(size_t n) {
 // element i is values[map[i]] (the SIMD scatter v[map[k]] = values[k] read
 // through the inverse map).
 struct SrcValues {
+  static constexpr bool kAnyWord = true;
   const uint64_t* values;  // [count][N]
   const uint32_t* map;     // null: identity
   uint32_t logn;
-  __device__ __forceinline__ uint64_t operator()(const NttJob& j, const DevPrime&, uint32_t i) const {
+  __device__ __forceinline__ uint64_t word(const NttJob& j, const DevPrime&, uint32_t i) const {
     return values[((uint64_t)j.poly << logn) + (map ? map[i] : i)];
+  }
+  __device__ __forceinline__ uint64_t operator()(const NttJob& j, const DevPrime& pr, uint32_t i) const {
+    return word(j, pr, i);
   }
 };
 
 // Power-basis values v < t (one row per polynomial) lifted into every limb
 // of the ciphertext context: v mod q_j, lazily reduced ([0, 2 q_j)).
 struct SrcLift {
+  static constexpr bool kAnyWord = true;
   const uint64_t* v;  // [count][N]
   uint32_t logn;
+  __device__ __forceinline__ uint64_t word(const NttJob& j, const DevPrime&, uint32_t i) const {
+    return v[((uint64_t)j.poly << logn) + i];
+  }
   __device__ __forceinline__ uint64_t operator()(const NttJob& j, const DevPrime& pr, uint32_t i) const {
-    return reduce64_lazy(v[((uint64_t)j.poly << logn) + i], pr);
+    return reduce64_lazy(word(j, pr, i), pr);
   }
 };
 
@@ -224,11 +232,11 @@ void plaintext_encode(const Params& par, size_t level, const uint64_t* values, b
     size_t off = 0;
     uint64_t* tmp = ws.take(count * c.N(), &off);
     const uint32_t* inv = static_cast<const uint32_t*>(ps.maps.ptr) + c.N();
-    NttGeom gt{ps.tctx->primes_dev(), 1, 0};
+    const NttGeom gt = ntt_geom(*ps.tctx);
     ntt_inverse_any(logn, gt, count, SrcValues{values, inv, logn}, DstPoly{plain_ref(tmp, 1, logn)}, st);
     v = tmp;
   }
-  NttGeom g{c.primes_dev(), (uint32_t)c.L(), 0};
+  const NttGeom g = ntt_geom(c);
   ntt_forward_any<true>(logn, g, count, SrcLift{v, logn}, DstPoly{plain_ref(pt_ntt, c.L(), logn)}, st);
 }
 
@@ -271,11 +279,11 @@ void encrypt(const SecretKeyDev& sk, size_t level, const uint64_t* values, bool 
   if (simd) {
     if (!ps.tctx) throw Error(FHEG_ERR_UNSUPPORTED, "the plaintext modulus does not support SIMD encoding");
     const uint32_t* inv = static_cast<const uint32_t*>(ps.maps.ptr) + c.N();
-    NttGeom gt{ps.tctx->primes_dev(), 1, 0};
+    const NttGeom gt = ntt_geom(*ps.tctx);
     ntt_inverse_any(logn, gt, count, SrcValues{values, inv, logn}, DstPoly{plain_ref(vbuf, 1, logn)}, st);
     v = vbuf;
   }
-  NttGeom g{c.primes_dev(), (uint32_t)L, 0};
+  const NttGeom g = ntt_geom(c);
   ntt_forward_any<true>(logn, g, count,
                         SrcEncrypt{e, v, reinterpret_cast<const ulonglong2*>(dbuf), t, q_mod_t, logn},
                         DstPoly{sub_ref(out, L, logn, 2, 0, 1)}, st);
@@ -304,7 +312,7 @@ void decrypt(const SecretKeyDev& sk, size_t level, size_t parts, const uint64_t*
   uint64_t* pb = ws.take(count * c.L() * c.N(), &off);
   uint64_t* d0 = ws.take(count * c.N(), &off);
   // Phase into the power basis.
-  NttGeom g{c.primes_dev(), (uint32_t)c.L(), 0};
+  const NttGeom g = ntt_geom(c);
   ntt_inverse_any(logn, g, count,
                   SrcPhase{plain_ref(const_cast<uint64_t*>(ct), c.L(), logn), sk.s_ntt.u64(), (uint32_t)parts, logn},
                   DstPoly{plain_ref(pb, c.L(), logn)}, st);
@@ -319,7 +327,7 @@ void decrypt(const SecretKeyDev& sk, size_t level, size_t parts, const uint64_t*
     return;
   }
   const uint32_t* inv = static_cast<const uint32_t*>(ps.maps.ptr) + c.N();
-  NttGeom gt{ps.tctx->primes_dev(), 1, 0};
+  const NttGeom gt = ntt_geom(*ps.tctx);
   ntt_forward_any<true>(logn, gt, count, fin, DstSlots{values, inv, logn}, st);
 }
 

@@ -36,7 +36,22 @@ struct DevPrime {
   // omegas_shoup[i]), itw[i] = (zetas_inv[i], zetas_inv_shoup[i]).
   const ulonglong2* tw;
   const ulonglong2* itw;
+  // Primes just below a power of two, p = 2^k - f_c (40 <= k <= 62, see
+  // fold_params): the same tables as pairs of 32-bit digits for fold_mul
+  // (ftw[i] of omegas[i], fitw[i] of zetas_inv[i]), the constants of the
+  // transforms in that form, f_sh = k - 32 and f_bias, a multiple of p above
+  // every magnitude fold_canon meets. f_c = 0 for any other prime.
+  const int4* ftw;
+  const int4* fitw;
+  int4 f_ninv, f_zlast;  // N^-1 and zetas_inv[N - 2] * N^-1
+  uint64_t f_bias;
+  int32_t f_c, f_sh;
 };
+
+// p = 2^k - c with c below 2^28 and 2^(k - 17), 40 <= k <= 62: every prime that
+// generate_prime finds below 2^k for k >= 43 or so. Sets *c, *k and *bias (a
+// multiple of p, see DevPrime::f_bias) and returns true, else false.
+bool fold_params(uint64_t p, int32_t* c, int32_t* k, uint64_t* bias);
 
 // Counts every kernel launch issued by the library (reported by benchmarks).
 extern std::atomic<uint64_t> g_launches;
@@ -329,6 +344,128 @@ __device__ __forceinline__ void inv_bfly_final(uint64_t& x, uint64_t& y, uint64_
   const uint64_t t = x;
   x = mul_shoup(x + y, s, s_shoup, p);
   y = mul_shoup(t + p2 - y, zs, zs_shoup, p);
+}
+
+// ---------------------------------------------------------------------------
+// Arithmetic for primes p = 2^k - c just below a power of two (DevPrime::f_c).
+//
+// A product by a table constant w is T = a0 W0 + a1 W1 with a = a1 2^32 + a0
+// (32-bit signed digits) and W0 = w, W1 = w 2^32 mod p, both in (-p/2, p/2):
+// four 32 x 32-bit products give a 96-bit T, and since 2^k = c (mod p) one more
+// folds its top word, t = (T mod 2^k) + (T >> k) c. The tables hold
+// W 2^(64 - k) as two signed 32-bit digits (Z = zh 2^32 + zl), which puts bit
+// k of T at the word boundary: T 2^(64-k) = H 2^32 + lo32(L), its low 64 bits
+// M (a multiple of 2^(64-k)) shift back, its top word multiplies c.
+// Against a Shoup product that is 5 wide multiplies instead of 6 wide and 4
+// narrow ones (the wide ones take the multiplier twice as long): butterflies
+// in registers run in 36 cycles a warp and scheduler instead of 50 (radix-16
+// rounds with loaded twiddles), and 18.5 instructions instead of 28.
+//
+// Values are signed and lazy. In units of 2^k, for any |a| < 2 (at k = 62:
+// |a| <= 2^63 - 2^34) the result is within 0.5 + 2^(31-k) c: 0.625 at k = 62
+// with the largest c. fold_norm brings any x back to 0.5. Smaller k
+// leave all magnitudes below 2^60.
+
+// a * b + c of signed 32-bit factors. One asm block keeps the compiler from
+// reordering the sums, which then fuse into the multiplications.
+__device__ __forceinline__ int64_t fold_mad(int32_t a, int32_t b, int64_t c) {
+  int64_t d;
+  asm("{\n\t.reg .s64 t;\n\tmul.wide.s32 t, %1, %2;\n\tadd.s64 %0, t, %3;\n\t}" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ int64_t fold_wide(int32_t a, int32_t b) {
+  int64_t d;
+  asm("mul.wide.s32 %0, %1, %2;" : "=l"(d) : "r"(a), "r"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t fold_madu(uint32_t a, uint32_t b, uint64_t c) {
+  uint64_t d;
+  asm("{\n\t.reg .u64 t;\n\tmul.wide.u32 t, %1, %2;\n\tadd.u64 %0, t, %3;\n\t}" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t pack64(uint32_t lo, uint32_t hi) { return ((uint64_t)hi << 32) | lo; }
+
+// a w mod p, lazy and signed; z = (zl, zh) of W0, then of W1. With |a1| <=
+// 2^31 - 4 neither L nor H overflows: |L| <= 2^62 + |a1| 2^31, and the same
+// bound plus 2^31 for H.
+__device__ __forceinline__ int64_t fold_mul(int64_t a, const int4& z, const DevPrime& pr) {
+  const int32_t a0 = (int32_t)a;
+  const int32_t a1 = (int32_t)(a >> 32) + (int32_t)((uint32_t)a0 >> 31);
+  const int64_t L = fold_mad(a1, z.z, fold_wide(a0, z.x));
+  const int64_t H = fold_mad(a1, z.w, fold_mad(a0, z.y, L >> 32));
+  const int64_t M = (int64_t)pack64((uint32_t)L, (uint32_t)H);
+  const int32_t top = (int32_t)(H >> 32) + (int32_t)((uint32_t)H >> 31);
+  return fold_mad(top, pr.f_c, M >> (32 - pr.f_sh));
+}
+
+// x reduced to within 2^(k-1) plus a few c, any x: the multiple of 2^k nearest
+// to it, times c, on the sign-extended low k bits.
+__device__ __forceinline__ int64_t fold_norm(int64_t x, const DevPrime& pr) {
+  const int32_t h = (int32_t)(x >> 32);
+  const int32_t n = ((h >> (pr.f_sh - 1)) + 1) >> 1;
+  int32_t low;
+  asm("szext.wrap.s32 %0, %1, %2;" : "=r"(low) : "r"(h), "r"(pr.f_sh));
+  return fold_mad(n, pr.f_c, (int64_t)pack64((uint32_t)x, (uint32_t)low));
+}
+
+// The same for |x| < 1.5 * 2^62.
+__device__ __forceinline__ int64_t fold_norm_small(int64_t x, const DevPrime& pr) {
+  const int32_t half = 1 << (pr.f_sh - 1), mask = (1 << pr.f_sh) - 1;
+  const int32_t h = (int32_t)(x >> 32) + half;
+  return fold_mad(h >> pr.f_sh, pr.f_c, (int64_t)pack64((uint32_t)x, (uint32_t)((h & mask) - half)));
+}
+
+// The same for an unsigned x below 2^64 - 2^(k-1).
+__device__ __forceinline__ int64_t fold_norm_u(uint64_t x, const DevPrime& pr) {
+  const uint32_t half = 1u << (pr.f_sh - 1), mask = (1u << pr.f_sh) - 1;
+  const uint32_t h = (uint32_t)(x >> 32) + half;
+  return (int64_t)fold_madu(h >> pr.f_sh, (uint32_t)pr.f_c, pack64((uint32_t)x, (h & mask) - half));
+}
+
+// Any 64-bit word as a non-negative residue of at most 2^k + 2^(64-k) c.
+__device__ __forceinline__ int64_t fold_lift(uint64_t x, const DevPrime& pr) {
+  const uint32_t h = (uint32_t)(x >> 32);
+  return (int64_t)fold_madu(h >> pr.f_sh, (uint32_t)pr.f_c, pack64((uint32_t)x, h & ((1u << pr.f_sh) - 1)));
+}
+
+// The canonical residue of a lazy value: x + bias is positive and below
+// 2 * bias, so one fold leaves it below 2p (fold_params).
+__device__ __forceinline__ uint64_t fold_canon(int64_t x, const DevPrime& pr) {
+  return csub((uint64_t)fold_lift((uint64_t)x + pr.f_bias, pr), pr.p);
+}
+
+// (hi:lo) mod p for hi:lo < 2^(2k + 1): lazy, in [0, 2^k + 2 c^2 + c]. The bits
+// from k up (at most k + 1) times c, then the bits from k up of that sum
+// (below 2c + 1) times c.
+__device__ __forceinline__ uint64_t fold_wide_product(uint64_t hi, uint64_t lo, const DevPrime& pr) {
+  const uint32_t mask = (1u << pr.f_sh) - 1, c = (uint32_t)pr.f_c;
+  const uint32_t l1 = (uint32_t)(lo >> 32), h0 = (uint32_t)hi, h1 = (uint32_t)(hi >> 32);
+  const uint32_t q0 = __funnelshift_r(l1, h0, pr.f_sh), q1 = __funnelshift_r(h0, h1, pr.f_sh);
+  const uint64_t u = fold_madu(q0, c, pack64((uint32_t)lo, l1 & mask));
+  const uint64_t v = fold_madu(q1, c, u >> 32);
+  const uint32_t n = (uint32_t)(v >> pr.f_sh);
+  return fold_madu(n, c, pack64((uint32_t)u, (uint32_t)v & mask));
+}
+
+// Forward butterfly (x, y) -> (x + w y, x - w y). In units of 2^62: |x| up to
+// 1.75 with NORM, up to 1.125 without it; the results stay within 1.125 and
+// 1.75. So every second stage normalises, and a transform enters and leaves
+// at 1.125.
+template <bool NORM>
+__device__ __forceinline__ void fold_fwd_bfly(uint64_t& x, uint64_t& y, const int4& z, const DevPrime& pr) {
+  const int64_t t = fold_mul((int64_t)y, z, pr);
+  const int64_t a = NORM ? fold_norm((int64_t)x, pr) : (int64_t)x;
+  x = (uint64_t)(a + t);
+  y = (uint64_t)(a - t);
+}
+
+// Inverse butterfly (x, y) -> (x + y, (x - y) z): results within 0.625 for
+// inputs within 0.625, or (FIRST) non-negative inputs up to 1.04.
+template <bool FIRST>
+__device__ __forceinline__ void fold_inv_bfly(uint64_t& x, uint64_t& y, const int4& z, const DevPrime& pr) {
+  const uint64_t s = x + y;
+  y = (uint64_t)fold_mul((int64_t)(x - y), z, pr);
+  x = (uint64_t)(FIRST ? fold_norm_u(s, pr) : fold_norm_small((int64_t)s, pr));
 }
 
 // native.rs:238-243 `reduce3`: [0, 4p) -> [0, p).

@@ -49,7 +49,9 @@ void set_last_error(const std::string& msg);
 // every context that uses the prime (registry keyed by device, p, n, root).
 struct PrimeTables {
   NttTablesHost host;
-  DevBuf tables;  // 4 * n words: (omega, shoup) pairs, then (zeta_inv, shoup) pairs
+  // 4 * n words: (omega, shoup) pairs, then (zeta_inv, shoup) pairs; for
+  // primes just below a power of two, 4 * n more: their fold_mul digits.
+  DevBuf tables;
   DevPrime dev;
 };
 std::shared_ptr<PrimeTables> get_prime_tables(uint64_t p, size_t n, uint64_t root);
@@ -65,6 +67,8 @@ struct Context {
   // followed by (q_i - (floor(q_last/2) mod q_i)) for i < L-1.
   DevBuf d_switch;
   std::unique_ptr<RnsContextHost> rns;
+  // Every prime lies just below a power of two (fold_params).
+  bool fold = false;
   int device = 0;
 
   Context(const std::vector<uint64_t>& moduli, size_t degree, const uint64_t* roots);
@@ -132,10 +136,12 @@ void poly_switch_down_ntt(const Context& ctx, PolyRef in, PolyRef out, uint64_t 
 // The strided last stages of a two-pass inverse NTT left to the consumer:
 // `s1` stages of the source context (`primes`, one DevPrime per source
 // limb), final scale N^-1 * 2^64 when `mont` (Montgomery products), else N^-1.
+// With `fold` the values are those of the transforms in fold arithmetic.
 struct InverseTop {
   uint32_t s1;
   uint32_t mont;
   const DevPrime* primes;
+  bool fold = false;
 };
 // The strided first stages of two-pass forward NTTs applied by their
 // producer, the RNS scaler: `s1` stages. Polynomials with poly % period <
@@ -154,7 +160,7 @@ struct ForwardTop {
 };
 // top != nullptr: `in` is the block pass of such a transform, and the scaler
 // applies its last stages while loading (only where rns_scale_takes_top).
-// fwd != nullptr (with top, the same s1): the outputs are written after the
+// fwd != nullptr (with top, the same s1 and arithmetic): the outputs are written after the
 // first stages of the forward NTT that consumes them.
 void rns_scale(const RnsScalerD& s, uint32_t logn, PolyRef in, PolyRef out, uint32_t start, uint32_t out_len,
                uint64_t polys, cudaStream_t st, const InverseTop* top = nullptr, const ForwardTop* fwd = nullptr);

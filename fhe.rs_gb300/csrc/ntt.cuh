@@ -18,6 +18,18 @@
 // groups of 2^(logn - bl) elements for the first (forward) or last (inverse)
 // stages plus the block kernel for the others.
 //
+// Two arithmetics. Any prime below 2^62 takes Harvey's butterflies with Shoup
+// twiddles; where every prime of a launch lies just below a power of two
+// (DevPrime::f_c, NttGeom::fold) and the blocks hold 2^12 residues, reduced
+// transforms take the FOLD form of the same stages (common.cuh), with signed
+// lazy values between the passes and the same canonical outputs. Lazy forward
+// outputs ([0, 4p), a value callers see) stay with Harvey's butterflies.
+// The FOLD form took 256 polynomials of 6 limbs at N = 2^14, forward and
+// inverse, from 599 to 519 us and the batch of 64 multiplications there from
+// 2.365 to 2.120 ms (24 instructions a butterfly instead of 35 in the block
+// kernel); what bounds it now is the latency of the twiddle loads beside the
+// multiplier (61% busy).
+//
 // The kernels are templates over a source functor (produces the input
 // residue of element i; fuses element-wise prologues such as the BFV tensor
 // product) and a destination functor (consumes the output; fuses epilogues
@@ -27,6 +39,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "lib.hpp"
 
 namespace fheg {
 // Internal linkage: every translation unit that includes this header gets its
@@ -47,17 +60,52 @@ struct NttGeom {
   const uint4* jobs;       // optional ragged job table
   uint32_t mont;           // inverse transforms: inputs carry a factor 2^-64 (Montgomery products)
   uint32_t pf_stride;      // > 0: each CTA prefetches into L2 the input of CTA blockIdx.x + pf_stride
+  bool fold;               // every prime has DevPrime::f_c
 };
 
+// The launch geometry of whole polynomials over the limbs of `c` from `first`.
+inline NttGeom ntt_geom(const Context& c, size_t first, size_t limbs) {
+  NttGeom g{};
+  g.primes = c.primes_dev() + first;
+  g.limbs = (uint32_t)limbs;
+  g.fold = c.fold;
+  return g;
+}
+inline NttGeom ntt_geom(const Context& c) { return ntt_geom(c, 0, c.L()); }
+// A ragged launch over moduli of `c`.
+inline NttGeom ntt_geom(const Context& c, const uint4* jobs) {
+  NttGeom g = ntt_geom(c, 0, 1);
+  g.jobs = jobs;
+  return g;
+}
+
+// Whether a reduced transform of 2^logn in blocks of 2^bl runs in fold
+// arithmetic: the default block size only (the others are for tuning runs).
+inline bool ntt_folds(const NttGeom& g, uint32_t logn, uint32_t bl) { return g.fold && logn >= 12 && bl == 12; }
+
+// Sources whose values come from other moduli or from callers' arrays declare
+// kAnyWord = true and provide word(job, prime, i), the value before any
+// reduction, which FOLD kernels reduce their own way; the other ones are below
+// p, or come from an earlier pass.
+template <class S>
+constexpr auto src_any_word(int) -> decltype(S::kAnyWord) {
+  return S::kAnyWord;
+}
+template <class S>
+constexpr bool src_any_word(long) {
+  return false;
+}
 
 // Final scale of an inverse transform: N^-1, or N^-1 * 2^64 when the inputs
 // are Montgomery products (a * b * 2^-64), which cancels their factor.
+template <bool FOLD = false>
 __device__ __forceinline__ uint64_t inv_final_scale(const NttGeom& g, const DevPrime& pr, uint64_t v) {
-  return g.mont ? mul_shoup(v, pr.ninv_mont, pr.ninv_mont_shoup, pr.p) : mul_shoup(v, pr.ninv, pr.ninv_shoup, pr.p);
+  if constexpr (FOLD) return fold_canon(fold_mul((int64_t)v, pr.f_ninv, pr), pr);
+  else return g.mont ? mul_shoup(v, pr.ninv_mont, pr.ninv_mont_shoup, pr.p) : mul_shoup(v, pr.ninv, pr.ninv_shoup, pr.p);
 }
 
 // Sources that load their inputs themselves through shared memory declare
-// kStaged = true and provide stage<LOGN, T, E>(job, prime, base, sm, tid, x),
+// kStaged = true and provide stage<LOGN, T, E, FOLD>(job, prime, base, sm, tid, x),
 // which fills x[e] with the value of element base + tid + e * T and leaves the
 // shared buffer free (ending with a barrier).
 template <class S>
@@ -69,7 +117,8 @@ constexpr bool src_is_staged(long) {
   return false;
 }
 
-// Sources whose values are Montgomery products declare kMontgomery = true.
+// Sources whose values are Montgomery products (plain ones in FOLD kernels)
+// declare kMontgomery = true and provide product<FOLD>(job, prime, i).
 template <class S>
 constexpr auto src_is_montgomery(int) -> decltype(S::kMontgomery) {
   return S::kMontgomery;
@@ -82,6 +131,15 @@ constexpr bool src_is_montgomery(long) {
 struct NttJob {
   uint32_t poly, limb, beta, aux;
 };
+
+// The value a kernel transforms: Montgomery sources give plain products to
+// FOLD kernels.
+template <bool FOLD, class Src>
+__device__ __forceinline__ uint64_t src_load(const Src& src, const NttJob& j, const DevPrime& pr, uint32_t i) {
+  if constexpr (FOLD && src_any_word<Src>(0)) return (uint64_t)fold_lift(src.word(j, pr, i), pr);
+  else if constexpr (src_is_montgomery<Src>(0)) return src.template product<FOLD>(j, pr, i);
+  else return src(j, pr, i);
+}
 
 // L2 prefetch hint (no fault, no register result).
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
@@ -185,7 +243,8 @@ struct NttShape {
 // elements c * 2^(LOGN-S0) + b + t * 2^(LOGN-S0-K) for t < 2^K. The stage
 // with 2^s chunks uses omegas[2^s * tw_mult + chunk] (tw_mult = 1 for a whole
 // transform); the 2^r twiddles a group needs at round stage r are contiguous.
-template <int LOGN, int S0, int K>
+// FOLD normalises in every second stage, the last one included.
+template <int LOGN, int S0, int K, bool FOLD>
 __device__ __forceinline__ void fwd_round(uint64_t* x, uint32_t tid, const DevPrime& pr, uint32_t tw_mult) {
   constexpr int E = NttShape<LOGN>::E;
   constexpr int T = NttShape<LOGN>::T;
@@ -199,13 +258,19 @@ __device__ __forceinline__ void fwd_round(uint64_t* x, uint32_t tid, const DevPr
 #pragma unroll
     for (int r = 0; r < K; r++) {
       const int half = 1 << (K - 1 - r);
-      const ulonglong2* twr = pr.tw + (1u << (S0 + r)) * tw_mult + (c << r);
+      const uint32_t tw0 = (1u << (S0 + r)) * tw_mult + (c << r);
       // Constant trip counts at every level keep x[] in registers.
 #pragma unroll
       for (int t = 0; t < (1 << K); t++) {
         if (t & half) continue;
-        const ulonglong2 w = __ldg(twr + (t >> (K - r)));
-        fwd_bfly(xx[t], xx[t + half], w.x, w.y, pr.p, pr.p2);
+        if constexpr (FOLD) {
+          const int4 z = __ldg(pr.ftw + tw0 + (t >> (K - r)));
+          if ((LOGN - 1 - S0 - r) & 1) fold_fwd_bfly<false>(xx[t], xx[t + half], z, pr);
+          else fold_fwd_bfly<true>(xx[t], xx[t + half], z, pr);
+        } else {
+          const ulonglong2 w = __ldg(pr.tw + tw0 + (t >> (K - r)));
+          fwd_bfly(xx[t], xx[t + half], w.x, w.y, pr.p, pr.p2);
+        }
       }
     }
   }
@@ -241,19 +306,19 @@ __device__ __forceinline__ void fwd_from_smem(uint64_t* x, uint64_t* sm, uint32_
 }
 
 // Applies forward rounds S0, S0+LOGE, ... up to LOGN, exchanging through smem.
-template <int LOGN, int S0>
+template <int LOGN, int S0, bool FOLD>
 __device__ __forceinline__ void fwd_rounds(uint64_t* x, uint64_t* sm, uint32_t tid, const DevPrime& pr,
                                            uint32_t tw_mult) {
   constexpr int LOGE = NttShape<LOGN>::LOGE;
   constexpr int K = (LOGN - S0) < LOGE ? (LOGN - S0) : LOGE;
-  fwd_round<LOGN, S0, K>(x, tid, pr, tw_mult);
+  fwd_round<LOGN, S0, K, FOLD>(x, tid, pr, tw_mult);
   if constexpr (S0 + K < LOGN) {
     constexpr int K2 = (LOGN - S0 - K) < LOGE ? (LOGN - S0 - K) : LOGE;
     __syncthreads();
     fwd_to_smem<LOGN, S0, K>(x, sm, tid);
     __syncthreads();
     fwd_from_smem<LOGN, S0 + K, K2>(x, sm, tid);
-    fwd_rounds<LOGN, S0 + K>(x, sm, tid, pr, tw_mult);
+    fwd_rounds<LOGN, S0 + K, FOLD>(x, sm, tid, pr, tw_mult);
   } else {
     // Leave the output in shared memory for a coalesced store.
     __syncthreads();
@@ -265,7 +330,7 @@ __device__ __forceinline__ void fwd_rounds(uint64_t* x, uint64_t* sm, uint32_t t
 // Forward NTT of blocks of 2^LOGN elements. With g.s1 > 0 the block is block
 // `beta` of a transform of size 2^(LOGN + s1) whose first s1 stages already
 // ran (ntt_fwd_top). REDUCE selects reduced ([0, p)) or lazy ([0, 4p)) output.
-template <int LOGN, bool REDUCE, class Src, class Dst>
+template <int LOGN, bool REDUCE, bool FOLD, class Src, class Dst>
 __global__ void __launch_bounds__(NttShape<LOGN>::T, NttShape<LOGN>::MIN_BLOCKS) k_ntt_fwd(NttGeom g, Src src, Dst dst) {
   constexpr int E = NttShape<LOGN>::E;
   constexpr int T = NttShape<LOGN>::T;
@@ -278,14 +343,15 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, NttShape<LOGN>::MIN_BLOCKS)
   uint64_t x[E];
   // Round 0 holds elements tid + e*T: coalesced loads.
 #pragma unroll
-  for (int e = 0; e < E; e++) x[e] = src(jb, pr, base + tid + e * T);
-  fwd_rounds<LOGN, 0>(x, sm, tid, pr, (1u << g.s1) + jb.beta);
+  for (int e = 0; e < E; e++) x[e] = src_load<FOLD>(src, jb, pr, base + tid + e * T);
+  fwd_rounds<LOGN, 0, FOLD>(x, sm, tid, pr, (1u << g.s1) + jb.beta);
   const uint32_t sb = swz8(tid);
 #pragma unroll
   for (int e = 0; e < E; e++) {
     const uint32_t i = tid + e * T;
     uint64_t v = sm_at(sm, sb ^ swz8(e * T));
-    if (REDUCE) v = reduce4(v, pr.p, pr.p2);
+    if constexpr (FOLD) v = fold_canon((int64_t)v, pr);
+    else if (REDUCE) v = reduce4(v, pr.p, pr.p2);
     dst(jb, pr, base + i, v);
   }
 }
@@ -302,7 +368,7 @@ __host__ __device__ __forceinline__ constexpr uint32_t inv_index(uint32_t tid, i
   return (c << (U0 + K)) + b + ((uint32_t)t << U0);
 }
 
-template <int LOGN, int U0, int K>
+template <int LOGN, int U0, int K, bool FOLD>
 __device__ __forceinline__ void inv_round(uint64_t* x, uint32_t tid, const DevPrime& pr, uint32_t n_total,
                                           uint32_t s1, uint32_t beta) {
   constexpr int E = NttShape<LOGN>::E;
@@ -317,13 +383,19 @@ __device__ __forceinline__ void inv_round(uint64_t* x, uint32_t tid, const DevPr
     for (int r = 0; r < K; r++) {
       // m_local = N_local / (2l) chunks of this block at this stage.
       const uint32_t m_local = 1u << (LOGN - 1 - U0 - r);
-      const ulonglong2* twr = pr.itw + (n_total - (m_local << (s1 + 1)) + beta * m_local + (c << (K - 1 - r)));
+      const uint32_t tw0 = n_total - (m_local << (s1 + 1)) + beta * m_local + (c << (K - 1 - r));
       const int span = 1 << r;
 #pragma unroll
       for (int t = 0; t < (1 << K); t++) {
         if (t & span) continue;
-        const ulonglong2 z = __ldg(twr + (t >> (r + 1)));
-        inv_bfly(xx[t], xx[t + span], z.x, z.y, pr.p, pr.p2);
+        if constexpr (FOLD) {
+          const int4 z = __ldg(pr.fitw + tw0 + (t >> (r + 1)));
+          if (U0 + r == 0) fold_inv_bfly<true>(xx[t], xx[t + span], z, pr);
+          else fold_inv_bfly<false>(xx[t], xx[t + span], z, pr);
+        } else {
+          const ulonglong2 z = __ldg(pr.itw + tw0 + (t >> (r + 1)));
+          inv_bfly(xx[t], xx[t + span], z.x, z.y, pr.p, pr.p2);
+        }
       }
     }
   }
@@ -354,25 +426,25 @@ struct InvFirst {
   static constexpr int K = (LOGN % LOGE) ? (LOGN % LOGE) : LOGE;
 };
 
-template <int LOGN, int U0, int K>
+template <int LOGN, int U0, int K, bool FOLD>
 __device__ __forceinline__ void inv_rounds(uint64_t* x, uint64_t* sm, uint32_t tid, const DevPrime& pr,
                                            uint32_t n_total, uint32_t s1, uint32_t beta) {
   constexpr int LOGE = NttShape<LOGN>::LOGE;
-  inv_round<LOGN, U0, K>(x, tid, pr, n_total, s1, beta);
+  inv_round<LOGN, U0, K, FOLD>(x, tid, pr, n_total, s1, beta);
   if constexpr (U0 + K < LOGN) {
     constexpr int K2 = (LOGN - U0 - K) < LOGE ? (LOGN - U0 - K) : LOGE;
     __syncthreads();
     inv_to_smem<LOGN, U0, K>(x, sm, tid);
     __syncthreads();
     inv_from_smem<LOGN, U0 + K, K2>(x, sm, tid);
-    inv_rounds<LOGN, U0 + K, K2>(x, sm, tid, pr, n_total, s1, beta);
+    inv_rounds<LOGN, U0 + K, K2, FOLD>(x, sm, tid, pr, n_total, s1, beta);
   }
 }
 
 // Inverse NTT of blocks of 2^LOGN elements (all GS stages with l < 2^LOGN).
 // With g.s1 = 0 this is the whole `backward`, including the N^-1 scaling
 // (FINAL). With g.s1 > 0 the remaining stages run in ntt_inv_top.
-template <int LOGN, bool FINAL, class Src, class Dst>
+template <int LOGN, bool FINAL, bool FOLD, class Src, class Dst>
 __global__ void __launch_bounds__(NttShape<LOGN>::T, NttShape<LOGN>::MIN_BLOCKS) k_ntt_inv(NttGeom g, Src src, Dst dst) {
   constexpr int E = NttShape<LOGN>::E;
   constexpr int T = NttShape<LOGN>::T;
@@ -389,24 +461,24 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, NttShape<LOGN>::MIN_BLOCKS)
   // memory round trip costs more than the load latency it hides.)
   const uint32_t sb = swz8(tid);
   if constexpr (src_is_staged<Src>(0)) {
-    src.template stage<LOGN, T, E>(jb, pr, base, sm, tid, x);
+    src.template stage<LOGN, T, E, FOLD>(jb, pr, base, sm, tid, x);
 #pragma unroll
     for (int e = 0; e < E; e++) sm_at(sm, sb ^ swz8(e * T)) = x[e];
   } else {
 #pragma unroll
     for (int e = 0; e < E; e++) {
       const uint32_t i = tid + e * T;
-      sm_at(sm, sb ^ swz8(e * T)) = src(jb, pr, base + i);
+      sm_at(sm, sb ^ swz8(e * T)) = src_load<FOLD>(src, jb, pr, base + i);
     }
   }
   __syncthreads();
   inv_from_smem<LOGN, 0, K0>(x, sm, tid);
-  inv_rounds<LOGN, 0, K0>(x, sm, tid, pr, 1u << (LOGN + g.s1), g.s1, jb.beta);
+  inv_rounds<LOGN, 0, K0, FOLD>(x, sm, tid, pr, 1u << (LOGN + g.s1), g.s1, jb.beta);
   // The last round holds elements tid + e*T (b = tid, c = 0): coalesced stores.
 #pragma unroll
   for (int e = 0; e < E; e++) {
     uint64_t v = x[e];
-    if (FINAL) v = inv_final_scale(g, pr, v);
+    if (FINAL) v = inv_final_scale<FOLD>(g, pr, v);
     dst(jb, pr, base + tid + e * T, v);
   }
 }
@@ -422,7 +494,7 @@ __global__ void __launch_bounds__(1024) k_ntt_fwd_small(NttGeom g, uint32_t logn
   const uint32_t n = 1u << logn, tid = threadIdx.x, nt = blockDim.x;
   const NttJob jb = decode_job(g);
   const DevPrime pr = g.primes[jb.limb];
-  for (uint32_t i = tid; i < n; i += nt) sm[i] = src(jb, pr, i);
+  for (uint32_t i = tid; i < n; i += nt) sm[i] = src_load<false>(src, jb, pr, i);
   __syncthreads();
   for (uint32_t s = 0; s < logn; s++) {
     const uint32_t l = n >> (s + 1);
@@ -445,7 +517,7 @@ __global__ void __launch_bounds__(1024) k_ntt_inv_small(NttGeom g, uint32_t logn
   const uint32_t n = 1u << logn, tid = threadIdx.x, nt = blockDim.x;
   const NttJob jb = decode_job(g);
   const DevPrime pr = g.primes[jb.limb];
-  for (uint32_t i = tid; i < n; i += nt) sm[i] = src(jb, pr, i);
+  for (uint32_t i = tid; i < n; i += nt) sm[i] = src_load<false>(src, jb, pr, i);
   __syncthreads();
   for (uint32_t l = 1; l < n; l <<= 1) {
     const uint32_t m = n / (2 * l);
@@ -472,25 +544,35 @@ __global__ void __launch_bounds__(1024) k_ntt_inv_small(NttGeom g, uint32_t logn
 // in [0, 4p)): what the strided forward pass does per thread, also applied
 // by producers that write the block pass's input directly (the RNS scaler of
 // the multiplication).
-template <int S1>
+// FOLD: inputs within 1.125 units (common.cuh), outputs within it.
+template <int S1, bool FOLD>
 __device__ __forceinline__ void fwd_top_stages(uint64_t* x, const DevPrime& pr) {
 #pragma unroll
   for (int s = 0; s < S1; s++) {
     const int half = 1 << (S1 - 1 - s);
 #pragma unroll
     for (int k = 0; k < (1 << s); k++) {
-      const ulonglong2 wp = __ldg(pr.tw + (1u << s) + k);
-      const uint64_t w = wp.x, ws = wp.y;
+      if constexpr (FOLD) {
+        const int4 z = __ldg(pr.ftw + (1u << s) + k);
 #pragma unroll
-      for (int u = 0; u < half; u++) {
-        const int t = (k << (S1 - s)) + u;
-        fwd_bfly(x[t], x[t + half], w, ws, pr.p, pr.p2);
+        for (int u = 0; u < half; u++) {
+          const int t = (k << (S1 - s)) + u;
+          if ((S1 - 1 - s) & 1) fold_fwd_bfly<false>(x[t], x[t + half], z, pr);
+          else fold_fwd_bfly<true>(x[t], x[t + half], z, pr);
+        }
+      } else {
+        const ulonglong2 wp = __ldg(pr.tw + (1u << s) + k);
+#pragma unroll
+        for (int u = 0; u < half; u++) {
+          const int t = (k << (S1 - s)) + u;
+          fwd_bfly(x[t], x[t + half], wp.x, wp.y, pr.p, pr.p2);
+        }
       }
     }
   }
 }
 
-template <int S1, class Src, class Dst>
+template <int S1, bool FOLD, class Src, class Dst>
 __global__ void __launch_bounds__(256) k_ntt_fwd_top(NttGeom g, uint32_t logb, uint32_t groups_per_limb,
                                                      uint64_t total, Src src, Dst dst) {
   const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -500,8 +582,8 @@ __global__ void __launch_bounds__(256) k_ntt_fwd_top(NttGeom g, uint32_t logb, u
   const DevPrime pr = g.primes[jb.limb];
   uint64_t x[1 << S1];
 #pragma unroll
-  for (int t = 0; t < (1 << S1); t++) x[t] = src(jb, pr, b + ((uint32_t)t << logb));
-  fwd_top_stages<S1>(x, pr);
+  for (int t = 0; t < (1 << S1); t++) x[t] = src_load<FOLD>(src, jb, pr, b + ((uint32_t)t << logb));
+  fwd_top_stages<S1, FOLD>(x, pr);
 #pragma unroll
   for (int t = 0; t < (1 << S1); t++) dst(jb, pr, b + ((uint32_t)t << logb), x[t]);
 }
@@ -511,34 +593,59 @@ __global__ void __launch_bounds__(256) k_ntt_fwd_top(NttGeom g, uint32_t logb, u
 // x[t] = element b + t * n_total / 2^S1 of one limb: what the strided inverse
 // pass does per thread, also applied by consumers that read the block pass's
 // output directly (the RNS scaler of the multiplication).
-template <int S1>
+// FOLD: inputs within 0.625 units; no Montgomery factor.
+template <int S1, bool FOLD>
 __device__ __forceinline__ void inv_top_stages(uint64_t* x, const DevPrime& pr, uint32_t n_total, bool mont) {
+  if constexpr (FOLD) {
 #pragma unroll
-  for (int r = 0; r < S1 - 1; r++) {
-    const int span = 1 << r;
-    const uint32_t m = 1u << (S1 - 1 - r);  // chunks at this stage
+    for (int r = 0; r < S1 - 1; r++) {
+      const int span = 1 << r;
+      const uint32_t m = 1u << (S1 - 1 - r);  // chunks at this stage
 #pragma unroll
-    for (int k = 0; k < (1 << (S1 - 1 - r)); k++) {
-      const ulonglong2 zp = __ldg(pr.itw + (n_total - 2 * m + k));
-      const uint64_t z = zp.x, zs = zp.y;
+      for (int k = 0; k < (1 << (S1 - 1 - r)); k++) {
+        const int4 z = __ldg(pr.fitw + (n_total - 2 * m + k));
 #pragma unroll
-      for (int u = 0; u < span; u++) {
-        const int t = (k << (r + 1)) + u;
-        inv_bfly(x[t], x[t + span], z, zs, pr.p, pr.p2);
+        for (int u = 0; u < span; u++) {
+          const int t = (k << (r + 1)) + u;
+          fold_inv_bfly<false>(x[t], x[t + span], z, pr);
+        }
       }
     }
-  }
-  // The last stage (one chunk, twiddle zetas_inv[N - 2]) with the final
-  // scale folded into its products.
-  const uint64_t s = mont ? pr.ninv_mont : pr.ninv, s_shoup = mont ? pr.ninv_mont_shoup : pr.ninv_shoup;
-  const uint64_t zs = mont ? pr.zlast_ninv_mont : pr.zlast_ninv;
-  const uint64_t zs_shoup = mont ? pr.zlast_ninv_mont_shoup : pr.zlast_ninv_shoup;
-  constexpr int kHalf = 1 << (S1 - 1);
+    constexpr int kSpan = 1 << (S1 - 1);
 #pragma unroll
-  for (int u = 0; u < kHalf; u++) inv_bfly_final(x[u], x[u + kHalf], zs, zs_shoup, s, s_shoup, pr.p, pr.p2);
+    for (int u = 0; u < kSpan; u++) {
+      const int64_t a = (int64_t)x[u], b = (int64_t)x[u + kSpan];
+      x[u] = fold_canon(fold_mul(a + b, pr.f_ninv, pr), pr);
+      x[u + kSpan] = fold_canon(fold_mul(a - b, pr.f_zlast, pr), pr);
+    }
+  } else {
+#pragma unroll
+    for (int r = 0; r < S1 - 1; r++) {
+      const int span = 1 << r;
+      const uint32_t m = 1u << (S1 - 1 - r);  // chunks at this stage
+#pragma unroll
+      for (int k = 0; k < (1 << (S1 - 1 - r)); k++) {
+        const ulonglong2 zp = __ldg(pr.itw + (n_total - 2 * m + k));
+        const uint64_t z = zp.x, zs = zp.y;
+#pragma unroll
+        for (int u = 0; u < span; u++) {
+          const int t = (k << (r + 1)) + u;
+          inv_bfly(x[t], x[t + span], z, zs, pr.p, pr.p2);
+        }
+      }
+    }
+    // The last stage (one chunk, twiddle zetas_inv[N - 2]) with the final
+    // scale folded into its products.
+    const uint64_t s = mont ? pr.ninv_mont : pr.ninv, s_shoup = mont ? pr.ninv_mont_shoup : pr.ninv_shoup;
+    const uint64_t zs = mont ? pr.zlast_ninv_mont : pr.zlast_ninv;
+    const uint64_t zs_shoup = mont ? pr.zlast_ninv_mont_shoup : pr.zlast_ninv_shoup;
+    constexpr int kHalf = 1 << (S1 - 1);
+#pragma unroll
+    for (int u = 0; u < kHalf; u++) inv_bfly_final(x[u], x[u + kHalf], zs, zs_shoup, s, s_shoup, pr.p, pr.p2);
+  }
 }
 
-template <int S1, class Src, class Dst>
+template <int S1, bool FOLD, class Src, class Dst>
 __global__ void __launch_bounds__(256) k_ntt_inv_top(NttGeom g, uint32_t logb, uint32_t groups_per_limb,
                                                      uint64_t total, Src src, Dst dst) {
   const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -549,7 +656,7 @@ __global__ void __launch_bounds__(256) k_ntt_inv_top(NttGeom g, uint32_t logb, u
   uint64_t x[1 << S1];
 #pragma unroll
   for (int t = 0; t < (1 << S1); t++) x[t] = src(jb, pr, b + ((uint32_t)t << logb));
-  inv_top_stages<S1>(x, pr, 1u << (logb + S1), g.mont != 0);
+  inv_top_stages<S1, FOLD>(x, pr, 1u << (logb + S1), g.mont != 0);
 #pragma unroll
   for (int t = 0; t < (1 << S1); t++) dst(jb, pr, b + ((uint32_t)t << logb), x[t]);
 }
@@ -593,7 +700,7 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 // Forward phase 1: the first S1 stages on the groups b + t 2^LOGB (t < 2^S1)
 // with b in this CTA's share of [0, 2^LOGB); element b + t 2^LOGB lands at
 // local index b of CTA t.
-template <int LOGB, int S1, class Src>
+template <int LOGB, int S1, bool FOLD, class Src>
 __device__ __forceinline__ void fwd_cluster_top(const Src& src, const NttJob& jb, const DevPrime& pr, uint64_t* sm,
                                                 uint32_t tid, uint32_t rank) {
   constexpr int E = NttShape<LOGB>::E, T = NttShape<LOGB>::T, C = 1 << S1, GPT = E / C;
@@ -604,9 +711,9 @@ __device__ __forceinline__ void fwd_cluster_top(const Src& src, const NttJob& jb
 #pragma unroll
   for (int q = 0; q < GPT; q++)
 #pragma unroll
-    for (int t = 0; t < C; t++) x[q * C + t] = src(jb, pr, b0 + q * T + t * NB);
+    for (int t = 0; t < C; t++) x[q * C + t] = src_load<FOLD>(src, jb, pr, b0 + q * T + t * NB);
 #pragma unroll
-  for (int q = 0; q < GPT; q++) fwd_top_stages<S1>(x + q * C, pr);
+  for (int q = 0; q < GPT; q++) fwd_top_stages<S1, FOLD>(x + q * C, pr);
   const uint32_t sb = swz8(b0);
   cluster_wait();  // every peer has started (arrival at kernel entry)
 #pragma unroll
@@ -617,7 +724,7 @@ __device__ __forceinline__ void fwd_cluster_top(const Src& src, const NttJob& jb
   }
 }
 
-template <int LOGN, bool REDUCE, class Src, class Dst>
+template <int LOGN, bool REDUCE, bool FOLD, class Src, class Dst>
 __global__ void __launch_bounds__(NttShape<LOGN>::T, NttShape<LOGN>::MIN_BLOCKS)
     k_ntt_fwd_cl(NttGeom g, Src src, Dst dst) {
   constexpr int E = NttShape<LOGN>::E;
@@ -628,29 +735,30 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, NttShape<LOGN>::MIN_BLOCKS)
   const NttJob jb = decode_job(g);  // beta = the CTA's rank in its cluster
   const DevPrime pr = g.primes[jb.limb];
   switch (g.s1) {
-    case 1: fwd_cluster_top<LOGN, 1>(src, jb, pr, sm, tid, jb.beta); break;
-    case 2: fwd_cluster_top<LOGN, 2>(src, jb, pr, sm, tid, jb.beta); break;
-    case 3: fwd_cluster_top<LOGN, 3>(src, jb, pr, sm, tid, jb.beta); break;
-    default: fwd_cluster_top<LOGN, 4>(src, jb, pr, sm, tid, jb.beta); break;
+    case 1: fwd_cluster_top<LOGN, 1, FOLD>(src, jb, pr, sm, tid, jb.beta); break;
+    case 2: fwd_cluster_top<LOGN, 2, FOLD>(src, jb, pr, sm, tid, jb.beta); break;
+    case 3: fwd_cluster_top<LOGN, 3, FOLD>(src, jb, pr, sm, tid, jb.beta); break;
+    default: fwd_cluster_top<LOGN, 4, FOLD>(src, jb, pr, sm, tid, jb.beta); break;
   }
   cluster_sync();
   uint64_t x[E];
   const uint32_t sb = swz8(tid);
 #pragma unroll
   for (int e = 0; e < E; e++) x[e] = sm_at(sm, sb ^ swz8(e * T));
-  fwd_rounds<LOGN, 0>(x, sm, tid, pr, (1u << g.s1) + jb.beta);
+  fwd_rounds<LOGN, 0, FOLD>(x, sm, tid, pr, (1u << g.s1) + jb.beta);
   const uint32_t base = jb.beta << LOGN;
 #pragma unroll
   for (int e = 0; e < E; e++) {
     uint64_t v = sm_at(sm, sb ^ swz8(e * T));
-    if (REDUCE) v = reduce4(v, pr.p, pr.p2);
+    if constexpr (FOLD) v = fold_canon((int64_t)v, pr);
+    else if (REDUCE) v = reduce4(v, pr.p, pr.p2);
     dst(jb, pr, base + tid + e * T, v);
   }
 }
 
 // Inverse phase 2: the last S1 stages (and the final scale) on the groups of
 // this CTA's share, read from the cluster's blocks.
-template <int LOGB, int S1, class Dst>
+template <int LOGB, int S1, bool FOLD, class Dst>
 __device__ __forceinline__ void inv_cluster_top(const NttGeom& g, const Dst& dst, const NttJob& jb,
                                                 const DevPrime& pr, uint64_t* sm, uint32_t tid, uint32_t rank) {
   constexpr int E = NttShape<LOGB>::E, T = NttShape<LOGB>::T, C = 1 << S1, GPT = E / C;
@@ -665,14 +773,14 @@ __device__ __forceinline__ void inv_cluster_top(const NttGeom& g, const Dst& dst
     for (int q = 0; q < GPT; q++) x[q * C + t] = ld_cluster(peer + (sb ^ swz8(q * T)));
   }
 #pragma unroll
-  for (int q = 0; q < GPT; q++) inv_top_stages<S1>(x + q * C, pr, NB << S1, g.mont != 0);
+  for (int q = 0; q < GPT; q++) inv_top_stages<S1, FOLD>(x + q * C, pr, NB << S1, g.mont != 0);
 #pragma unroll
   for (int q = 0; q < GPT; q++)
 #pragma unroll
     for (int t = 0; t < C; t++) dst(jb, pr, b0 + q * T + t * NB, x[q * C + t]);
 }
 
-template <int LOGN, class Src, class Dst>
+template <int LOGN, bool FOLD, class Src, class Dst>
 __global__ void __launch_bounds__(NttShape<LOGN>::T, NttShape<LOGN>::MIN_BLOCKS)
     k_ntt_inv_cl(NttGeom g, Src src, Dst dst) {
   constexpr int E = NttShape<LOGN>::E;
@@ -686,16 +794,16 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, NttShape<LOGN>::MIN_BLOCKS)
   uint64_t x[E];
   const uint32_t sb = swz8(tid);
   if constexpr (src_is_staged<Src>(0)) {
-    src.template stage<LOGN, T, E>(jb, pr, base, sm, tid, x);
+    src.template stage<LOGN, T, E, FOLD>(jb, pr, base, sm, tid, x);
 #pragma unroll
     for (int e = 0; e < E; e++) sm_at(sm, sb ^ swz8(e * T)) = x[e];
   } else {
 #pragma unroll
-    for (int e = 0; e < E; e++) sm_at(sm, sb ^ swz8(e * T)) = src(jb, pr, base + tid + e * T);
+    for (int e = 0; e < E; e++) sm_at(sm, sb ^ swz8(e * T)) = src_load<FOLD>(src, jb, pr, base + tid + e * T);
   }
   __syncthreads();
   inv_from_smem<LOGN, 0, K0>(x, sm, tid);
-  inv_rounds<LOGN, 0, K0>(x, sm, tid, pr, 1u << (LOGN + g.s1), g.s1, jb.beta);
+  inv_rounds<LOGN, 0, K0, FOLD>(x, sm, tid, pr, 1u << (LOGN + g.s1), g.s1, jb.beta);
   // Every thread has read its last exchange: the block's results go to
   // shared memory for the cluster.
   __syncthreads();
@@ -703,10 +811,10 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, NttShape<LOGN>::MIN_BLOCKS)
   for (int e = 0; e < E; e++) sm_at(sm, sb ^ swz8(e * T)) = x[e];
   cluster_sync();
   switch (g.s1) {
-    case 1: inv_cluster_top<LOGN, 1>(g, dst, jb, pr, sm, tid, jb.beta); break;
-    case 2: inv_cluster_top<LOGN, 2>(g, dst, jb, pr, sm, tid, jb.beta); break;
-    case 3: inv_cluster_top<LOGN, 3>(g, dst, jb, pr, sm, tid, jb.beta); break;
-    default: inv_cluster_top<LOGN, 4>(g, dst, jb, pr, sm, tid, jb.beta); break;
+    case 1: inv_cluster_top<LOGN, 1, FOLD>(g, dst, jb, pr, sm, tid, jb.beta); break;
+    case 2: inv_cluster_top<LOGN, 2, FOLD>(g, dst, jb, pr, sm, tid, jb.beta); break;
+    case 3: inv_cluster_top<LOGN, 3, FOLD>(g, dst, jb, pr, sm, tid, jb.beta); break;
+    default: inv_cluster_top<LOGN, 4, FOLD>(g, dst, jb, pr, sm, tid, jb.beta); break;
   }
   // No CTA leaves while another may still read its shared memory.
   cluster_sync();
@@ -715,13 +823,22 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, NttShape<LOGN>::MIN_BLOCKS)
 // ---------------------------------------------------------------------------
 // Basic source / destination functors.
 
-struct SrcPoly {
+// Rows of canonical residues; ANY: of any 64-bit words (callers' arrays).
+template <bool ANY>
+struct SrcRows {
+  static constexpr bool kAnyWord = ANY;
+  __device__ __forceinline__ uint64_t word(const NttJob& j, const DevPrime&, uint32_t i) const {
+    return r.at(j.poly, j.limb)[i];
+  }
   PolyRef r;
   __device__ __forceinline__ uint64_t operator()(const NttJob& j, const DevPrime&, uint32_t i) const {
     return r.at(j.poly, j.limb)[i];
   }
   __device__ __forceinline__ void prefetch(const NttJob& j, uint32_t i) const { prefetch_l2(r.at(j.poly, j.limb) + i); }
 };
+
+using SrcPoly = SrcRows<false>;
+using SrcWords = SrcRows<true>;
 
 // Destinations also provide `reload`, which the two-pass sizes use to read
 // back the intermediate values the first pass stored.
@@ -776,9 +893,9 @@ inline uint32_t resident_ctas(K kernel, int threads, size_t smem, uint32_t* cach
   return *cache;
 }
 
-template <int LOGN, bool REDUCE, class Src, class Dst>
-void launch_fwd_block(NttGeom g, uint64_t polys, Src src, Dst dst, cudaStream_t st) {
-  auto kern = k_ntt_fwd<LOGN, REDUCE, Src, Dst>;
+template <int LOGN, bool REDUCE, bool FOLD, class Src, class Dst>
+void launch_fwd_block_as(NttGeom g, uint64_t polys, Src src, Dst dst, cudaStream_t st) {
+  auto kern = k_ntt_fwd<LOGN, REDUCE, FOLD, Src, Dst>;
   const size_t smem = ntt_smem_bytes<LOGN>();
   static bool done = false;
   set_smem(kern, smem, &done);
@@ -789,9 +906,19 @@ void launch_fwd_block(NttGeom g, uint64_t polys, Src src, Dst dst, cudaStream_t 
   after_launch("k_ntt_fwd");
 }
 
-template <int LOGN, bool FINAL, class Src, class Dst>
-void launch_inv_block(NttGeom g, uint64_t polys, Src src, Dst dst, cudaStream_t st) {
-  auto kern = k_ntt_inv<LOGN, FINAL, Src, Dst>;
+// g.fold and blocks of 2^12 give the FOLD kernels (ntt_folds): both passes
+// of a transform, and its callers that run one of them, come to the same choice.
+template <int LOGN, bool REDUCE, class Src, class Dst>
+void launch_fwd_block(NttGeom g, uint64_t polys, Src src, Dst dst, cudaStream_t st) {
+  if constexpr (REDUCE && LOGN == 12) {
+    if (g.fold) return launch_fwd_block_as<LOGN, REDUCE, true>(g, polys, src, dst, st);
+  }
+  launch_fwd_block_as<LOGN, REDUCE, false>(g, polys, src, dst, st);
+}
+
+template <int LOGN, bool FINAL, bool FOLD, class Src, class Dst>
+void launch_inv_block_as(NttGeom g, uint64_t polys, Src src, Dst dst, cudaStream_t st) {
+  auto kern = k_ntt_inv<LOGN, FINAL, FOLD, Src, Dst>;
   const size_t smem = ntt_smem_bytes<LOGN>();
   static bool done = false;
   set_smem(kern, smem, &done);
@@ -800,6 +927,14 @@ void launch_inv_block(NttGeom g, uint64_t polys, Src src, Dst dst, cudaStream_t 
   const uint64_t blocks = polys * g.limbs << g.s1;
   kern<<<(unsigned)blocks, NttShape<LOGN>::T, smem, st>>>(g, src, dst);
   after_launch("k_ntt_inv");
+}
+
+template <int LOGN, bool FINAL, class Src, class Dst>
+void launch_inv_block(NttGeom g, uint64_t polys, Src src, Dst dst, cudaStream_t st) {
+  if constexpr (LOGN == 12) {
+    if (g.fold) return launch_inv_block_as<LOGN, FINAL, true>(g, polys, src, dst, st);
+  }
+  launch_inv_block_as<LOGN, FINAL, false>(g, polys, src, dst, st);
 }
 
 // Launch of a kernel on clusters of `csize` CTAs along x.
@@ -853,9 +988,9 @@ bool cluster_fits(K kern, uint32_t s1, unsigned threads, size_t smem, int* state
 
 // Single-pass cluster transforms of 2^(LOGN + s1) residues; false (nothing
 // launched) when the GPU cannot run the cluster size.
-template <int LOGN, bool REDUCE, class Src, class Dst>
-bool launch_fwd_cluster(NttGeom g, uint32_t s1, uint64_t polys, Src src, Dst dst, cudaStream_t st) {
-  auto kern = k_ntt_fwd_cl<LOGN, REDUCE, Src, Dst>;
+template <int LOGN, bool REDUCE, bool FOLD, class Src, class Dst>
+bool launch_fwd_cluster_as(NttGeom g, uint32_t s1, uint64_t polys, Src src, Dst dst, cudaStream_t st) {
+  auto kern = k_ntt_fwd_cl<LOGN, REDUCE, FOLD, Src, Dst>;
   const size_t smem = ntt_smem_bytes<LOGN>();
   static bool done = false;
   set_smem(kern, smem, &done);
@@ -868,9 +1003,17 @@ bool launch_fwd_cluster(NttGeom g, uint32_t s1, uint64_t polys, Src src, Dst dst
   return true;
 }
 
-template <int LOGN, class Src, class Dst>
-bool launch_inv_cluster(NttGeom g, uint32_t s1, uint64_t polys, Src src, Dst dst, cudaStream_t st) {
-  auto kern = k_ntt_inv_cl<LOGN, Src, Dst>;
+template <int LOGN, bool REDUCE, class Src, class Dst>
+bool launch_fwd_cluster(NttGeom g, uint32_t s1, uint64_t polys, Src src, Dst dst, cudaStream_t st) {
+  if constexpr (REDUCE) {
+    if (g.fold) return launch_fwd_cluster_as<LOGN, REDUCE, true>(g, s1, polys, src, dst, st);
+  }
+  return launch_fwd_cluster_as<LOGN, REDUCE, false>(g, s1, polys, src, dst, st);
+}
+
+template <int LOGN, bool FOLD, class Src, class Dst>
+bool launch_inv_cluster_as(NttGeom g, uint32_t s1, uint64_t polys, Src src, Dst dst, cudaStream_t st) {
+  auto kern = k_ntt_inv_cl<LOGN, FOLD, Src, Dst>;
   const size_t smem = ntt_smem_bytes<LOGN>();
   static bool done = false;
   set_smem(kern, smem, &done);
@@ -881,6 +1024,12 @@ bool launch_inv_cluster(NttGeom g, uint32_t s1, uint64_t polys, Src src, Dst dst
   launch_cluster(kern, polys * g.limbs << s1, NttShape<LOGN>::T, smem, 1u << s1, st, g, src, dst);
   after_launch("k_ntt_inv_cl");
   return true;
+}
+
+template <int LOGN, class Src, class Dst>
+bool launch_inv_cluster(NttGeom g, uint32_t s1, uint64_t polys, Src src, Dst dst, cudaStream_t st) {
+  if (g.fold) return launch_inv_cluster_as<LOGN, true>(g, s1, polys, src, dst, st);
+  return launch_inv_cluster_as<LOGN, false>(g, s1, polys, src, dst, st);
 }
 
 // Dispatch over log2(N) for a single-pass transform (3 <= logn <= 14).
@@ -921,36 +1070,48 @@ void ntt_inv_single(uint32_t logn, NttGeom g, uint64_t polys, Src src, Dst dst, 
 // Two-pass transforms: a strided pass runs the first (forward) or last
 // (inverse) s1 stages on groups of 2^s1 elements b + t * 2^bl, and the block
 // kernel runs the other bl stages on 2^s1 blocks of 2^bl elements.
-template <class Src, class Dst>
-void launch_fwd_top(uint32_t s1, NttGeom g, uint32_t bl, uint64_t polys, Src src, Dst dst, cudaStream_t st) {
+template <bool FOLD, class Src, class Dst>
+void launch_fwd_top_as(uint32_t s1, NttGeom g, uint32_t bl, uint64_t polys, Src src, Dst dst, cudaStream_t st) {
   const uint32_t groups = 1u << bl;
   const uint64_t threads = polys * g.limbs * groups;
   const unsigned blocks = (unsigned)((threads + 255) / 256);
   g.s1 = 0;
   switch (s1) {
-    case 1: k_ntt_fwd_top<1><<<blocks, 256, 0, st>>>(g, bl, groups, threads, src, dst); break;
-    case 2: k_ntt_fwd_top<2><<<blocks, 256, 0, st>>>(g, bl, groups, threads, src, dst); break;
-    case 3: k_ntt_fwd_top<3><<<blocks, 256, 0, st>>>(g, bl, groups, threads, src, dst); break;
-    case 4: k_ntt_fwd_top<4><<<blocks, 256, 0, st>>>(g, bl, groups, threads, src, dst); break;
+    case 1: k_ntt_fwd_top<1, FOLD><<<blocks, 256, 0, st>>>(g, bl, groups, threads, src, dst); break;
+    case 2: k_ntt_fwd_top<2, FOLD><<<blocks, 256, 0, st>>>(g, bl, groups, threads, src, dst); break;
+    case 3: k_ntt_fwd_top<3, FOLD><<<blocks, 256, 0, st>>>(g, bl, groups, threads, src, dst); break;
+    case 4: k_ntt_fwd_top<4, FOLD><<<blocks, 256, 0, st>>>(g, bl, groups, threads, src, dst); break;
     default: throw Error(12, "unsupported NTT plan");
   }
   after_launch("k_ntt_fwd_top");
 }
 
-template <class Src, class Dst>
-void launch_inv_top(uint32_t s1, NttGeom g, uint32_t bl, uint64_t polys, Src src, Dst dst, cudaStream_t st) {
+template <bool REDUCE, class Src, class Dst>
+void launch_fwd_top(uint32_t s1, NttGeom g, uint32_t bl, uint64_t polys, Src src, Dst dst, cudaStream_t st) {
+  if (REDUCE && ntt_folds(g, bl + s1, bl)) launch_fwd_top_as<true>(s1, g, bl, polys, src, dst, st);
+  else launch_fwd_top_as<false>(s1, g, bl, polys, src, dst, st);
+}
+
+template <bool FOLD, class Src, class Dst>
+void launch_inv_top_as(uint32_t s1, NttGeom g, uint32_t bl, uint64_t polys, Src src, Dst dst, cudaStream_t st) {
   const uint32_t groups = 1u << bl;
   const uint64_t threads = polys * g.limbs * groups;
   const unsigned blocks = (unsigned)((threads + 255) / 256);
   g.s1 = 0;
   switch (s1) {
-    case 1: k_ntt_inv_top<1><<<blocks, 256, 0, st>>>(g, bl, groups, threads, src, dst); break;
-    case 2: k_ntt_inv_top<2><<<blocks, 256, 0, st>>>(g, bl, groups, threads, src, dst); break;
-    case 3: k_ntt_inv_top<3><<<blocks, 256, 0, st>>>(g, bl, groups, threads, src, dst); break;
-    case 4: k_ntt_inv_top<4><<<blocks, 256, 0, st>>>(g, bl, groups, threads, src, dst); break;
+    case 1: k_ntt_inv_top<1, FOLD><<<blocks, 256, 0, st>>>(g, bl, groups, threads, src, dst); break;
+    case 2: k_ntt_inv_top<2, FOLD><<<blocks, 256, 0, st>>>(g, bl, groups, threads, src, dst); break;
+    case 3: k_ntt_inv_top<3, FOLD><<<blocks, 256, 0, st>>>(g, bl, groups, threads, src, dst); break;
+    case 4: k_ntt_inv_top<4, FOLD><<<blocks, 256, 0, st>>>(g, bl, groups, threads, src, dst); break;
     default: throw Error(12, "unsupported NTT plan");
   }
   after_launch("k_ntt_inv_top");
+}
+
+template <class Src, class Dst>
+void launch_inv_top(uint32_t s1, NttGeom g, uint32_t bl, uint64_t polys, Src src, Dst dst, cudaStream_t st) {
+  if (ntt_folds(g, bl + s1, bl)) launch_inv_top_as<true>(s1, g, bl, polys, src, dst, st);
+  else launch_inv_top_as<false>(s1, g, bl, polys, src, dst, st);
 }
 
 // Full forward NTT, any 3 <= logn <= 16, following the plan of
@@ -968,7 +1129,7 @@ void ntt_forward_any(uint32_t logn, NttGeom g, uint64_t polys, Src src, Dst dst,
   }
   const uint32_t s1 = logn - bl;
   if (bl == 12 && ntt_cluster_enabled(logn) && launch_fwd_cluster<12, REDUCE>(g, s1, polys, src, dst, st)) return;
-  launch_fwd_top(s1, g, bl, polys, src, dst, st);
+  launch_fwd_top<REDUCE>(s1, g, bl, polys, src, dst, st);
   g.s1 = s1;
   switch (bl) {
     case 12: launch_fwd_block<12, REDUCE>(g, polys, SrcReload<Dst>{dst}, dst, st); break;

@@ -67,6 +67,63 @@ void upload(void* dst, const void* src, size_t bytes) {
 // ---------------------------------------------------------------------------
 // Prime table registry.
 
+bool fold_params(uint64_t p, int32_t* c, int32_t* k, uint64_t* bias) {
+  const int bits = 64 - __builtin_clzll(p);
+  if (bits < 40 || bits > 62) return false;
+  const uint64_t cc = (1ull << bits) - p;
+  if (cc > (1ull << 28) || cc > (1ull << (bits - 17))) return false;
+  // The transforms' values stay below 1.25 * 2^k + 2^33 c (common.cuh).
+  const unsigned __int128 most = ((unsigned __int128)5 << (bits - 2)) + ((unsigned __int128)cc << 33);
+  unsigned __int128 b = p;
+  while (b < most) b *= 2;
+  // x + b < 2 b: one fold must leave it below 2p.
+  if (b >> 63) return false;
+  if (((unsigned __int128)1 << bits) + (2 * b >> bits) * cc >= 2 * (unsigned __int128)p) return false;
+  *c = (int32_t)cc;
+  *k = bits;
+  *bias = (uint64_t)b;
+  return true;
+}
+
+// The residue w < p as the digits fold_mul multiplies by: W 2^(64 - k) =
+// zh 2^32 + zl with zl and zh signed and W = w or w - p. W = w - p too where the
+// rounding would take zh to 2^31.
+__host__ __device__ static inline int2 fold_digits(uint64_t w, uint64_t p, int32_t c, int32_t k) {
+  const int32_t s = 64 - k;
+  const bool neg = w > p / 2;
+  uint64_t z = (neg ? w - p : w) << s;
+  uint32_t hi = (uint32_t)((z + 0x80000000ull) >> 32);
+  if (!neg && hi == 0x80000000u) {  // less p 2^s = 2^64 - c 2^s
+    z += (uint64_t)c << s;
+    hi = (uint32_t)((z + 0x80000000ull) >> 32);
+  }
+  int2 d;
+  d.x = (int32_t)(uint32_t)z;
+  d.y = (int32_t)hi;
+  return d;
+}
+
+// The digits of w and of w 2^32 mod p.
+__host__ __device__ static inline int4 fold_entry(uint64_t w, uint64_t w32, uint64_t p, int32_t c, int32_t k) {
+  const int2 a = fold_digits(w, p, c, k), b = fold_digits(w32, p, c, k);
+  int4 e;
+  e.x = a.x;
+  e.y = a.y;
+  e.z = b.x;
+  e.w = b.y;
+  return e;
+}
+
+// fold_mul's tables from the (w, Shoup) pairs: one thread per entry, w 2^32
+// mod p by a Shoup product with 2^32 mod p.
+__global__ void k_fold_tables(const ulonglong2* tw, int4* out, uint64_t p, uint64_t r32, uint64_t r32_shoup, int32_t c,
+                              int32_t k, uint32_t total) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= total) return;
+  const uint64_t w = tw[i].x;
+  out[i] = fold_entry(w, mul_shoup(w, r32, r32_shoup, p), p, c, k);
+}
+
 std::shared_ptr<PrimeTables> get_prime_tables(uint64_t p, size_t n, uint64_t root) {
   static std::mutex mu;
   static std::map<std::tuple<int, uint64_t, size_t, uint64_t>, std::weak_ptr<PrimeTables>> registry;
@@ -81,7 +138,10 @@ std::shared_ptr<PrimeTables> get_prime_tables(uint64_t p, size_t n, uint64_t roo
   }
   auto t = std::make_shared<PrimeTables>();
   t->host = make_ntt_tables(p, n, root);
-  t->tables.alloc(4 * n * sizeof(uint64_t));
+  int32_t fc = 0, fk = 0;
+  uint64_t fbias = 0;
+  const bool fold = n >= 16 && fold_params(p, &fc, &fk, &fbias);
+  t->tables.alloc((fold ? 8 : 4) * n * sizeof(uint64_t));
   std::vector<uint64_t> inter(4 * n);
   for (size_t i = 0; i < n; i++) {
     inter[2 * i] = t->host.omegas[i];
@@ -110,6 +170,25 @@ std::shared_ptr<PrimeTables> get_prime_tables(uint64_t p, size_t n, uint64_t roo
   dp.zlast_ninv_mont_shoup = shoup(dp.zlast_ninv_mont, p);
   dp.tw = reinterpret_cast<const ulonglong2*>(d);
   dp.itw = reinterpret_cast<const ulonglong2*>(d + 2 * n);
+  dp.ftw = dp.fitw = nullptr;
+  dp.f_ninv = dp.f_zlast = make_int4(0, 0, 0, 0);
+  dp.f_bias = 0;
+  dp.f_c = dp.f_sh = 0;
+  if (fold) {
+    int4* ft = reinterpret_cast<int4*>(d + 4 * n);
+    const uint64_t r32 = (1ull << 32) % p;
+    k_fold_tables<<<(unsigned)((2 * n + 255) / 256), 256>>>(dp.tw, ft, p, r32, shoup(r32, p), fc, fk,
+                                                            (uint32_t)(2 * n));
+    after_launch("k_fold_tables");
+    check_cuda(cudaStreamSynchronize(nullptr), "cudaStreamSynchronize");
+    dp.ftw = ft;
+    dp.fitw = ft + n;
+    dp.f_ninv = fold_entry(dp.ninv, mulmod(dp.ninv, r32, p), p, fc, fk);
+    dp.f_zlast = fold_entry(dp.zlast_ninv, mulmod(dp.zlast_ninv, r32, p), p, fc, fk);
+    dp.f_bias = fbias;
+    dp.f_c = fc;
+    dp.f_sh = fk - 32;
+  }
   registry[key] = t;
   return t;
 }
@@ -131,6 +210,8 @@ Context::Context(const std::vector<uint64_t>& m, size_t n, const uint64_t* roots
     primes.push_back(get_prime_tables(m[i], n, roots ? roots[i] : 0));
     host[i] = primes.back()->dev;
   }
+  fold = true;
+  for (const DevPrime& d : host) fold = fold && d.f_c != 0;
   d_primes.alloc(sizeof(DevPrime) * m.size());
   upload(d_primes.ptr, host.data(), sizeof(DevPrime) * m.size());
   // rq/context.rs:66-73 plus the constant of rq/mod.rs:427.
@@ -166,15 +247,14 @@ std::shared_ptr<Context> Context::prefix(size_t count) const {
 
 void ntt_forward(const Context& ctx, PolyRef src, PolyRef dst, uint64_t polys, bool lazy, cudaStream_t st) {
   if (polys == 0) return;
-  NttGeom g{ctx.primes_dev(), (uint32_t)ctx.L(), 0};
-  if (lazy) ntt_forward_any<false>(ctx.logn, g, polys, SrcPoly{src}, DstPoly{dst}, st);
-  else ntt_forward_any<true>(ctx.logn, g, polys, SrcPoly{src}, DstPoly{dst}, st);
+  const NttGeom g = ntt_geom(ctx);
+  if (lazy) ntt_forward_any<false>(ctx.logn, g, polys, SrcWords{src}, DstPoly{dst}, st);
+  else ntt_forward_any<true>(ctx.logn, g, polys, SrcWords{src}, DstPoly{dst}, st);
 }
 
 void ntt_backward(const Context& ctx, PolyRef src, PolyRef dst, uint64_t polys, cudaStream_t st) {
   if (polys == 0) return;
-  NttGeom g{ctx.primes_dev(), (uint32_t)ctx.L(), 0};
-  ntt_inverse_any(ctx.logn, g, polys, SrcPoly{src}, DstPoly{dst}, st);
+  ntt_inverse_any(ctx.logn, ntt_geom(ctx), polys, SrcWords{src}, DstPoly{dst}, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -409,7 +489,7 @@ void poly_switch_down_ntt(const Context& ctx, PolyRef in, PolyRef out, uint64_t 
   SwitchConsts c = switch_consts(ctx);
   if (polys == 0) return;
   ntt_backward(ctx, in, in, polys, st);
-  NttGeom g{ctx.primes_dev(), c.lm1, 0};
+  const NttGeom g = ntt_geom(ctx, 0, c.lm1);
   ntt_forward_any<true>(ctx.logn, g, polys, SrcSwitchDown{in, c}, DstPoly{out}, st);
 }
 
@@ -447,7 +527,7 @@ void scaler_scale(const Scaler& s, bool ntt, PolyRef in, PolyRef out, uint64_t p
   rns_scale(*s.rns, logn, src, dst, (uint32_t)ncm, (uint32_t)(Lt - ncm), polys, st);
   if (ntt) {  // rq/scaler.rs:96-114: forward NTT of the new limbs.
     // The target context restricted to limbs ncm.. : same tables, offset primes.
-    NttGeom g{s.to->primes_dev() + ncm, (uint32_t)(Lt - ncm), 0};
+    const NttGeom g = ntt_geom(*s.to, ncm, Lt - ncm);
     ntt_forward_any<true>(logn, g, polys, SrcPoly{dst}, DstPoly{dst}, st);
   }
 }

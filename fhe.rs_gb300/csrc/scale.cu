@@ -412,7 +412,8 @@ __device__ __forceinline__ uint64_t* scale_stage() {
 // stage buffer then lives in the dynamic shared memory, where A overlays it
 // once every thread holds its residues. SPLIT (with TC): the split form, a
 // kernel of its own so that the two-pass form carries none of its branches.
-template <int MAXF, int MAXT, bool EXACT, int TOP, bool FASTV, bool TC, bool SPLIT = false>
+// FOLD (with TOP): the transforms on either side run in fold arithmetic.
+template <int MAXF, int MAXT, bool EXACT, int TOP, bool FASTV, bool TC, bool FOLD, bool SPLIT = false>
 __global__ void __launch_bounds__(128) k_rns_scale(const __grid_constant__ RnsLaunch<MAXF, MAXT> s, uint32_t logn,
                                                    PolyRef in, PolyRef out, uint64_t total,
                                                    const DevPrime* src_primes, uint32_t src_mont,
@@ -481,7 +482,7 @@ __global__ void __launch_bounds__(128) k_rns_scale(const __grid_constant__ RnsLa
         const uint32_t item = threadIdx.x + 128 * u;
         if (item < F * G) {
           const uint32_t k = item / G, gi = item % G;
-          inv_top_stages<TOP>(x[u], src_primes[k], 1u << logn, src_mont != 0);
+          inv_top_stages<TOP, FOLD>(x[u], src_primes[k], 1u << logn, src_mont != 0);
 #pragma unroll
           for (int t = 0; t < (1 << TOP); t++) staged[(k * (1 << TOP) + t) * G + gi] = x[u][t];
         }
@@ -493,7 +494,7 @@ __global__ void __launch_bounds__(128) k_rns_scale(const __grid_constant__ RnsLa
         uint64_t x[1 << TOP];
 #pragma unroll
         for (int t = 0; t < (1 << TOP); t++) x[t] = row[(uint64_t)t << logb];
-        inv_top_stages<TOP>(x, src_primes[k], 1u << logn, src_mont != 0);
+        inv_top_stages<TOP, FOLD>(x, src_primes[k], 1u << logn, src_mont != 0);
 #pragma unroll
         for (int t = 0; t < (1 << TOP); t++) staged[(k * (1 << TOP) + t) * G + gi] = x[t];
       }
@@ -808,7 +809,7 @@ __global__ void __launch_bounds__(128) k_rns_scale(const __grid_constant__ RnsLa
           uint64_t x[1 << TOP];
 #pragma unroll
           for (int u = 0; u < (1 << TOP); u++) x[u] = staged[(o * (1 << TOP) + u) * G + g2];
-          fwd_top_stages<TOP>(x, fe.primes[o]);
+          fwd_top_stages<TOP, FOLD>(x, fe.primes[o]);
           uint64_t* row = out.at(poly, o) + b0 + g2;
 #pragma unroll
           for (int u = 0; u < (1 << TOP); u++) row[(uint64_t)u << logb] = x[u];
@@ -826,9 +827,10 @@ __global__ void __launch_bounds__(128) k_rns_scale(const __grid_constant__ RnsLa
 #pragma unroll
           for (int u = 0; u < (1 << TOP); u++) {
             const uint64_t v = staged[(d * (1 << TOP) + u) * G + g2];
-            x[u] = fe.digit_raw ? v : reduce64_lazy(v, kp);
+            if constexpr (FOLD) x[u] = (uint64_t)fold_lift(v, kp);
+            else x[u] = fe.digit_raw ? v : reduce64_lazy(v, kp);
           }
-          fwd_top_stages<TOP>(x, kp);
+          fwd_top_stages<TOP, FOLD>(x, kp);
           uint64_t* row = fe.digits.at(pbase + d, j) + b0 + g2;
 #pragma unroll
           for (int u = 0; u < (1 << TOP); u++) row[(uint64_t)u << logb] = x[u];
@@ -877,7 +879,7 @@ static size_t tc_prepare(const void* kern, size_t operands) {
   return a.sharedSizeBytes;
 }
 
-template <int MAXF, int MAXT, bool EXACT = false, int TOP = 0>
+template <int MAXF, int MAXT, bool EXACT = false, int TOP = 0, bool FOLD = false>
 void launch_rns_scale(const RnsScalerD& sc, uint32_t logn, PolyRef in, PolyRef out, uint32_t start,
                       uint32_t out_len, uint64_t total, cudaStream_t st, const InverseTop* top = nullptr,
                       const ForwardTop* fwd = nullptr) {
@@ -942,7 +944,7 @@ void launch_rns_scale(const RnsScalerD& sc, uint32_t logn, PolyRef in, PolyRef o
       if (sc.tc_mat.ptr && rns_tc_enabled() && n1 <= 128 && (TOP > 0 || total % 128 == 0)) {
         constexpr uint32_t KP = (8 * MAXF + 15) / 16 * 16;
         if (sc.tc_kp != KP) throw Error(FHEG_ERR_INTERNAL, "tensor-core scaler matrix of another width");
-        auto kern = k_rns_scale<MAXF, MAXT, EXACT, TOP, false, true>;
+        auto kern = k_rns_scale<MAXF, MAXT, EXACT, TOP, false, true, FOLD>;
         // The stage buffer (TOP > 0) overlaid by A, then B (the larger pass).
         constexpr size_t kStage = TOP > 0 ? (size_t)(MAXF > MAXT ? MAXF : MAXT) * 128 * 8 : 0;
         constexpr size_t kBOff = ((128 * KP * 2 > kStage ? 128 * KP * 2 : kStage) + 127) / 128 * 128;
@@ -968,7 +970,7 @@ void launch_rns_scale(const RnsScalerD& sc, uint32_t logn, PolyRef in, PolyRef o
         if constexpr (MAXT > 8 && MAXF > 16) {
           if (!h.is_one && n >= 2) {
             const uint32_t chunk = (n + 1) / 2, s1 = (8 * chunk + 15) / 16 * 16, s2 = (8 * (n - chunk) + 15) / 16 * 16;
-            auto skern = k_rns_scale<MAXF, MAXT, EXACT, TOP, false, true, true>;
+            auto skern = k_rns_scale<MAXF, MAXT, EXACT, TOP, false, true, FOLD, true>;
             const size_t sstat = tc_prepare(reinterpret_cast<const void*>(skern), kBOff + 128 * 2 * KP);
             const size_t sdyn = std::max<size_t>(kBOff + (size_t)std::max(32u, s1) * 2 * KP,
                                                  128 * kTcSmemPerColumn - 1024 - sstat);
@@ -994,9 +996,21 @@ void launch_rns_scale(const RnsScalerD& sc, uint32_t logn, PolyRef in, PolyRef o
     // The kept-high-word sums for the source counts of the default
     // extensions (L = 3, 6, 12); correct for any scaler, faster for these.
     constexpr bool kFastV = EXACT && (MAXF == 3 || MAXF == 6 || MAXF == 12);
-    k_rns_scale<MAXF, MAXT, EXACT, TOP, kFastV, false><<<blocks_for(total, threads), threads, 0, st>>>(
+    k_rns_scale<MAXF, MAXT, EXACT, TOP, kFastV, false, FOLD><<<blocks_for(total, threads), threads, 0, st>>>(
         s, logn, in, o, total, top ? top->primes : nullptr, top ? top->mont : 0u, fe, TcMat{});
     after_launch("k_rns_scale");
+  }
+}
+
+template <int MAXF, int MAXT, bool FOLD>
+static void launch_rns_scale_top_as(const RnsScalerD& s, uint32_t logn, PolyRef in, PolyRef out, uint32_t start,
+                                 uint32_t out_len, uint64_t total, cudaStream_t st, const InverseTop& top,
+                                 const ForwardTop* fwd) {
+  switch (top.s1) {
+    case 1: launch_rns_scale<MAXF, MAXT, true, 1, FOLD>(s, logn, in, out, start, out_len, total, st, &top, fwd); break;
+    case 2: launch_rns_scale<MAXF, MAXT, true, 2, FOLD>(s, logn, in, out, start, out_len, total, st, &top, fwd); break;
+    case 3: launch_rns_scale<MAXF, MAXT, true, 3, FOLD>(s, logn, in, out, start, out_len, total, st, &top, fwd); break;
+    default: throw Error(FHEG_ERR_INTERNAL, "unsupported strided stage count");
   }
 }
 
@@ -1004,12 +1018,8 @@ template <int MAXF, int MAXT>
 static void launch_rns_scale_top(const RnsScalerD& s, uint32_t logn, PolyRef in, PolyRef out, uint32_t start,
                                  uint32_t out_len, uint64_t total, cudaStream_t st, const InverseTop& top,
                                  const ForwardTop* fwd) {
-  switch (top.s1) {
-    case 1: launch_rns_scale<MAXF, MAXT, true, 1>(s, logn, in, out, start, out_len, total, st, &top, fwd); break;
-    case 2: launch_rns_scale<MAXF, MAXT, true, 2>(s, logn, in, out, start, out_len, total, st, &top, fwd); break;
-    case 3: launch_rns_scale<MAXF, MAXT, true, 3>(s, logn, in, out, start, out_len, total, st, &top, fwd); break;
-    default: throw Error(FHEG_ERR_INTERNAL, "unsupported strided stage count");
-  }
+  if (top.fold) launch_rns_scale_top_as<MAXF, MAXT, true>(s, logn, in, out, start, out_len, total, st, top, fwd);
+  else launch_rns_scale_top_as<MAXF, MAXT, false>(s, logn, in, out, start, out_len, total, st, top, fwd);
 }
 
 bool rns_scale_takes_top(const RnsScalerD& s, uint32_t logn, uint32_t out_len, uint32_t s1) {
