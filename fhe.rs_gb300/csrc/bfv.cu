@@ -1007,6 +1007,7 @@ static RotBatchPlan prepare_rot_batch(const Params& par, const RotRequest* req, 
   std::vector<uint2> rows;
   rows.reserve(cnt.n_rows + cnt.n_chain + cnt.n_add);
   size_t dpos = 0, Dpos = 0, kpos = 0, spos = 0;
+  uint32_t max_l = 0;
   for (size_t b = 0; b < count; b++) {
     const Ksk& k = *req[b].key;
     const uint32_t L = (uint32_t)k.ctx_ct->L(), Lk = (uint32_t)k.ctx_ksk->L();
@@ -1033,11 +1034,17 @@ static RotBatchPlan prepare_rot_batch(const Params& par, const RotRequest* req, 
     r.log_base = k.log_base;
     dpos += (size_t)L * N;
     Dpos += (size_t)r.nd * Lk * N;
-    for (uint32_t i = 0; i < L; i++) jobs.push_back(make_uint4((uint32_t)b, i, 0, 0));
+    max_l = std::max(max_l, std::max(L, Lk));
   }
-  for (size_t b = 0; b < count; b++)
-    for (uint32_t dd = 0; dd < desc[b].nd; dd++)
-      for (uint32_t j = 0; j < desc[b].Lk; j++) jobs.push_back(make_uint4((uint32_t)b, j, dd, 0));
+  // The jobs of the two large launches by limb: CTAs that run together then
+  // share the limb's twiddles.
+  for (uint32_t i = 0; i < max_l; i++)
+    for (size_t b = 0; b < count; b++)
+      if (i < desc[b].L) jobs.push_back(make_uint4((uint32_t)b, i, 0, 0));
+  for (uint32_t j = 0; j < max_l; j++)
+    for (size_t b = 0; b < count; b++)
+      if (j < desc[b].Lk)
+        for (uint32_t dd = 0; dd < desc[b].nd; dd++) jobs.push_back(make_uint4((uint32_t)b, j, dd, 0));
   for (size_t b = 0; b < count; b++)
     if (desc[b].ks)
       for (uint32_t part = 0; part < 2; part++)

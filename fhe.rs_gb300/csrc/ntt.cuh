@@ -48,7 +48,7 @@ namespace fheg {
 namespace {
 
 // Job decoding shared by all NTT kernels: blockIdx.x enumerates
-// (poly, limb, block) with block fastest.
+// (poly, limb, block).
 // With `jobs` set, the launch is ragged: unit u is jobs[u] = (poly, limb,
 // aux, -) instead of (u / limbs, u % limbs, 0), so one launch can cover
 // polynomials with different numbers of limbs (ciphertexts at different
@@ -56,6 +56,7 @@ namespace {
 struct NttGeom {
   const DevPrime* primes;  // one entry per limb (modulus index)
   uint32_t limbs;          // limbs per polynomial (1 for ragged launches)
+  uint32_t units;          // block kernels: polynomials (ragged: jobs) of the launch
   uint32_t s1;             // stages handled by the strided pass (0 to 4)
   const uint4* jobs;       // optional ragged job table
   uint32_t mont;           // inverse transforms: inputs carry a factor 2^-64 (Montgomery products)
@@ -172,11 +173,38 @@ __device__ __forceinline__ NttJob unit_job(const NttGeom& g, uint32_t unit) {
   return j;
 }
 
-__device__ __forceinline__ NttJob decode_job_at(const NttGeom& g, uint32_t block) {
-  uint32_t job = block;
-  const uint32_t beta = job & ((1u << g.s1) - 1);
-  NttJob j = unit_job(g, job >> g.s1);
-  j.beta = beta;
+// Block kernels take the polynomials fastest, then the blocks of a limb, then
+// the limbs: the CTAs an SM runs one after the other mostly share one block of
+// one limb, whose twiddles (64 KB) then stay in its L1. With the transposed
+// tables of the last round (fold_table_index) that took the 64
+// multiplications at N = 2^14 from 2.120 to 2.030 ms.
+__device__ __forceinline__ NttJob block_job(const NttGeom& g, uint32_t block) {
+  const uint32_t row = block / g.units, unit = block - row * g.units;
+  NttJob j;
+  if (g.jobs) {
+    j = unit_job(g, unit);
+  } else {
+    j.poly = unit;
+    j.limb = row >> g.s1;
+    j.aux = 0;
+  }
+  j.beta = row & ((1u << g.s1) - 1);
+  return j;
+}
+
+// Clusters hold the blocks of one limb: the block fastest, then the
+// polynomials, then the limbs.
+__device__ __forceinline__ NttJob cluster_job(const NttGeom& g, uint32_t block) {
+  const uint32_t u = block >> g.s1;
+  NttJob j;
+  if (g.jobs) {
+    j = unit_job(g, u);
+  } else {
+    j.limb = u / g.units;
+    j.poly = u - j.limb * g.units;
+    j.aux = 0;
+  }
+  j.beta = block & ((1u << g.s1) - 1);
   return j;
 }
 
@@ -188,17 +216,9 @@ __device__ __forceinline__ void prefetch_next(const NttGeom& g, const Src& src, 
   if (!g.pf_stride) return;
   const uint32_t nb = blockIdx.x + g.pf_stride;
   if (nb >= gridDim.x) return;
-  const NttJob jn = decode_job_at(g, nb);
+  const NttJob jn = block_job(g, nb);
   const uint32_t base = jn.beta << LOGN;
   for (uint32_t k = tid * 16; k < (1u << LOGN); k += T * 16) src_prefetch(src, jn, base + k, 0);
-}
-
-__device__ __forceinline__ NttJob decode_job(const NttGeom& g) {
-  uint32_t job = blockIdx.x;
-  const uint32_t beta = job & ((1u << g.s1) - 1);
-  NttJob j = unit_job(g, job >> g.s1);
-  j.beta = beta;
-  return j;
 }
 
 // Shared-memory swizzle: the low 4 bits of the word index are XORed with
@@ -258,13 +278,16 @@ __device__ __forceinline__ void fwd_round(uint64_t* x, uint32_t tid, const DevPr
 #pragma unroll
     for (int r = 0; r < K; r++) {
       const int half = 1 << (K - 1 - r);
-      const uint32_t tw0 = (1u << (S0 + r)) * tw_mult + (c << r);
+      // The last round of a FOLD block has its twiddles transposed
+      // (fold_table_index), so that a warp's loads are contiguous.
+      constexpr bool kLast = FOLD && S0 + K == LOGN;
+      const uint32_t tw0 = (1u << (S0 + r)) * tw_mult + (kLast ? c : c << r);
       // Constant trip counts at every level keep x[] in registers.
 #pragma unroll
       for (int t = 0; t < (1 << K); t++) {
         if (t & half) continue;
         if constexpr (FOLD) {
-          const int4 z = __ldg(pr.ftw + tw0 + (t >> (K - r)));
+          const int4 z = __ldg(pr.ftw + tw0 + (t >> (K - r)) * (kLast ? T : 1));
           if ((LOGN - 1 - S0 - r) & 1) fold_fwd_bfly<false>(xx[t], xx[t + half], z, pr);
           else fold_fwd_bfly<true>(xx[t], xx[t + half], z, pr);
         } else {
@@ -336,7 +359,7 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, NttShape<LOGN>::MIN_BLOCKS)
   constexpr int T = NttShape<LOGN>::T;
   extern __shared__ uint64_t sm[];
   const uint32_t tid = threadIdx.x;
-  const NttJob jb = decode_job(g);
+  const NttJob jb = block_job(g, blockIdx.x);
   const DevPrime pr = g.primes[jb.limb];
   const uint32_t base = jb.beta << LOGN;
   prefetch_next<LOGN, T>(g, src, tid);
@@ -383,13 +406,16 @@ __device__ __forceinline__ void inv_round(uint64_t* x, uint32_t tid, const DevPr
     for (int r = 0; r < K; r++) {
       // m_local = N_local / (2l) chunks of this block at this stage.
       const uint32_t m_local = 1u << (LOGN - 1 - U0 - r);
-      const uint32_t tw0 = n_total - (m_local << (s1 + 1)) + beta * m_local + (c << (K - 1 - r));
+      // The first round of a FOLD block has its twiddles transposed, as the
+      // last forward one.
+      constexpr bool kFirst = FOLD && U0 == 0;
+      const uint32_t tw0 = n_total - (m_local << (s1 + 1)) + beta * m_local + (kFirst ? c : c << (K - 1 - r));
       const int span = 1 << r;
 #pragma unroll
       for (int t = 0; t < (1 << K); t++) {
         if (t & span) continue;
         if constexpr (FOLD) {
-          const int4 z = __ldg(pr.fitw + tw0 + (t >> (r + 1)));
+          const int4 z = __ldg(pr.fitw + tw0 + (t >> (r + 1)) * (kFirst ? T : 1));
           if (U0 + r == 0) fold_inv_bfly<true>(xx[t], xx[t + span], z, pr);
           else fold_inv_bfly<false>(xx[t], xx[t + span], z, pr);
         } else {
@@ -451,7 +477,7 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, NttShape<LOGN>::MIN_BLOCKS)
   constexpr int K0 = InvFirst<LOGN>::K;
   extern __shared__ uint64_t sm[];
   const uint32_t tid = threadIdx.x;
-  const NttJob jb = decode_job(g);
+  const NttJob jb = block_job(g, blockIdx.x);
   const DevPrime pr = g.primes[jb.limb];
   const uint32_t base = jb.beta << LOGN;
   prefetch_next<LOGN, T>(g, src, tid);
@@ -492,7 +518,7 @@ template <bool REDUCE, class Src, class Dst>
 __global__ void __launch_bounds__(1024) k_ntt_fwd_small(NttGeom g, uint32_t logn, Src src, Dst dst) {
   extern __shared__ uint64_t sm[];
   const uint32_t n = 1u << logn, tid = threadIdx.x, nt = blockDim.x;
-  const NttJob jb = decode_job(g);
+  const NttJob jb = unit_job(g, blockIdx.x);
   const DevPrime pr = g.primes[jb.limb];
   for (uint32_t i = tid; i < n; i += nt) sm[i] = src_load<false>(src, jb, pr, i);
   __syncthreads();
@@ -515,7 +541,7 @@ template <class Src, class Dst>
 __global__ void __launch_bounds__(1024) k_ntt_inv_small(NttGeom g, uint32_t logn, Src src, Dst dst) {
   extern __shared__ uint64_t sm[];
   const uint32_t n = 1u << logn, tid = threadIdx.x, nt = blockDim.x;
-  const NttJob jb = decode_job(g);
+  const NttJob jb = unit_job(g, blockIdx.x);
   const DevPrime pr = g.primes[jb.limb];
   for (uint32_t i = tid; i < n; i += nt) sm[i] = src_load<false>(src, jb, pr, i);
   __syncthreads();
@@ -732,7 +758,7 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, NttShape<LOGN>::MIN_BLOCKS)
   extern __shared__ uint64_t sm[];
   const uint32_t tid = threadIdx.x;
   cluster_arrive_relaxed();
-  const NttJob jb = decode_job(g);  // beta = the CTA's rank in its cluster
+  const NttJob jb = cluster_job(g, blockIdx.x);  // beta = the CTA's rank in its cluster
   const DevPrime pr = g.primes[jb.limb];
   switch (g.s1) {
     case 1: fwd_cluster_top<LOGN, 1, FOLD>(src, jb, pr, sm, tid, jb.beta); break;
@@ -788,7 +814,7 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, NttShape<LOGN>::MIN_BLOCKS)
   constexpr int K0 = InvFirst<LOGN>::K;
   extern __shared__ uint64_t sm[];
   const uint32_t tid = threadIdx.x;
-  const NttJob jb = decode_job(g);
+  const NttJob jb = cluster_job(g, blockIdx.x);
   const DevPrime pr = g.primes[jb.limb];
   const uint32_t base = jb.beta << LOGN;
   uint64_t x[E];
@@ -902,6 +928,7 @@ void launch_fwd_block_as(NttGeom g, uint64_t polys, Src src, Dst dst, cudaStream
   static uint32_t resident = 0;
   g.pf_stride = ntt_prefetch_enabled() ? resident_ctas(kern, NttShape<LOGN>::T, smem, &resident) : 0;
   const uint64_t blocks = polys * g.limbs << g.s1;
+  g.units = (uint32_t)polys;
   kern<<<(unsigned)blocks, NttShape<LOGN>::T, smem, st>>>(g, src, dst);
   after_launch("k_ntt_fwd");
 }
@@ -925,6 +952,7 @@ void launch_inv_block_as(NttGeom g, uint64_t polys, Src src, Dst dst, cudaStream
   static uint32_t resident = 0;
   g.pf_stride = ntt_prefetch_enabled() ? resident_ctas(kern, NttShape<LOGN>::T, smem, &resident) : 0;
   const uint64_t blocks = polys * g.limbs << g.s1;
+  g.units = (uint32_t)polys;
   kern<<<(unsigned)blocks, NttShape<LOGN>::T, smem, st>>>(g, src, dst);
   after_launch("k_ntt_inv");
 }
@@ -997,6 +1025,7 @@ bool launch_fwd_cluster_as(NttGeom g, uint32_t s1, uint64_t polys, Src src, Dst 
   static int fits[5] = {0, 0, 0, 0, 0};
   if (!cluster_fits(kern, s1, NttShape<LOGN>::T, smem, fits)) return false;
   g.s1 = s1;
+  g.units = (uint32_t)polys;
   g.pf_stride = 0;
   launch_cluster(kern, polys * g.limbs << s1, NttShape<LOGN>::T, smem, 1u << s1, st, g, src, dst);
   after_launch("k_ntt_fwd_cl");
@@ -1020,6 +1049,7 @@ bool launch_inv_cluster_as(NttGeom g, uint32_t s1, uint64_t polys, Src src, Dst 
   static int fits[5] = {0, 0, 0, 0, 0};
   if (!cluster_fits(kern, s1, NttShape<LOGN>::T, smem, fits)) return false;
   g.s1 = s1;
+  g.units = (uint32_t)polys;
   g.pf_stride = 0;
   launch_cluster(kern, polys * g.limbs << s1, NttShape<LOGN>::T, smem, 1u << s1, st, g, src, dst);
   after_launch("k_ntt_inv_cl");

@@ -114,14 +114,35 @@ __host__ __device__ static inline int4 fold_entry(uint64_t w, uint64_t w32, uint
   return e;
 }
 
-// fold_mul's tables from the (w, Shoup) pairs: one thread per entry, w 2^32
-// mod p by a Shoup product with 2^32 mod p.
+// Where the fold tables hold twiddle i of a stage with m chunks (i < m). The
+// stages with m >= N / 16, one round of a 2^12-block whose 256 threads take m'
+// = 16 m / N consecutive twiddles each, keep every 256 m' of them transposed:
+// the threads' first ones, then their second ones, and so on (16-byte loads of
+// a warp then cover four lines instead of up to 32: 59% of the L1's
+// throughput went into them). Other stages are in the tables' own order.
+__device__ __forceinline__ uint32_t fold_table_index(uint32_t i, uint32_t m, uint32_t n) {
+  if (m < n / 16) return i;
+  const uint32_t per = 16 * m / n, group = i & ~(256 * per - 1), at = i & (256 * per - 1);
+  return group + (at % per) * 256 + at / per;
+}
+
+// fold_mul's tables from the (w, Shoup) pairs: one thread per entry of both
+// tables (forward: twiddle i of the stage with m chunks at m + i; inverse: at
+// N - 2m + i), w 2^32 mod p by a Shoup product with 2^32 mod p.
 __global__ void k_fold_tables(const ulonglong2* tw, int4* out, uint64_t p, uint64_t r32, uint64_t r32_shoup, int32_t c,
-                              int32_t k, uint32_t total) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= total) return;
-  const uint64_t w = tw[i].x;
-  out[i] = fold_entry(w, mul_shoup(w, r32, r32_shoup, p), p, c, k);
+                              int32_t k, uint32_t n) {
+  const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= 2 * n) return;
+  const uint64_t w = tw[e].x;
+  uint32_t at = e;
+  if (e > 0 && e < n) {
+    const uint32_t m = 1u << (31 - __clz(e));
+    at = m + fold_table_index(e - m, m, n);
+  } else if (e > n && e < 2 * n - 1) {  // N - 2m <= i < N - m for the largest m with N - i <= 2m
+    const uint32_t i = e - n, m = 1u << (31 - __clz(n - i - 1));
+    at = n + n - 2 * m + fold_table_index(i - (n - 2 * m), m, n);
+  }
+  out[at] = fold_entry(w, mul_shoup(w, r32, r32_shoup, p), p, c, k);
 }
 
 std::shared_ptr<PrimeTables> get_prime_tables(uint64_t p, size_t n, uint64_t root) {
@@ -140,7 +161,7 @@ std::shared_ptr<PrimeTables> get_prime_tables(uint64_t p, size_t n, uint64_t roo
   t->host = make_ntt_tables(p, n, root);
   int32_t fc = 0, fk = 0;
   uint64_t fbias = 0;
-  const bool fold = n >= 16 && fold_params(p, &fc, &fk, &fbias);
+  const bool fold = n >= 4096 && fold_params(p, &fc, &fk, &fbias);
   t->tables.alloc((fold ? 8 : 4) * n * sizeof(uint64_t));
   std::vector<uint64_t> inter(4 * n);
   for (size_t i = 0; i < n; i++) {
@@ -178,7 +199,7 @@ std::shared_ptr<PrimeTables> get_prime_tables(uint64_t p, size_t n, uint64_t roo
     int4* ft = reinterpret_cast<int4*>(d + 4 * n);
     const uint64_t r32 = (1ull << 32) % p;
     k_fold_tables<<<(unsigned)((2 * n + 255) / 256), 256>>>(dp.tw, ft, p, r32, shoup(r32, p), fc, fk,
-                                                            (uint32_t)(2 * n));
+                                                            (uint32_t)n);
     after_launch("k_fold_tables");
     check_cuda(cudaStreamSynchronize(nullptr), "cudaStreamSynchronize");
     dp.ftw = ft;
