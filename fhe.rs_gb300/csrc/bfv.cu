@@ -1155,7 +1155,8 @@ std::unique_ptr<Multiplicator> make_multiplicator(const Params& par, size_t leve
       if (ext[i] == m->base->moduli[k]) roots[i] = m->base->primes[k]->host.root;
   m->mul = std::make_shared<Context>(ext, par.degree, roots.data());
   m->ext_lhs.reset(new Scaler(m->base, m->mul, lhs_n, lhs_d));
-  m->ext_rhs.reset(new Scaler(m->base, m->mul, rhs_n, rhs_d));
+  if (lhs_n == rhs_n && lhs_d == rhs_d) m->ext_rhs = m->ext_lhs;
+  else m->ext_rhs.reset(new Scaler(m->base, m->mul, rhs_n, rhs_d));
   m->down.reset(new Scaler(m->mul, m->base, post_n, post_d));
   if (m->down->number_common_moduli != 0)
     throw Error(FHEG_ERR_UNSUPPORTED, "a post-multiplication scaling factor of one is not supported");
@@ -1247,18 +1248,6 @@ void Multiplicator::multiply(const uint64_t* lhs, const uint64_t* rhs, uint64_t*
   PolyRef pbref = plain_ref(pb, L, logn);
   PolyRef extref = plain_ref(ext, M, logn);
 
-  // Strided last stages of a two-pass inverse NTT that the RNS scaler after
-  // it can apply while loading (its only consumer): 0 when the plan is single
-  // pass or the scaler cannot.
-  auto top_stages = [&](uint32_t plan, const Scaler& s1c, const Scaler* s2c, uint32_t out_len) -> uint32_t {
-    const uint32_t bl = plan ? plan : ntt_block_logn(logn);
-    if (bl >= logn || logn < 13) return 0;
-    const uint32_t s1 = logn - bl;
-    if (!rns_scale_takes_top(*s1c.rns, logn, out_len, s1)) return 0;
-    if (s2c && !rns_scale_takes_top(*s2c->rns, logn, out_len, s1)) return 0;
-    return s1;
-  };
-
   // One arithmetic for every transform (the scaler kernels pass lazy values
   // from one to the next): the fold form when every modulus involved has it.
   const bool fold = mc.fold && bc.fold && (!rk || rk->ctx_ksk->fold);
@@ -1268,6 +1257,19 @@ void Multiplicator::multiply(const uint64_t* lhs, const uint64_t* rhs, uint64_t*
     return g;
   };
   const uint32_t bl_a = plan_a ? plan_a : ntt_block_logn(logn), bl_d = plan_d ? plan_d : ntt_block_logn(logn);
+
+  // Strided last stages of a two-pass inverse NTT that the RNS scaler after
+  // it can apply while loading (its only consumer): 0 when the plan is single
+  // pass or the scaler cannot.
+  auto top_stages = [&](uint32_t plan, const Scaler& s1c, const Scaler* s2c, uint32_t out_len) -> uint32_t {
+    const uint32_t bl = plan ? plan : ntt_block_logn(logn);
+    if (bl >= logn || logn < 13) return 0;
+    const uint32_t s1 = logn - bl;
+    const bool folds = fold && bl == 12;
+    if (!rns_scale_takes_top(*s1c.rns, logn, out_len, s1, folds)) return 0;
+    if (s2c && !rns_scale_takes_top(*s2c->rns, logn, out_len, s1, folds)) return 0;
+    return s1;
+  };
 
   // A: inverse NTT of the four operands (without its strided last stages
   // when B applies them).

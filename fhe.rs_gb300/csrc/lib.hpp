@@ -81,6 +81,26 @@ struct Context {
   std::shared_ptr<Context> prefix(size_t count) const;
 };
 
+// The digits of w < d.p that fold_mul multiplies by (d.f_c != 0).
+int4 fold_constant(uint64_t w, const DevPrime& d);
+
+// Constants of the scaler between primes just below a power of two
+// (scale_hat.cu): what its launches copy, and its device tables.
+struct RnsHatD {
+  uint32_t maxf, maxt, kp, frac;  // kernel class, matrix width, sources with a fraction
+  std::vector<uint32_t> inv, zsh, th, c, sh;
+  std::vector<uint64_t> gneg;
+  uint32_t g1, g2;
+  uint64_t v_margin, w_margin;
+  const DevPrime* from_primes;
+  // Device tables (in `tables`): the byte matrix, three constants a source, and
+  // what the reference's own sums need.
+  const uint16_t* mat;
+  const int4* zc;
+  const void* exact;
+  DevBuf tables;
+};
+
 // rns::RnsScaler (fhe-math/src/rns/scaler.rs:51-72): the host constants and
 // the per-target-modulus values each launch copies into its parameters.
 struct RnsScalerD {
@@ -97,6 +117,7 @@ struct RnsScalerD {
   // empty when that form does not apply.
   DevBuf tc_mat;
   uint32_t tc_kp = 0;
+  std::unique_ptr<RnsHatD> hat;  // null where scale_hat.cu does not apply
   RnsScalerD(const Context& from, const Context& to, const BigUint& num, const BigUint& den);
 
  private:
@@ -169,7 +190,15 @@ void rns_scale(const RnsScalerD& s, uint32_t logn, PolyRef in, PolyRef out, uint
 bool rns_tc_enabled();
 void set_rns_tc(bool on);
 uint64_t rns_tc_wait_failures();
-bool rns_scale_takes_top(const RnsScalerD& s, uint32_t logn, uint32_t out_len, uint32_t s1);
+bool rns_scale_takes_top(const RnsScalerD& s, uint32_t logn, uint32_t out_len, uint32_t s1, bool fold);
+// The scaler of scale_hat.cu (s.hat set, out_len <= s.hat->maxt, logn >= 7) and
+// its construction (null where it does not apply).
+void rns_scale_hat(const RnsScalerD& s, uint32_t logn, PolyRef in, PolyRef out, uint32_t start, uint32_t out_len,
+                   uint64_t polys, cudaStream_t st, const InverseTop* top, const ForwardTop* fwd);
+std::unique_ptr<RnsHatD> make_rns_hat(const Context& from, const Context& to, const RnsScalerHost& host,
+                                      const std::vector<uint64_t>& gneg, const std::vector<uint64_t>& gneg_hi,
+                                      const BigUint& num, const BigUint& den);
+uint64_t hat_wait_failures();
 // Scaler::scale. `scratch` must hold polys * max(L_from, L_to) * N words.
 void scaler_scale(const Scaler& s, bool ntt, PolyRef in, PolyRef out, uint64_t polys, uint64_t* scratch,
                   cudaStream_t st);
@@ -287,7 +316,8 @@ struct Multiplicator {
   const Params* par = nullptr;
   size_t level = 0;
   std::shared_ptr<Context> base, mul;
-  std::unique_ptr<Scaler> ext_lhs, ext_rhs, down;
+  std::shared_ptr<Scaler> ext_lhs, ext_rhs;  // the same one when their factors are equal
+  std::unique_ptr<Scaler> down;
   const Ksk* rk = nullptr;
   bool mod_switch = false;
   // NTT block sizes of the stages (0 = the process-wide plan): A inverse of

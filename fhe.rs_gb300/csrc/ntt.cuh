@@ -614,36 +614,52 @@ __global__ void __launch_bounds__(256) k_ntt_fwd_top(NttGeom g, uint32_t logb, u
   for (int t = 0; t < (1 << S1); t++) dst(jb, pr, b + ((uint32_t)t << logb), x[t]);
 }
 
+// The FOLD form, with the last constants as digits: zn = N^-1 and zl =
+// zetas_inv[N - 2] N^-1, both possibly times a factor of the caller's. Inputs
+// within 0.625 units; outputs canonical, or (CANON false) non-negative and at
+// most a few c above 2^k.
+template <bool CANON>
+__device__ __forceinline__ uint64_t fold_out(int64_t x, const DevPrime& pr) {
+  if constexpr (CANON) return fold_canon(x, pr);
+  else return (uint64_t)fold_lift((uint64_t)x + pr.f_bias, pr);
+}
+
+template <int S1, bool CANON>
+__device__ __forceinline__ void inv_top_fold(uint64_t* x, const DevPrime& pr, uint32_t n_total, const int4& zn,
+                                             const int4& zl) {
+#pragma unroll
+  for (int r = 0; r < S1 - 1; r++) {
+    const int span = 1 << r;
+    const uint32_t m = 1u << (S1 - 1 - r);  // chunks at this stage
+#pragma unroll
+    for (int k = 0; k < (1 << (S1 - 1 - r)); k++) {
+      const int4 z = __ldg(pr.fitw + (n_total - 2 * m + k));
+#pragma unroll
+      for (int u = 0; u < span; u++) {
+        const int t = (k << (r + 1)) + u;
+        fold_inv_bfly<false>(x[t], x[t + span], z, pr);
+      }
+    }
+  }
+  constexpr int kSpan = 1 << (S1 - 1);
+#pragma unroll
+  for (int u = 0; u < kSpan; u++) {
+    const int64_t a = (int64_t)x[u], b = (int64_t)x[u + kSpan];
+    x[u] = fold_out<CANON>(fold_mul(a + b, zn, pr), pr);
+    x[u + kSpan] = fold_out<CANON>(fold_mul(a - b, zl, pr), pr);
+  }
+}
+
 // The last S1 inverse stages of a transform of n_total residues and its
 // final scale (N^-1, or N^-1 * 2^64 when `mont`), on the 2^S1 elements
 // x[t] = element b + t * n_total / 2^S1 of one limb: what the strided inverse
 // pass does per thread, also applied by consumers that read the block pass's
 // output directly (the RNS scaler of the multiplication).
-// FOLD: inputs within 0.625 units; no Montgomery factor.
+// FOLD: inv_top_fold; no Montgomery factor.
 template <int S1, bool FOLD>
 __device__ __forceinline__ void inv_top_stages(uint64_t* x, const DevPrime& pr, uint32_t n_total, bool mont) {
   if constexpr (FOLD) {
-#pragma unroll
-    for (int r = 0; r < S1 - 1; r++) {
-      const int span = 1 << r;
-      const uint32_t m = 1u << (S1 - 1 - r);  // chunks at this stage
-#pragma unroll
-      for (int k = 0; k < (1 << (S1 - 1 - r)); k++) {
-        const int4 z = __ldg(pr.fitw + (n_total - 2 * m + k));
-#pragma unroll
-        for (int u = 0; u < span; u++) {
-          const int t = (k << (r + 1)) + u;
-          fold_inv_bfly<false>(x[t], x[t + span], z, pr);
-        }
-      }
-    }
-    constexpr int kSpan = 1 << (S1 - 1);
-#pragma unroll
-    for (int u = 0; u < kSpan; u++) {
-      const int64_t a = (int64_t)x[u], b = (int64_t)x[u + kSpan];
-      x[u] = fold_canon(fold_mul(a + b, pr.f_ninv, pr), pr);
-      x[u + kSpan] = fold_canon(fold_mul(a - b, pr.f_zlast, pr), pr);
-    }
+    inv_top_fold<S1, true>(x, pr, n_total, pr.f_ninv, pr.f_zlast);
   } else {
 #pragma unroll
     for (int r = 0; r < S1 - 1; r++) {

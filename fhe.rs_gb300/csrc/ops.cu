@@ -114,6 +114,10 @@ __host__ __device__ static inline int4 fold_entry(uint64_t w, uint64_t w32, uint
   return e;
 }
 
+int4 fold_constant(uint64_t w, const DevPrime& d) {
+  return fold_entry(w, mulmod(w, (1ull << 32) % d.p, d.p), d.p, d.f_c, d.f_sh + 32);
+}
+
 // Where the fold tables hold twiddle i of a stage with m chunks (i < m). The
 // stages with m >= N / 16, one round of a 2^12-block whose 256 threads take m'
 // = 16 m / N consecutive twiddles each, keep every 256 m' of them transposed:
@@ -200,15 +204,16 @@ std::shared_ptr<PrimeTables> get_prime_tables(uint64_t p, size_t n, uint64_t roo
     const uint64_t r32 = (1ull << 32) % p;
     k_fold_tables<<<(unsigned)((2 * n + 255) / 256), 256>>>(dp.tw, ft, p, r32, shoup(r32, p), fc, fk,
                                                             (uint32_t)n);
+    // Complete before any use: every context uploads its primes after this,
+    // on the same stream.
     after_launch("k_fold_tables");
-    check_cuda(cudaStreamSynchronize(nullptr), "cudaStreamSynchronize");
     dp.ftw = ft;
     dp.fitw = ft + n;
-    dp.f_ninv = fold_entry(dp.ninv, mulmod(dp.ninv, r32, p), p, fc, fk);
-    dp.f_zlast = fold_entry(dp.zlast_ninv, mulmod(dp.zlast_ninv, r32, p), p, fc, fk);
     dp.f_bias = fbias;
     dp.f_c = fc;
     dp.f_sh = fk - 32;
+    dp.f_ninv = fold_constant(dp.ninv, dp);
+    dp.f_zlast = fold_constant(dp.zlast_ninv, dp);
   }
   registry[key] = t;
   return t;

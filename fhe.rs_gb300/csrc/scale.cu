@@ -8,11 +8,7 @@
 #include <mutex>
 #include <vector>
 
-#include <cuda_fp16.h>
-
-#include "lib.hpp"
-#include "ntt.cuh"
-#include "tc.cuh"
+#include "scale.cuh"
 
 namespace fheg {
 
@@ -27,42 +23,6 @@ static unsigned blocks_for(uint64_t total, unsigned threads) { return (unsigned)
 // and each output residue is one exact dot product reduced once:
 //   y_j = sum_k r_k * omega_jk + v_j * (q_j - gamma_j) + w_term  (mod q_j),
 // which equals the reference's lazily reduced sum modulo q_j.
-
-__device__ __forceinline__ uint64_t join(uint32_t lo, uint32_t hi) { return ((uint64_t)hi << 32) | lo; }
-
-// Low 128 bits of (w >> s) for an nw-word little-endian value (32-bit words).
-__device__ __forceinline__ void shr_words(const uint32_t* w, int nw, uint32_t s, uint64_t* lo, uint64_t* hi) {
-  uint32_t o[4];
-  const uint32_t ws = s >> 5, bs = s & 31;
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const uint32_t idx = ws + k;
-    uint32_t a = 0, b = 0;
-#pragma unroll
-    for (int m = 0; m < 8; m++) {
-      if (m < nw && (uint32_t)m == idx) a = w[m];
-      if (m < nw && (uint32_t)m == idx + 1) b = w[m];
-    }
-    o[k] = bs ? ((a >> bs) | (b << (32 - bs))) : a;
-  }
-  *lo = join(o[0], o[1]);
-  *hi = join(o[2], o[3]);
-}
-
-// 256-bit a += b, a -= b (32-bit words).
-__device__ __forceinline__ void add256w(uint32_t* a, const uint32_t* b) {
-  asm("add.cc.u32 %0, %0, %8;\n\taddc.cc.u32 %1, %1, %9;\n\taddc.cc.u32 %2, %2, %10;\n\taddc.cc.u32 %3, %3, %11;\n\t"
-      "addc.cc.u32 %4, %4, %12;\n\taddc.cc.u32 %5, %5, %13;\n\taddc.cc.u32 %6, %6, %14;\n\taddc.u32 %7, %7, %15;"
-      : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7])
-      : "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]), "r"(b[5]), "r"(b[6]), "r"(b[7]));
-}
-
-__device__ __forceinline__ void sub256w(uint32_t* a, const uint32_t* b) {
-  asm("sub.cc.u32 %0, %0, %8;\n\tsubc.cc.u32 %1, %1, %9;\n\tsubc.cc.u32 %2, %2, %10;\n\tsubc.cc.u32 %3, %3, %11;\n\t"
-      "subc.cc.u32 %4, %4, %12;\n\tsubc.cc.u32 %5, %5, %13;\n\tsubc.cc.u32 %6, %6, %14;\n\tsubc.u32 %7, %7, %15;"
-      : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7])
-      : "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]), "r"(b[5]), "r"(b[6]), "r"(b[7]));
-}
 
 // High parts of the scaler's sums. The sums only matter at bit 96 and above
 // (v needs G >> (shift - 1) with shift >= 123, w needs S >> 126), so the
@@ -174,20 +134,6 @@ __device__ __forceinline__ void sub160w(uint32_t* a, const uint32_t* b) {
       : "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]));
 }
 
-// Full 128 x 128 -> 256-bit product (32-bit words).
-__device__ __forceinline__ void mul128x128w(uint32_t* r, uint64_t alo, uint64_t ahi, uint64_t blo, uint64_t bhi) {
-#pragma unroll
-  for (int k = 0; k < 8; k++) r[k] = 0;
-  uint32_t t[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-  mac256(t, alo, blo, bhi);  // alo * b at word 0
-  uint32_t hi6[6] = {0, 0, 0, 0, 0, 0};
-  mac192(hi6, ahi, blo, bhi);  // ahi * b at word 2 (< 2^192)
-  uint32_t u[8] = {0, 0, hi6[0], hi6[1], hi6[2], hi6[3], hi6[4], hi6[5]};
-  add256w(t, u);
-#pragma unroll
-  for (int k = 0; k < 8; k++) r[k] = t[k];
-}
-
 // All constants of one launch travel in the kernel's parameter space, so
 // every multiply-add reads its constant operand straight from the constant
 // bank (fully unrolled loops give compile-time offsets). Outputs are limbs
@@ -241,16 +187,6 @@ __device__ __forceinline__ uint64_t* rns_stage_buffer() {
   __shared__ uint64_t buf[WORDS];
   return buf;
 }
-
-// Forward stages of the kernel's epilogue (ForwardTop for one launch; primes
-// null: none).
-struct FwdEpilogue {
-  const DevPrime* primes;
-  uint32_t period, take;
-  const DevPrime* digit_primes;
-  uint32_t digit_limbs, digit_raw;
-  PolyRef digits;
-};
 
 // The exact sums of the rare coefficients whose fast high-word sums sit next
 // to a rounding boundary, kept out of line so that the hot kernel body stays
@@ -326,8 +262,6 @@ struct TcMat {
 // operand copy did not complete in time); read by rns_tc_wait_failures.
 __device__ uint32_t g_tc_wait_failures;
 
-constexpr uint32_t kTcWaitTries = 1u << 20;
-
 // Thread 0: the MMAs of pass `phase` (K / 16 of them, N = n, into the
 // columns at `tmem`) once its operand B has landed (that phase of bar_b),
 // committed to bar_mma, the pass's own single-use barrier (waited at parity
@@ -353,16 +287,6 @@ __device__ __forceinline__ void tc_pass(uint32_t bar_b, uint32_t bar_mma, uint32
   }
 }
 
-// Two bytes of w (prmt selector sel) as the half2 (b0, b1): 0x64bb is the
-// FP16 value 1024 + b, less 1024.
-__device__ __forceinline__ uint32_t tc_bytes_half2(uint32_t w, uint32_t sel) {
-  uint32_t t;
-  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(t) : "r"(w), "r"(0x64646464u), "r"(sel));
-  __half2 h = *reinterpret_cast<__half2*>(&t);
-  h = __hsub2(h, __halves2half2(__ushort_as_half(0x6400), __ushort_as_half(0x6400)));
-  return *reinterpret_cast<uint32_t*>(&h);
-}
-
 // An exact FP32 integer as an integer: below 2^23 (SMALL), its mantissa after
 // adding 2^23; below 2^24, by conversion.
 template <bool SMALL>
@@ -384,13 +308,6 @@ __device__ __forceinline__ void tc_words(const uint32_t* c, uint64_t& acc, uint3
          ((uint64_t)tc_int<SMALL>(c[6]) << 16) + ((uint64_t)tc_int<SMALL>(c[7]) << 24);
   w[1] = (uint32_t)acc;
   acc >>= 32;
-}
-
-// The dynamic shared memory of a TC launch: the stage buffer, overlaid by A
-// (128 x KP FP16) once the residues are in registers, then B.
-__device__ __forceinline__ uint8_t* tc_dyn_smem() {
-  extern __shared__ __align__(128) uint8_t tc_dyn[];
-  return tc_dyn;
 }
 
 template <int WORDS, bool TC>
@@ -803,39 +720,7 @@ __global__ void __launch_bounds__(128) k_rns_scale(const __grid_constant__ RnsLa
     if (fwd_here || dig_here) {
       __syncthreads();
       const uint64_t* staged = scale_stage<(MAXF > MAXT ? MAXF : MAXT) * 128, TC>();
-      if (fwd_here) {
-        for (uint32_t item = threadIdx.x; item < s.out_len * G; item += 128) {
-          const uint32_t o = item / G, g2 = item % G;
-          uint64_t x[1 << TOP];
-#pragma unroll
-          for (int u = 0; u < (1 << TOP); u++) x[u] = staged[(o * (1 << TOP) + u) * G + g2];
-          fwd_top_stages<TOP, FOLD>(x, fe.primes[o]);
-          uint64_t* row = out.at(poly, o) + b0 + g2;
-#pragma unroll
-          for (int u = 0; u < (1 << TOP); u++) row[(uint64_t)u << logb] = x[u];
-        }
-      } else {
-        // Digit d (output limb d) in key limb j: key_switching_key.rs:227-235
-        // with rq/mod.rs:518-540, the first forward stages of its transform.
-        const uint32_t per_digit = fe.digit_limbs * G;
-        const uint32_t pbase = (poly / fe.period) * s.out_len;
-        for (uint32_t item = threadIdx.x; item < s.out_len * per_digit; item += 128) {
-          const uint32_t d = item / per_digit, rem = item - d * per_digit;
-          const uint32_t j = rem / G, g2 = rem % G;
-          const DevPrime kp = fe.digit_primes[j];
-          uint64_t x[1 << TOP];
-#pragma unroll
-          for (int u = 0; u < (1 << TOP); u++) {
-            const uint64_t v = staged[(d * (1 << TOP) + u) * G + g2];
-            if constexpr (FOLD) x[u] = (uint64_t)fold_lift(v, kp);
-            else x[u] = fe.digit_raw ? v : reduce64_lazy(v, kp);
-          }
-          fwd_top_stages<TOP, FOLD>(x, kp);
-          uint64_t* row = fe.digits.at(pbase + d, j) + b0 + g2;
-#pragma unroll
-          for (int u = 0; u < (1 << TOP); u++) row[(uint64_t)u << logb] = x[u];
-        }
-      }
+      scale_epilogue<TOP, FOLD>(staged, fwd_here, s.out_len, poly, b0, logb, out, fe);
     }
   }
 }
@@ -847,11 +732,8 @@ void set_rns_tc(bool on) { g_rns_tc.store(on, std::memory_order_relaxed); }
 uint64_t rns_tc_wait_failures() {
   uint32_t v = 0;
   check_cuda(cudaMemcpyFromSymbol(&v, g_tc_wait_failures, sizeof(v)), "cudaMemcpyFromSymbol");
-  return v;
+  return v + hat_wait_failures();
 }
-
-// 228 KB of shared memory per SM over its 512 tensor-memory columns.
-constexpr size_t kTcSmemPerColumn = 233472 / 512;
 
 // Once per tensor-core kernel and device: reads the kernel's static shared
 // memory and raises its dynamic limit to cover its largest operands
@@ -938,7 +820,7 @@ void launch_rns_scale(const RnsScalerD& sc, uint32_t logn, PolyRef in, PolyRef o
     // The tensor-core form from 12 source moduli: with fewer, its carries
     // cost about what the multiplies they replace did, and its shared memory
     // halves the CTAs per SM (6 sources: 0.40 against 0.33 ms on GB300).
-    if constexpr (EXACT && MAXF >= 12 && MAXF <= 32) {
+    if constexpr (EXACT && MAXF >= 12 && MAXF <= 32 && !FOLD) {
       const uint32_t head = h.is_one ? 3 : 7;
       const uint32_t n0 = (8 * head + 15) / 16 * 16, n1 = (8 * n + 15) / 16 * 16;
       if (sc.tc_mat.ptr && rns_tc_enabled() && n1 <= 128 && (TOP > 0 || total % 128 == 0)) {
@@ -1022,7 +904,13 @@ static void launch_rns_scale_top(const RnsScalerD& s, uint32_t logn, PolyRef in,
   else launch_rns_scale_top_as<MAXF, MAXT, false>(s, logn, in, out, start, out_len, total, st, top, fwd);
 }
 
-bool rns_scale_takes_top(const RnsScalerD& s, uint32_t logn, uint32_t out_len, uint32_t s1) {
+// Whether scale_hat.cu takes the call.
+static bool uses_hat(const RnsScalerD& s, uint32_t logn, uint32_t out_len) {
+  return s.hat && rns_tc_enabled() && out_len <= s.hat->maxt && logn >= 7;
+}
+
+bool rns_scale_takes_top(const RnsScalerD& s, uint32_t logn, uint32_t out_len, uint32_t s1, bool fold) {
+  if (fold && uses_hat(s, logn, out_len)) return s1 >= 1 && s1 <= 3;
   const size_t F = s.host.from_len;
   const bool exact = (F == 6 || F == 13 || F == 3 || F == 7) ? out_len <= 8 : (F == 12 || F == 25) && out_len <= 16;
   return exact && s.mont && s1 >= 1 && s1 <= 3 && logn >= 7;
@@ -1035,8 +923,12 @@ void rns_scale(const RnsScalerD& s, uint32_t logn, PolyRef in, PolyRef out, uint
   const size_t F = s.host.from_len;
   if (fwd && (!top || fwd->s1 != top->s1))
     throw Error(FHEG_ERR_INTERNAL, "forward strided stages need the same count of inverse ones");
+  if (uses_hat(s, logn, out_len) && (!top || top->fold)) {
+    rns_scale_hat(s, logn, in, out, start, out_len, polys, st, top, fwd);
+    return;
+  }
   if (top) {
-    if (!rns_scale_takes_top(s, logn, out_len, top->s1))
+    if (!rns_scale_takes_top(s, logn, out_len, top->s1, top->fold))
       throw Error(FHEG_ERR_INTERNAL, "RNS scaling cannot apply these strided stages");
     if (F == 6) launch_rns_scale_top<6, 8>(s, logn, in, out, start, out_len, total, st, *top, fwd);
     else if (F == 13) launch_rns_scale_top<13, 8>(s, logn, in, out, start, out_len, total, st, *top, fwd);
@@ -1100,7 +992,8 @@ RnsScalerD::RnsScalerD(const Context& from, const Context& to, const BigUint& nu
       for (int it = 0; it < 6; it++) inv *= 2 - q * inv;
       to_pinv[j] = 0 - inv;
     }
-    build_tc_matrix();
+    hat = make_rns_hat(from, to, host, gamma_neg, gamma_neg_hi, num, den);
+    if (!hat) build_tc_matrix();
   }
 }
 
