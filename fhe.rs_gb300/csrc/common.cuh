@@ -428,10 +428,12 @@ __device__ __forceinline__ int64_t fold_lift(uint64_t x, const DevPrime& pr) {
   return (int64_t)fold_madu(h >> pr.f_sh, (uint32_t)pr.f_c, pack64((uint32_t)x, h & ((1u << pr.f_sh) - 1)));
 }
 
-// The canonical residue of a lazy value: x + bias is positive and below
-// 2 * bias, so one fold leaves it below 2p (fold_params).
+// The canonical residue of a lazy value |x| <= bias: normalised it lies in
+// (-p, p) (fold_params).
 __device__ __forceinline__ uint64_t fold_canon(int64_t x, const DevPrime& pr) {
-  return csub((uint64_t)fold_lift((uint64_t)x + pr.f_bias, pr), pr.p);
+  int64_t r = fold_norm(x, pr);
+  if (r < 0) r += (int64_t)pr.p;
+  return (uint64_t)r;
 }
 
 // (hi:lo) mod p for hi:lo < 2^(2k + 1): lazy, in [0, 2^k + 2 c^2 + c]. The bits

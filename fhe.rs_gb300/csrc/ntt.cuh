@@ -488,15 +488,14 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, NttShape<LOGN>::MIN_BLOCKS)
   const uint32_t sb = swz8(tid);
   if constexpr (src_is_staged<Src>(0)) {
     src.template stage<LOGN, T, E, FOLD>(jb, pr, base, sm, tid, x);
-#pragma unroll
-    for (int e = 0; e < E; e++) sm_at(sm, sb ^ swz8(e * T)) = x[e];
   } else {
+    // Every load before the first store: in one loop each store would hold
+    // the next load back.
 #pragma unroll
-    for (int e = 0; e < E; e++) {
-      const uint32_t i = tid + e * T;
-      sm_at(sm, sb ^ swz8(e * T)) = src_load<FOLD>(src, jb, pr, base + i);
-    }
+    for (int e = 0; e < E; e++) x[e] = src_load<FOLD>(src, jb, pr, base + tid + e * T);
   }
+#pragma unroll
+  for (int e = 0; e < E; e++) sm_at(sm, sb ^ swz8(e * T)) = x[e];
   __syncthreads();
   inv_from_smem<LOGN, 0, K0>(x, sm, tid);
   inv_rounds<LOGN, 0, K0, FOLD>(x, sm, tid, pr, 1u << (LOGN + g.s1), g.s1, jb.beta);
@@ -837,12 +836,12 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, NttShape<LOGN>::MIN_BLOCKS)
   const uint32_t sb = swz8(tid);
   if constexpr (src_is_staged<Src>(0)) {
     src.template stage<LOGN, T, E, FOLD>(jb, pr, base, sm, tid, x);
-#pragma unroll
-    for (int e = 0; e < E; e++) sm_at(sm, sb ^ swz8(e * T)) = x[e];
   } else {
 #pragma unroll
-    for (int e = 0; e < E; e++) sm_at(sm, sb ^ swz8(e * T)) = src_load<FOLD>(src, jb, pr, base + tid + e * T);
+    for (int e = 0; e < E; e++) x[e] = src_load<FOLD>(src, jb, pr, base + tid + e * T);
   }
+#pragma unroll
+  for (int e = 0; e < E; e++) sm_at(sm, sb ^ swz8(e * T)) = x[e];
   __syncthreads();
   inv_from_smem<LOGN, 0, K0>(x, sm, tid);
   inv_rounds<LOGN, 0, K0, FOLD>(x, sm, tid, pr, 1u << (LOGN + g.s1), g.s1, jb.beta);

@@ -76,8 +76,10 @@ bool fold_params(uint64_t p, int32_t* c, int32_t* k, uint64_t* bias) {
   const unsigned __int128 most = ((unsigned __int128)5 << (bits - 2)) + ((unsigned __int128)cc << 33);
   unsigned __int128 b = p;
   while (b < most) b *= 2;
-  // x + b < 2 b: one fold must leave it below 2p.
+  // |x| <= b: normalised, x must lie in (-p, p); x + b < 2 b: one fold must
+  // leave it below 2p.
   if (b >> 63) return false;
+  if (((unsigned __int128)1 << (bits - 1)) + ((b >> bits) + 1) * cc >= (unsigned __int128)p) return false;
   if (((unsigned __int128)1 << bits) + (2 * b >> bits) * cc >= 2 * (unsigned __int128)p) return false;
   *c = (int32_t)cc;
   *k = bits;
