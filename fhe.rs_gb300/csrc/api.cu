@@ -171,7 +171,7 @@ FHEG_API int fheg_ntt_cluster_set(uint32_t logn, int on) {
 FHEG_API int fheg_ntt_cluster_get(uint32_t logn, int* on) {
   return abi_call([&] {
     abi_need(on && logn <= 16, "bad size or null output");
-    *on = ntt_cluster_enabled(logn) ? 1 : 0;
+    *on = ntt_cluster_enabled(logn, false) ? 1 : 0;
   });
 }
 
@@ -212,13 +212,13 @@ uint32_t autotune_plans(uint32_t logn, cudaStream_t st, F run) {
       if (bl == 12 && bl < logn) plans.push_back({bl, true});
     }
   const uint32_t before = ntt_block_logn(logn);
-  const bool before_cluster = ntt_cluster_enabled(logn);
+  const int before_cluster = ntt_cluster_state(logn);
   if (plans.empty()) return before;
   cudaEvent_t e0, e1;
   check_cuda(cudaEventCreate(&e0), "cudaEventCreate");
   check_cuda(cudaEventCreate(&e1), "cudaEventCreate");
   float best_ms = 0;
-  std::pair<uint32_t, bool> best{before, before_cluster};
+  std::pair<uint32_t, bool> best{before, false};
   try {
     for (const auto& plan : plans) {
       set_ntt_block_logn(logn, plan.first);
@@ -238,7 +238,7 @@ uint32_t autotune_plans(uint32_t logn, cudaStream_t st, F run) {
     }
   } catch (...) {
     set_ntt_block_logn(logn, before);
-    set_ntt_cluster(logn, before_cluster);
+    restore_ntt_cluster(logn, before_cluster);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     throw;

@@ -590,7 +590,7 @@ void ntt_forward_into(uint32_t logn, NttGeom g, uint64_t polys, PolyRef inplace,
     ntt_fwd_single<true>(logn, g, polys, SrcPoly{inplace}, dst, st);
     return;
   }
-  if (bl == 12 && ntt_cluster_enabled(logn) &&
+  if (bl == 12 && ntt_cluster_enabled(logn, g.fold) &&
       launch_fwd_cluster<12, true>(g, logn - bl, polys, SrcPoly{inplace}, dst, st))
     return;
   launch_fwd_top<true>(logn - bl, g, bl, polys, SrcPoly{inplace}, DstPoly{inplace}, st);

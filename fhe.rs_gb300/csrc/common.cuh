@@ -72,8 +72,12 @@ std::vector<uint32_t> ntt_plans(uint32_t logn);
 // Whether two-pass plans with 2^12-residue blocks run instead as one pass on
 // clusters of 2^(logn - 12) CTAs exchanging through distributed shared
 // memory (fheg_ntt_cluster_set).
-bool ntt_cluster_enabled(uint32_t logn);
+// `fold`: the transform runs in fold arithmetic.
+bool ntt_cluster_enabled(uint32_t logn, bool fold);
 void set_ntt_cluster(uint32_t logn, bool on);
+// The setting itself (-1: never set), and putting it back.
+int ntt_cluster_state(uint32_t logn);
+void restore_ntt_cluster(uint32_t logn, int state);
 
 inline void check_cuda(cudaError_t e, const char* what) {
   if (e != cudaSuccess) throw Error(10 /*FHEG_ERR_CUDA*/, std::string(what) + ": " + cudaGetErrorString(e));

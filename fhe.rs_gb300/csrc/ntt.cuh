@@ -255,6 +255,13 @@ struct NttShape {
   static constexpr int T = N / E;
   // Blocks per SM the register budget must allow: 3 for 2^12 blocks, else
   // at least 512 threads' worth (a 128-register budget).
+  // The FOLD kernels with long waits of their own, clusters and the staged
+  // tensor product, gain from a fourth block under 64 registers (a few words
+  // spilled): 2^14 x 6 x 256 forward 233 -> 219 us and inverse 246 -> 239, 2^15
+  // x 6 x 128 259 -> 238 and 282 -> 254, the tensor product's inverse 364 -> 356.
+  // The plain FOLD block kernels lose 2-5% that way (2^12 x 6 x 512 forward 93
+  // -> 97, inverse 109 -> 115).
+  static constexpr int FOLD_BLOCKS = LOGN == 12 ? 4 : 1;
   static constexpr int MIN_BLOCKS = LOGN == 12 ? 3 : (T >= 512 ? 1 : (512 / T > 32 ? 32 : 512 / T));
 };
 
@@ -471,7 +478,9 @@ __device__ __forceinline__ void inv_rounds(uint64_t* x, uint64_t* sm, uint32_t t
 // With g.s1 = 0 this is the whole `backward`, including the N^-1 scaling
 // (FINAL). With g.s1 > 0 the remaining stages run in ntt_inv_top.
 template <int LOGN, bool FINAL, bool FOLD, class Src, class Dst>
-__global__ void __launch_bounds__(NttShape<LOGN>::T, NttShape<LOGN>::MIN_BLOCKS) k_ntt_inv(NttGeom g, Src src, Dst dst) {
+__global__ void __launch_bounds__(NttShape<LOGN>::T, FOLD && src_is_montgomery<Src>(0) && src_is_staged<Src>(0)
+                                                          ? NttShape<LOGN>::FOLD_BLOCKS
+                                                          : NttShape<LOGN>::MIN_BLOCKS) k_ntt_inv(NttGeom g, Src src, Dst dst) {
   constexpr int E = NttShape<LOGN>::E;
   constexpr int T = NttShape<LOGN>::T;
   constexpr int K0 = InvFirst<LOGN>::K;
@@ -766,7 +775,7 @@ __device__ __forceinline__ void fwd_cluster_top(const Src& src, const NttJob& jb
 }
 
 template <int LOGN, bool REDUCE, bool FOLD, class Src, class Dst>
-__global__ void __launch_bounds__(NttShape<LOGN>::T, NttShape<LOGN>::MIN_BLOCKS)
+__global__ void __launch_bounds__(NttShape<LOGN>::T, FOLD ? NttShape<LOGN>::FOLD_BLOCKS : NttShape<LOGN>::MIN_BLOCKS)
     k_ntt_fwd_cl(NttGeom g, Src src, Dst dst) {
   constexpr int E = NttShape<LOGN>::E;
   constexpr int T = NttShape<LOGN>::T;
@@ -822,7 +831,7 @@ __device__ __forceinline__ void inv_cluster_top(const NttGeom& g, const Dst& dst
 }
 
 template <int LOGN, bool FOLD, class Src, class Dst>
-__global__ void __launch_bounds__(NttShape<LOGN>::T, NttShape<LOGN>::MIN_BLOCKS)
+__global__ void __launch_bounds__(NttShape<LOGN>::T, FOLD ? NttShape<LOGN>::FOLD_BLOCKS : NttShape<LOGN>::MIN_BLOCKS)
     k_ntt_inv_cl(NttGeom g, Src src, Dst dst) {
   constexpr int E = NttShape<LOGN>::E;
   constexpr int T = NttShape<LOGN>::T;
@@ -1173,7 +1182,7 @@ void ntt_forward_any(uint32_t logn, NttGeom g, uint64_t polys, Src src, Dst dst,
     return;
   }
   const uint32_t s1 = logn - bl;
-  if (bl == 12 && ntt_cluster_enabled(logn) && launch_fwd_cluster<12, REDUCE>(g, s1, polys, src, dst, st)) return;
+  if (bl == 12 && ntt_cluster_enabled(logn, g.fold) && launch_fwd_cluster<12, REDUCE>(g, s1, polys, src, dst, st)) return;
   launch_fwd_top<REDUCE>(s1, g, bl, polys, src, dst, st);
   g.s1 = s1;
   switch (bl) {
@@ -1221,7 +1230,7 @@ void ntt_inverse_any(uint32_t logn, NttGeom g, uint64_t polys, Src src, Dst dst,
     return;
   }
   const uint32_t s1 = logn - bl;
-  if (bl == 12 && ntt_cluster_enabled(logn) && launch_inv_cluster<12>(g, s1, polys, src, dst, st)) return;
+  if (bl == 12 && ntt_cluster_enabled(logn, g.fold) && launch_inv_cluster<12>(g, s1, polys, src, dst, st)) return;
   g.s1 = s1;
   switch (bl) {
     case 12: launch_inv_block<12, false>(g, polys, src, dst, st); break;

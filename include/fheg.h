@@ -164,7 +164,9 @@ FHEG_API int fheg_ntt_prefetch_set(int on);
  * transform runs as one pass on clusters of 2^(logn - 12) CTAs that exchange
  * the strided stages through distributed shared memory instead of a second
  * pass over device memory (GPUs that cannot run the cluster size fall back
- * to two passes). Schedules only; process-wide per logn. */
+ * to two passes). Schedules only; process-wide per logn. On by default at 2^13
+ * and 2^14, and at 2^15 for contexts whose primes lie just below powers of two;
+ * the setting reads as off at 2^15 until it is set. */
 FHEG_API int fheg_ntt_cluster_set(uint32_t logn, int on);
 FHEG_API int fheg_ntt_cluster_get(uint32_t logn, int* on);
 /* Tensor-core form of the exact RNS scalings (rns/scaler.rs:249-352 through
