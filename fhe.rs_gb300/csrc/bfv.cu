@@ -580,23 +580,6 @@ struct DstAddParts {
   }
 };
 
-// Forward NTT of `inplace` (reduced) whose final values go to `dst`; a
-// two-pass plan runs its strided pass in place first.
-template <class Dst>
-void ntt_forward_into(uint32_t logn, NttGeom g, uint64_t polys, PolyRef inplace, Dst dst, cudaStream_t st) {
-  const uint32_t bl = ntt_block_logn(logn);
-  if (bl >= logn || logn < 13) {
-    g.s1 = 0;
-    ntt_fwd_single<true>(logn, g, polys, SrcPoly{inplace}, dst, st);
-    return;
-  }
-  if (bl == 12 && ntt_cluster_enabled(logn, g.fold) &&
-      launch_fwd_cluster<12, true>(g, logn - bl, polys, SrcPoly{inplace}, dst, st))
-    return;
-  launch_fwd_top<true>(logn - bl, g, bl, polys, SrcPoly{inplace}, DstPoly{inplace}, st);
-  ntt_forward_after_top<true>(logn, g, polys, DstPoly{inplace}, dst, st, bl);
-}
-
 // The key context's (c0, c1) of `batch` key switches in `ks` ([batch][2][Lk][N],
 // Ntt; overwritten) into the power basis, down to the ciphertext context
 // (`sd`, [batch][2][L][N]), back to Ntt, plus add0 / add1, into out.
@@ -613,7 +596,7 @@ static void finish_switch_down(const Ksk& k, uint64_t* ks, uint64_t* sd, uint64_
   const NttGeom g = ntt_geom(cc);
   DstAddParts dst{out, out_poly_stride, add0, add0_poly_stride, add0_exponent, add1, add1_poly_stride,
                   (uint32_t)cc.L(), logn};
-  ntt_forward_into(logn, g, 2 * batch, sdref, dst, st);
+  ntt_forward_into(logn, g, 2 * batch, SrcPoly{sdref}, sdref, dst, st);
 }
 
 // ---------------------------------------------------------------------------

@@ -82,6 +82,17 @@ struct SrcPhase {
   __device__ __forceinline__ void prefetch(const NttJob& j, uint32_t i) const {
     for (uint32_t k = 0; k < parts; k++) prefetch_l2(ct.at(j.poly * parts + k, j.limb) + i);
   }
+  // c_k s^k: FOLD kernels have the cheaper reduction, and take any
+  // representative in [0, 2p) (kAnyWord).
+  static constexpr bool kAnyWord = true;
+  __device__ __forceinline__ uint64_t word(const NttJob& j, const DevPrime& pr, uint32_t i) const {
+    if (parts != 2) return (*this)(j, pr, i);
+    const uint64_t* c = ct.at(2 * j.poly, j.limb) + i;
+    const uint64_t s0 = s[((uint64_t)j.limb << logn) + i], c0 = c[0], c1 = c[ct.poly_stride];
+    uint64_t hi = 0, lo = c0;
+    mac128(hi, lo, c1, s0);
+    return fold_wide_product(hi, lo, pr);
+  }
   __device__ __forceinline__ uint64_t operator()(const NttJob& j, const DevPrime& pr, uint32_t i) const {
     const uint64_t sj = s[((uint64_t)j.limb << logn) + i];
     uint64_t acc = ct.at(j.poly * parts, j.limb)[i];
@@ -131,34 +142,38 @@ struct SrcEncrypt {
   const int64_t* e;   // [count][N]
   const uint64_t* v;  // [count][N], < t
   const ulonglong2* delta;  // (Delta_j, Shoup) per limb
-  uint64_t t, q_mod_t;
+  uint64_t t, q_mod_t, q_mod_t_shoup;
   uint32_t logn;
+  // x mod p, whose division almost no x needs.
+  __device__ __forceinline__ static uint64_t mod(uint64_t x, uint64_t p) { return x < p ? x : x % p; }
   __device__ __forceinline__ uint64_t operator()(const NttJob& j, const DevPrime& pr, uint32_t i) const {
     const uint64_t k = ((uint64_t)j.poly << logn) + i;
-    const uint64_t m = (uint64_t)(((unsigned __int128)v[k] * q_mod_t) % t);
+    // v (Q mod t) mod t by a Shoup product with Q mod t. For t of 2^63 or more,
+    // whose lazy products could overflow, by division.
+    const uint64_t m = t >> 63 ? (uint64_t)(((unsigned __int128)v[k] * q_mod_t) % t)
+                               : mul_shoup(v[k], q_mod_t, q_mod_t_shoup, t);
     const int64_t ei = e[k];
-    const uint64_t ev = ei >= 0 ? (uint64_t)ei % pr.p : (pr.p - (uint64_t)(-(ei + 1)) % pr.p - 1);
+    const uint64_t ev = ei >= 0 ? mod((uint64_t)ei, pr.p) : pr.p - mod((uint64_t)(-(ei + 1)), pr.p) - 1;
     const ulonglong2 d = delta[j.limb];
-    return add_mod(ev, mul_shoup(m % pr.p, d.x, d.y, pr.p), pr.p);
+    return add_mod(ev, mul_shoup(mod(m, pr.p), d.x, d.y, pr.p), pr.p);
   }
 };
 
-// b -= a s and the copy of a: ciphertext (b, a), one thread per residue.
-__global__ void k_encrypt_finish(const DevPrime* primes, uint64_t* out, const uint64_t* a, const uint64_t* s,
-                                 uint32_t limbs, uint32_t logn, uint64_t total) {
-  const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= total) return;
-  const uint32_t i = gid & ((1u << logn) - 1);
-  const uint32_t row = row_of(gid, logn);  // poly * limbs + limb
-  const uint32_t limb = row % limbs;
-  const uint64_t poly = row / limbs;
-  const DevPrime pr = primes[limb];
-  const uint64_t ai = a[gid];
-  const uint64_t as = mul_mod(ai, s[((uint64_t)limb << logn) + i], pr);
-  uint64_t* o = out + ((poly * 2 * limbs + limb) << logn) + i;
-  o[0] = sub_mod(o[0], as, pr.p);
-  o[(uint64_t)limbs << logn] = ai;
-}
+// Destination of the encryption's transform x = e + Delta m: the ciphertext
+// (x - a s, a) of polynomial j.poly.
+struct DstEncrypt {
+  uint64_t* out;      // [count][2][L][N]
+  const uint64_t* a;  // [count][L][N]
+  const uint64_t* s;  // [L][N]
+  uint32_t limbs, logn;
+  __device__ __forceinline__ void operator()(const NttJob& j, const DevPrime& pr, uint32_t i, uint64_t v) const {
+    const uint64_t row = ((uint64_t)j.limb << logn) + i, plane = (uint64_t)limbs << logn;
+    const uint64_t ai = a[j.poly * plane + row];
+    uint64_t* o = out + 2 * j.poly * plane + row;
+    o[0] = sub_mod(v, mul_residues(ai, s[row], pr), pr.p);
+    o[plane] = ai;
+  }
+};
 
 __global__ void k_finish(SrcFinish f, uint64_t* out, uint64_t total) {
   const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -284,13 +299,9 @@ void encrypt(const SecretKeyDev& sk, size_t level, const uint64_t* values, bool 
     v = vbuf;
   }
   const NttGeom g = ntt_geom(c);
-  ntt_forward_any<true>(logn, g, count,
-                        SrcEncrypt{e, v, reinterpret_cast<const ulonglong2*>(dbuf), t, q_mod_t, logn},
-                        DstPoly{sub_ref(out, L, logn, 2, 0, 1)}, st);
-  const uint64_t total = count * L << logn;
-  k_encrypt_finish<<<nblk(total, 256), 256, 0, st>>>(c.primes_dev(), out, a, sk.s_ntt.u64(), (uint32_t)L, logn,
-                                                     total);
-  after_launch("k_encrypt_finish");
+  const SrcEncrypt src{e, v, reinterpret_cast<const ulonglong2*>(dbuf), t, q_mod_t, shoup(q_mod_t, t), logn};
+  const DstEncrypt dst{out, a, sk.s_ntt.u64(), (uint32_t)L, logn};
+  ntt_forward_into(logn, g, count, src, sub_ref(out, L, logn, 2, 0, 1), dst, st);
 }
 
 size_t decrypt_scratch_bytes(const Params& par, size_t level, uint64_t count) {

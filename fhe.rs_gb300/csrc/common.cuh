@@ -453,6 +453,14 @@ __device__ __forceinline__ uint64_t fold_wide_product(uint64_t hi, uint64_t lo, 
   return fold_madu(n, c, pack64((uint32_t)u, (uint32_t)v & mask));
 }
 
+// a * b mod p, canonical, for residues a, b: by folds where the prime has them
+// (a branch all threads of a limb take alike), else by Barrett.
+__device__ __forceinline__ uint64_t mul_residues(uint64_t a, uint64_t b, const DevPrime& pr) {
+  const uint64_t hi = __umul64hi(a, b), lo = a * b;
+  if (pr.f_c) return fold_canon((int64_t)fold_wide_product(hi, lo, pr), pr);
+  return reduce128(hi, lo, pr);
+}
+
 // Forward butterfly (x, y) -> (x + w y, x - w y). In units of 2^62: |x| up to
 // 1.75 with NORM, up to 1.125 without it; the results stay within 1.125 and
 // 1.75. So every second stage normalises, and a transform enters and leaves

@@ -1217,6 +1217,22 @@ void ntt_forward_after_top(uint32_t logn, NttGeom g, uint64_t polys, Dst dst, cu
   ntt_forward_after_top<REDUCE>(logn, g, polys, dst, dst, st, bl);
 }
 
+// Forward NTT of `src` (reduced) whose final values go to `dst`; a two-pass
+// plan keeps the values between its passes in `tmp`.
+template <class Src, class Dst>
+void ntt_forward_into(uint32_t logn, NttGeom g, uint64_t polys, Src src, PolyRef tmp, Dst dst, cudaStream_t st) {
+  const uint32_t bl = ntt_block_logn(logn);
+  if (bl >= logn || logn < 13) {
+    g.s1 = 0;
+    ntt_fwd_single<true>(logn, g, polys, src, dst, st);
+    return;
+  }
+  if (bl == 12 && ntt_cluster_enabled(logn, g.fold) && launch_fwd_cluster<12, true>(g, logn - bl, polys, src, dst, st))
+    return;
+  launch_fwd_top<true>(logn - bl, g, bl, polys, src, DstPoly{tmp}, st);
+  ntt_forward_after_top<true>(logn, g, polys, DstPoly{tmp}, dst, st, bl);
+}
+
 // Full inverse NTT, any 3 <= logn <= 16: single pass, or the block pass into
 // `dst` followed by the strided pass in place.
 template <class Src, class Dst>
