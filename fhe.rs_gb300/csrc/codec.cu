@@ -109,10 +109,15 @@ struct SrcPhase {
 // first limb.
 struct SrcFinish {
   const uint64_t* d;  // [count][N]
-  uint64_t t, q0;
+  uint64_t t, q0, t_inv;  // t_inv = floor((2^64 - 1) / t)
   uint32_t logn;
   __device__ __forceinline__ uint64_t value(uint32_t poly, uint32_t i) const {
-    return ((d[((uint64_t)poly << logn) + i] + t) % q0) % t;
+    uint64_t x = d[((uint64_t)poly << logn) + i] + t;
+    if (x >= q0) x = x - q0 < q0 ? x - q0 : x % q0;
+    // The quotient by t, at most 2 short (x < 2^62).
+    uint64_t r = x - __umul64hi(x, t_inv) * t;
+    r = csub(r, t);
+    return csub(r, t);
   }
   __device__ __forceinline__ uint64_t operator()(const NttJob& j, const DevPrime&, uint32_t i) const {
     return value(j.poly, i);
@@ -146,7 +151,9 @@ struct SrcEncrypt {
   uint32_t logn;
   // x mod p, whose division almost no x needs.
   __device__ __forceinline__ static uint64_t mod(uint64_t x, uint64_t p) { return x < p ? x : x % p; }
-  __device__ __forceinline__ uint64_t operator()(const NttJob& j, const DevPrime& pr, uint32_t i) const {
+  static constexpr bool kAnyWord = true;
+  // In [0, 3p): FOLD kernels reduce it themselves.
+  __device__ __forceinline__ uint64_t word(const NttJob& j, const DevPrime& pr, uint32_t i) const {
     const uint64_t k = ((uint64_t)j.poly << logn) + i;
     // v (Q mod t) mod t by a Shoup product with Q mod t. For t of 2^63 or more,
     // whose lazy products could overflow, by division.
@@ -155,7 +162,10 @@ struct SrcEncrypt {
     const int64_t ei = e[k];
     const uint64_t ev = ei >= 0 ? mod((uint64_t)ei, pr.p) : pr.p - mod((uint64_t)(-(ei + 1)), pr.p) - 1;
     const ulonglong2 d = delta[j.limb];
-    return add_mod(ev, mul_shoup(mod(m, pr.p), d.x, d.y, pr.p), pr.p);
+    return ev + mul_shoup_lazy(mod(m, pr.p), d.x, d.y, pr.p);
+  }
+  __device__ __forceinline__ uint64_t operator()(const NttJob& j, const DevPrime& pr, uint32_t i) const {
+    return reduce4(word(j, pr, i), pr.p, pr.p2);
   }
 };
 
@@ -330,7 +340,7 @@ void decrypt(const SecretKeyDev& sk, size_t level, size_t parts, const uint64_t*
   // t/Q scaling; only the first plaintext-context limb is read afterwards.
   const Scaler& sc = *ps.dec[level];
   rns_scale(*sc.rns, logn, plain_ref(pb, c.L(), logn), plain_ref(d0, 1, logn), 0, 1, count, st);
-  const SrcFinish fin{d0, par.plaintext, par.moduli[0], logn};
+  const SrcFinish fin{d0, par.plaintext, par.moduli[0], par.plaintext ? ~0ull / par.plaintext : 0, logn};
   if (!simd) {
     const uint64_t total = count << logn;
     k_finish<<<nblk(total, 256), 256, 0, st>>>(fin, values, total);

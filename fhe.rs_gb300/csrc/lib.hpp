@@ -41,6 +41,23 @@ struct DevBuf {
   uint64_t* u64() const { return static_cast<uint64_t*>(ptr); }
 };
 
+// Scratch of one call in the order of its stream (cudaMallocAsync): no
+// synchronisation, and calls on other streams or threads have their own. The
+// device's default pool gives freed memory back at the next synchronisation.
+struct StreamScratch {
+  void* ptr = nullptr;
+  cudaStream_t st;
+  StreamScratch(size_t bytes, cudaStream_t s) : st(s) {
+    if (bytes) check_cuda(cudaMallocAsync(&ptr, bytes, s), "cudaMallocAsync");
+  }
+  StreamScratch(const StreamScratch&) = delete;
+  StreamScratch& operator=(const StreamScratch&) = delete;
+  ~StreamScratch() {
+    if (ptr) cudaFreeAsync(ptr, st);
+  }
+  uint64_t* u64() const { return static_cast<uint64_t*>(ptr); }
+};
+
 void upload(void* dst, const void* src, size_t bytes);
 // Sets the message returned by fheg_last_error() on this thread.
 void set_last_error(const std::string& msg);
@@ -397,7 +414,7 @@ void ciphertext_switch_down(const Params& par, size_t level, size_t parts, uint6
 // ---- wire format (serialize.cu) ----
 size_t poly_serialized_bytes(const Context& c);
 void poly_serialize(const Context& c, int representation, const uint64_t* polys, uint8_t* bytes, uint64_t count,
-                    DevBuf& scratch, cudaStream_t st);
+                    cudaStream_t st);
 void poly_deserialize(const Context& c, int representation, const uint8_t* bytes, uint64_t* polys, uint64_t count,
                       cudaStream_t st);
 

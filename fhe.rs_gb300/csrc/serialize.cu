@@ -6,6 +6,7 @@
 // (inverse NTT before packing, forward NTT after unpacking), as the
 // reference's conversion does.
 
+#include <algorithm>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -14,6 +15,7 @@
 #include "handles.hpp"
 #include "abi_call.hpp"
 #include "lib.hpp"
+#include "ntt.cuh"
 
 namespace fheg {
 
@@ -24,9 +26,7 @@ constexpr int kMaxLimbs = 64;
 struct PackLayout {
   uint32_t limbs, logn;
   uint64_t poly_bytes;  // payload of one polynomial
-  uint64_t poly_chunks;  // 8-byte chunks of one payload, counted per limb (the last of a limb may be short)
   uint64_t offset[kMaxLimbs + 1];  // byte offset of limb j within a payload
-  uint64_t chunk0[kMaxLimbs + 1];  // first chunk of limb j
   uint32_t nbits[kMaxLimbs];
   uint64_t q[kMaxLimbs];
 };
@@ -36,84 +36,116 @@ PackLayout make_layout(const Context& c) {
   PackLayout lay{};
   lay.limbs = (uint32_t)c.L();
   lay.logn = c.logn;
-  uint64_t off = 0, chunks = 0;
+  uint64_t off = 0;
   for (size_t j = 0; j < c.L(); j++) {
     uint32_t nb = 0;
     while (nb < 64 && ((c.moduli[j] - 1) >> nb)) nb++;
     lay.nbits[j] = nb;
     lay.q[j] = c.moduli[j];
     lay.offset[j] = off;
-    lay.chunk0[j] = chunks;
     const uint64_t bytes = ((uint64_t)c.N() * nb + 7) / 8;  // zq serialization_length
     off += bytes;
-    chunks += (bytes + 7) / 8;
   }
   lay.offset[c.L()] = off;
-  lay.chunk0[c.L()] = chunks;
   lay.poly_bytes = off;
-  lay.poly_chunks = chunks;
   return lay;
 }
 
-// One 8-byte chunk of a limb's packed stream per thread: bits [64c, 64c + 64)
-// gathered from the (at most 64 / nb + 2) coefficients they overlap, stored
-// as one word when the destination is aligned, else byte by byte (a limb's
-// last chunk may be short).
-__global__ void k_pack(const __grid_constant__ PackLayout lay, const PolyRef in, uint8_t* out, uint64_t total) {
-  const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= total) return;
-  const uint64_t poly = gid / lay.poly_chunks;
-  const uint64_t pos = gid - poly * lay.poly_chunks;
-  uint32_t j = 0;
-  while (j + 1 < lay.limbs && pos >= lay.chunk0[j + 1]) j++;
-  const uint64_t c = pos - lay.chunk0[j];
-  const uint64_t n = 1ull << lay.logn;
-  const uint32_t nb = lay.nbits[j];
+// Word c of a limb's packed stream: bits [64c, 64c + 64), gathered from the (at
+// most 64 / nb + 2) coefficients they overlap.
+__device__ __forceinline__ uint64_t pack_word(const uint64_t* row, uint32_t n, uint32_t nb, uint32_t c) {
   const uint64_t mask = nb == 64 ? ~0ull : ((1ull << nb) - 1);
-  const uint64_t* row = in.at((uint32_t)poly, j);
-  const uint64_t bit0 = c * 64;
-  uint64_t word = 0;
-  for (uint64_t k = bit0 / nb; k < n && k * nb < bit0 + 64; k++) {
-    const uint64_t v = row[k] & mask;
-    const int64_t sh = (int64_t)(k * nb) - (int64_t)bit0;  // position of v's bit 0 within the word
-    if (sh >= 0) word |= v << sh;
-    else word |= v >> (-sh);
-  }
-  const uint64_t limb_bytes = lay.offset[j + 1] - lay.offset[j];
-  const uint64_t nbytes = limb_bytes - c * 8 < 8 ? limb_bytes - c * 8 : 8;
-  uint8_t* dst = out + poly * lay.poly_bytes + lay.offset[j] + c * 8;
-  if (nbytes == 8 && ((uintptr_t)dst & 7) == 0) {
-    *reinterpret_cast<uint64_t*>(dst) = word;
-  } else {
-    for (uint64_t b = 0; b < nbytes; b++) dst[b] = (uint8_t)(word >> (8 * b));
-  }
+  const uint32_t bit0 = c * 64, k0 = bit0 / nb;  // n * nb < 2^23
+  uint64_t word = (row[k0] & mask) >> (bit0 - k0 * nb);
+  for (uint32_t k = k0 + 1, at = (k0 + 1) * nb - bit0; at < 64 && k < n; k++, at += nb) word |= (row[k] & mask) << at;
+  return word;
 }
 
-// One coefficient per thread: bits [k nb, k nb + nb) of the limb's stream
-// (at most 9 bytes), reduced once modulo q_j.
+// Packed payloads of whole limbs: row blockIdx.y (polynomial * limbs + limb),
+// two words of its stream per thread, stored together when the destination
+// is aligned to 16 bytes, as one word each when to 8, else byte by byte (a limb's
+// last word may be short). A grid over rows leaves no 64-bit divisions: the kernel
+// over flat indexes spent its time on them (128 polynomials of 2^14 x 6: 100 us).
+__global__ void __launch_bounds__(256) k_pack(const __grid_constant__ PackLayout lay, const PolyRef in, uint8_t* out,
+                                              uint32_t row0) {
+  const uint32_t r = row0 + blockIdx.y, poly = r / lay.limbs, j = r - poly * lay.limbs;
+  const uint32_t c = 2 * (blockIdx.x * 256 + threadIdx.x);
+  const uint32_t bytes = (uint32_t)(lay.offset[j + 1] - lay.offset[j]);
+  if (c * 8 >= bytes) return;
+  const uint32_t n = 1u << lay.logn, nb = lay.nbits[j];
+  const uint64_t* row = in.at(poly, j);
+  uint8_t* dst = out + poly * lay.poly_bytes + lay.offset[j] + (uint64_t)c * 8;
+  const uint64_t w0 = pack_word(row, n, nb, c), w1 = c * 8 + 8 < bytes ? pack_word(row, n, nb, c + 1) : 0;
+  if (c * 8 + 16 <= bytes && ((uintptr_t)dst & 15) == 0) {
+    *reinterpret_cast<ulonglong2*>(dst) = make_ulonglong2(w0, w1);
+    return;
+  }
+  if (c * 8 + 16 <= bytes && ((uintptr_t)dst & 7) == 0) {
+    reinterpret_cast<uint64_t*>(dst)[0] = w0;
+    reinterpret_cast<uint64_t*>(dst)[1] = w1;
+    return;
+  }
+  const uint32_t left = bytes - c * 8 < 16 ? bytes - c * 8 : 16;
+  for (uint32_t b = 0; b < left; b++) dst[b] = (uint8_t)((b < 8 ? w0 : w1) >> (8 * (b & 7)));
+}
+
+// Coefficient k of a limb's stream of `bytes` bytes at p: bits [k nb, k nb + nb),
+// reduced once modulo q. Streams at 8-byte boundaries are read as one or two
+// words (the second only where it holds bits of the coefficient), others byte by
+// byte.
+__device__ __forceinline__ uint64_t unpack_value(const uint8_t* p, uint32_t bytes, uint32_t nb, uint64_t q, uint32_t k) {
+  const uint32_t bit = k * nb;
+  uint64_t v;
+  if ((((uintptr_t)p | bytes) & 7) == 0) {
+    const uint64_t* w = reinterpret_cast<const uint64_t*>(p) + (bit >> 6);
+    const uint32_t s = bit & 63;
+    v = w[0] >> s;
+    if (s + nb > 64) v |= w[1] << (64 - s);
+  } else {
+    const uint32_t b0 = bit >> 3, s = bit & 7;
+    uint64_t lo = 0, hi = 0;  // bytes b0 .. b0 + 8 as a 72-bit little-endian value
+#pragma unroll
+    for (int t = 0; t < 8; t++)
+      if (b0 + t < bytes) lo |= (uint64_t)p[b0 + t] << (8 * t);
+    if (b0 + 8 < bytes) hi = p[b0 + 8];
+    v = (lo >> s) | (s ? hi << (64 - s) : 0);
+  }
+  if (nb < 64) v &= (1ull << nb) - 1;
+  return v >= q ? v - q : v;
+}
+
+// One coefficient per thread.
 __global__ void k_unpack(const __grid_constant__ PackLayout lay, const uint8_t* in, const PolyRef out, uint64_t total) {
   const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= total) return;
-  const uint64_t n = 1ull << lay.logn;
-  const uint64_t k = gid & (n - 1);
+  const uint32_t k = (uint32_t)gid & ((1u << lay.logn) - 1);
   const uint32_t row = row_of(gid, lay.logn);  // poly * limbs + j
-  const uint32_t j = row % lay.limbs;
-  const uint64_t poly = row / lay.limbs;
-  const uint32_t nb = lay.nbits[j];
-  const uint8_t* p = in + poly * lay.poly_bytes + lay.offset[j];
-  const uint64_t limb_bytes = lay.offset[j + 1] - lay.offset[j];
-  const uint64_t bit = k * nb;
-  const uint64_t b0 = bit >> 3;
-  const uint32_t s = (uint32_t)(bit & 7);
-  uint64_t lo = 0, hi = 0;  // bytes b0 .. b0 + 8 as a 72-bit little-endian value
-#pragma unroll
-  for (int t = 0; t < 8; t++)
-    if (b0 + t < limb_bytes) lo |= (uint64_t)p[b0 + t] << (8 * t);
-  if (b0 + 8 < limb_bytes) hi = p[b0 + 8];
-  uint64_t v = (lo >> s) | (s ? hi << (64 - s) : 0);
-  if (nb < 64) v &= (1ull << nb) - 1;
-  out.at((uint32_t)poly, j)[k] = v >= lay.q[j] ? v - lay.q[j] : v;
+  const uint32_t poly = row / lay.limbs, j = row - poly * lay.limbs;
+  out.at(poly, j)[k] = unpack_value(in + poly * lay.poly_bytes + lay.offset[j],
+                                    (uint32_t)(lay.offset[j + 1] - lay.offset[j]), lay.nbits[j], lay.q[j], k);
 }
+
+// The payloads as the source of a forward transform: the polynomials never
+// exist in the power basis. `limbs` is the layout's per-limb part in device
+// constant space (a kernel parameter).
+struct PayloadLimbs {
+  uint32_t offset8[kMaxLimbs];  // byte offset / 8 of limb j
+  uint32_t nbits[kMaxLimbs];
+};
+struct SrcPayload {
+  static constexpr bool kAnyWord = true;
+  const uint8_t* in;
+  uint64_t poly_bytes;
+  uint32_t logn;
+  PayloadLimbs lim;
+  __device__ __forceinline__ uint64_t word(const NttJob& j, const DevPrime& pr, uint32_t i) const {
+    const uint32_t nb = lim.nbits[j.limb];
+    return unpack_value(in + j.poly * poly_bytes + (uint64_t)lim.offset8[j.limb] * 8, (nb << logn) >> 3, nb, pr.p, i);
+  }
+  __device__ __forceinline__ uint64_t operator()(const NttJob& j, const DevPrime& pr, uint32_t i) const {
+    return word(j, pr, i);
+  }
+};
 
 unsigned nblk(uint64_t total, unsigned threads) { return (unsigned)((total + threads - 1) / threads); }
 
@@ -132,9 +164,14 @@ void pack_polys(const Context& c, int representation, PolyRef in, uint8_t* bytes
     src = plain_ref(tmp, c.L(), c.logn);
     ntt_backward(c, in, src, count, st);
   }
-  const uint64_t total = count * lay.poly_chunks;
-  k_pack<<<nblk(total, 256), 256, 0, st>>>(lay, src, bytes, total);
-  after_launch("k_pack");
+  uint64_t longest = 0;
+  for (uint32_t j = 0; j < lay.limbs; j++) longest = std::max(longest, lay.offset[j + 1] - lay.offset[j]);
+  const uint64_t rows = count * lay.limbs;
+  for (uint64_t r = 0; r < rows; r += 65535) {  // the grid's limit along y
+    k_pack<<<dim3(nblk((longest + 15) / 16, 256), (unsigned)std::min<uint64_t>(65535, rows - r)), 256, 0, st>>>(
+        lay, src, bytes, (uint32_t)r);
+    after_launch("k_pack");
+  }
 }
 
 // Payloads back into `count` polynomials written through `out`.
@@ -142,6 +179,19 @@ void unpack_polys(const Context& c, int representation, const uint8_t* bytes, Po
                   cudaStream_t st) {
   if (count == 0) return;
   const PackLayout lay = make_layout(c);
+  // From 64 coefficients on every limb starts at a multiple of 8 bytes.
+  if (representation >= 1 && c.logn >= 12) {
+    SrcPayload src{};
+    src.in = bytes;
+    src.poly_bytes = lay.poly_bytes;
+    src.logn = c.logn;
+    for (uint32_t j = 0; j < lay.limbs; j++) {
+      src.lim.offset8[j] = (uint32_t)(lay.offset[j] / 8);
+      src.lim.nbits[j] = lay.nbits[j];
+    }
+    ntt_forward_any<true>(c.logn, ntt_geom(c), count, src, DstPoly{out}, st);
+    return;
+  }
   const uint64_t total = count * c.L() << c.logn;
   k_unpack<<<nblk(total, 256), 256, 0, st>>>(lay, bytes, out, total);
   after_launch("k_unpack");
@@ -149,11 +199,10 @@ void unpack_polys(const Context& c, int representation, const uint8_t* bytes, Po
 }
 
 void poly_serialize(const Context& c, int representation, const uint64_t* polys, uint8_t* bytes, uint64_t count,
-                    DevBuf& scratch, cudaStream_t st) {
+                    cudaStream_t st) {
   if (count == 0) return;
-  if (representation >= 1) scratch.reserve(count * c.L() * c.N() * 8);
-  pack_polys(c, representation, plain_ref(const_cast<uint64_t*>(polys), c.L(), c.logn), bytes, count,
-             representation >= 1 ? scratch.u64() : nullptr, st);
+  const StreamScratch tmp(representation >= 1 ? count * c.L() * c.N() * 8 : 0, st);
+  pack_polys(c, representation, plain_ref(const_cast<uint64_t*>(polys), c.L(), c.logn), bytes, count, tmp.u64(), st);
 }
 
 void poly_deserialize(const Context& c, int representation, const uint8_t* bytes, uint64_t* polys, uint64_t count,
@@ -604,9 +653,7 @@ FHEG_API int fheg_poly_serialize(const fheg_context* ctx, int representation, co
     abi_count(count);
     abi_need(ctx && representation >= 0 && representation <= 2, "bad context or representation");
     abi_need((d_polys && d_bytes) || !count, "null input");
-    DevBuf scratch;
-    poly_serialize(*ctx->c, representation, d_polys, d_bytes, count, scratch, static_cast<cudaStream_t>(stream));
-    if (scratch.ptr) check_cuda(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)), "cudaStreamSynchronize");
+    poly_serialize(*ctx->c, representation, d_polys, d_bytes, count, static_cast<cudaStream_t>(stream));
   });
 }
 
