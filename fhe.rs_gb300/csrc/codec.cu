@@ -105,6 +105,13 @@ struct SrcPhase {
   }
 };
 
+// Divisions that almost no value needs, out of line: the transform's unrolled
+// loads would carry a copy each.
+__device__ __noinline__ uint64_t far_mod(uint64_t x, uint64_t p) { return x % p; }
+__device__ __noinline__ uint64_t far_mulmod(uint64_t a, uint64_t b, uint64_t t) {
+  return (uint64_t)(((unsigned __int128)a * b) % t);
+}
+
 // secret_key.rs:233-245: ((d + t) mod q_0) mod t of the scaled phase's
 // first limb.
 struct SrcFinish {
@@ -113,7 +120,7 @@ struct SrcFinish {
   uint32_t logn;
   __device__ __forceinline__ uint64_t value(uint32_t poly, uint32_t i) const {
     uint64_t x = d[((uint64_t)poly << logn) + i] + t;
-    if (x >= q0) x = x - q0 < q0 ? x - q0 : x % q0;
+    if (x >= q0) x = x - q0 < q0 ? x - q0 : far_mod(x, q0);
     // The quotient by t, at most 2 short (x < 2^62).
     uint64_t r = x - __umul64hi(x, t_inv) * t;
     r = csub(r, t);
@@ -150,14 +157,14 @@ struct SrcEncrypt {
   uint64_t t, q_mod_t, q_mod_t_shoup;
   uint32_t logn;
   // x mod p, whose division almost no x needs.
-  __device__ __forceinline__ static uint64_t mod(uint64_t x, uint64_t p) { return x < p ? x : x % p; }
+  __device__ __forceinline__ static uint64_t mod(uint64_t x, uint64_t p) { return x < p ? x : far_mod(x, p); }
   static constexpr bool kAnyWord = true;
   // In [0, 3p): FOLD kernels reduce it themselves.
   __device__ __forceinline__ uint64_t word(const NttJob& j, const DevPrime& pr, uint32_t i) const {
     const uint64_t k = ((uint64_t)j.poly << logn) + i;
     // v (Q mod t) mod t by a Shoup product with Q mod t. For t of 2^63 or more,
     // whose lazy products could overflow, by division.
-    const uint64_t m = t >> 63 ? (uint64_t)(((unsigned __int128)v[k] * q_mod_t) % t)
+    const uint64_t m = t >> 63 ? far_mulmod(v[k], q_mod_t, t)
                                : mul_shoup(v[k], q_mod_t, q_mod_t_shoup, t);
     const int64_t ei = e[k];
     const uint64_t ev = ei >= 0 ? mod((uint64_t)ei, pr.p) : pr.p - mod((uint64_t)(-(ei + 1)), pr.p) - 1;
