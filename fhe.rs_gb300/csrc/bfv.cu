@@ -331,6 +331,7 @@ __global__ void k_key_mac(const DevPrime* primes, const uint64_t* D, uint64_t ds
                           const uint64_t* add0, uint64_t add0_stride, uint64_t add0_e, const uint64_t* add1,
                           uint64_t add1_stride, uint64_t* out, uint64_t out_stride, uint32_t ndig, uint32_t lk,
                           uint32_t logn, uint64_t batch, uint64_t total) {
+  pdl_wait();
   const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= total) return;
   const uint32_t i = gid & ((1u << logn) - 1);
@@ -422,17 +423,9 @@ void launch_key_mac(const DevPrime* primes, PolyRef D, const uint64_t* k0, const
   if (batch == 0) return;
   if (D.grp != 1) throw Error(FHEG_ERR_INTERNAL, "key inner product: digits must be a plain array");
   const uint64_t total = batch * lk << logn;
-  if (ndig <= 8)
-    k_key_mac<1, 8><<<nblocks(total, 256), 256, 0, st>>>(primes, D.base, D.grp_stride, k0, k1, add0, add0_stride,
-                                                         add0_e, add1, add1_stride, out, out_stride, ndig, lk, logn,
-                                                         batch, total);
-  else if (ndig <= 16)
-    k_key_mac<1, 16><<<nblocks(total, 256), 256, 0, st>>>(primes, D.base, D.grp_stride, k0, k1, add0, add0_stride,
-                                                          add0_e, add1, add1_stride, out, out_stride, ndig, lk, logn,
-                                                          batch, total);
-  else
-    k_key_mac<1><<<nblocks(total, 256), 256, 0, st>>>(primes, D.base, D.grp_stride, k0, k1, add0, add0_stride, add0_e,
-                                                      add1, add1_stride, out, out_stride, ndig, lk, logn, batch, total);
+  auto kern = ndig <= 8 ? k_key_mac<1, 8> : ndig <= 16 ? k_key_mac<1, 16> : k_key_mac<1>;
+  launch_dependent(kern, dim3(nblocks(total, 256)), 256, 0, st, primes, (const uint64_t*)D.base, D.grp_stride, k0, k1, add0,
+                   add0_stride, add0_e, add1, add1_stride, out, out_stride, ndig, lk, logn, batch, total);
   after_launch("k_key_mac");
 }
 
@@ -808,6 +801,7 @@ struct DstRotD {
 // for row (poly, limb) = rows[blockIdx.y]; exact sums reduced once. Requests
 // whose key switches down write the bare sums (key context) to ks instead.
 __global__ void k_rot_mac(const DevPrime* primes, const RotDesc* d, const uint2* rows, uint32_t logn) {
+  pdl_wait();
   const uint2 row = rows[blockIdx.y];
   const RotDesc& r = d[row.x];
   const uint32_t j = row.y;
@@ -1078,7 +1072,7 @@ static void launch_rot_batch(const RotBatchPlan& pl, cudaStream_t st) {
   ntt_forward_any<true>(logn, g2, cnt.n_f, SrcRotDigit{d_desc, logn}, DstRotD{d_desc, logn}, st);
   // G: inner products and the substituted c0.
   const unsigned gx = (unsigned)((N + 255) / 256);
-  k_rot_mac<<<dim3(gx, (unsigned)cnt.n_rows), 256, 0, st>>>(top.primes_dev(), d_desc, d_rows, logn);
+  launch_dependent(k_rot_mac, dim3(gx, (unsigned)cnt.n_rows), 256, 0, st, top.primes_dev(), d_desc, d_rows, logn);
   after_launch("k_rot_mac");
   if (cnt.n_chain == 0) return;
   // Requests with keys below their level: the sums into the power basis, down

@@ -366,8 +366,10 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, NttShape<LOGN>::MIN_BLOCKS)
   constexpr int T = NttShape<LOGN>::T;
   extern __shared__ uint64_t sm[];
   const uint32_t tid = threadIdx.x;
+  if (g.jobs) pdl_wait();  // the table may be new
   const NttJob jb = block_job(g, blockIdx.x);
   const DevPrime pr = g.primes[jb.limb];
+  pdl_wait();
   const uint32_t base = jb.beta << LOGN;
   prefetch_next<LOGN, T>(g, src, tid);
   uint64_t x[E];
@@ -375,6 +377,7 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, NttShape<LOGN>::MIN_BLOCKS)
 #pragma unroll
   for (int e = 0; e < E; e++) x[e] = src_load<FOLD>(src, jb, pr, base + tid + e * T);
   fwd_rounds<LOGN, 0, FOLD>(x, sm, tid, pr, (1u << g.s1) + jb.beta);
+  pdl_trigger();
   const uint32_t sb = swz8(tid);
 #pragma unroll
   for (int e = 0; e < E; e++) {
@@ -486,8 +489,10 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, FOLD && src_is_montgomery<S
   constexpr int K0 = InvFirst<LOGN>::K;
   extern __shared__ uint64_t sm[];
   const uint32_t tid = threadIdx.x;
+  if (g.jobs) pdl_wait();  // the table may be new
   const NttJob jb = block_job(g, blockIdx.x);
   const DevPrime pr = g.primes[jb.limb];
+  pdl_wait();
   const uint32_t base = jb.beta << LOGN;
   prefetch_next<LOGN, T>(g, src, tid);
   uint64_t x[E];
@@ -508,6 +513,7 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, FOLD && src_is_montgomery<S
   __syncthreads();
   inv_from_smem<LOGN, 0, K0>(x, sm, tid);
   inv_rounds<LOGN, 0, K0, FOLD>(x, sm, tid, pr, 1u << (LOGN + g.s1), g.s1, jb.beta);
+  pdl_trigger();
   // The last round holds elements tid + e*T (b = tid, c = 0): coalesced stores.
 #pragma unroll
   for (int e = 0; e < E; e++) {
@@ -526,8 +532,10 @@ template <bool REDUCE, class Src, class Dst>
 __global__ void __launch_bounds__(1024) k_ntt_fwd_small(NttGeom g, uint32_t logn, Src src, Dst dst) {
   extern __shared__ uint64_t sm[];
   const uint32_t n = 1u << logn, tid = threadIdx.x, nt = blockDim.x;
+  if (g.jobs) pdl_wait();
   const NttJob jb = unit_job(g, blockIdx.x);
   const DevPrime pr = g.primes[jb.limb];
+  pdl_wait();
   for (uint32_t i = tid; i < n; i += nt) sm[i] = src_load<false>(src, jb, pr, i);
   __syncthreads();
   for (uint32_t s = 0; s < logn; s++) {
@@ -542,6 +550,7 @@ __global__ void __launch_bounds__(1024) k_ntt_fwd_small(NttGeom g, uint32_t logn
     }
     __syncthreads();
   }
+  pdl_trigger();
   for (uint32_t i = tid; i < n; i += nt) dst(jb, pr, i, REDUCE ? reduce4(sm[i], pr.p, pr.p2) : sm[i]);
 }
 
@@ -549,8 +558,10 @@ template <class Src, class Dst>
 __global__ void __launch_bounds__(1024) k_ntt_inv_small(NttGeom g, uint32_t logn, Src src, Dst dst) {
   extern __shared__ uint64_t sm[];
   const uint32_t n = 1u << logn, tid = threadIdx.x, nt = blockDim.x;
+  if (g.jobs) pdl_wait();
   const NttJob jb = unit_job(g, blockIdx.x);
   const DevPrime pr = g.primes[jb.limb];
+  pdl_wait();
   for (uint32_t i = tid; i < n; i += nt) sm[i] = src_load<false>(src, jb, pr, i);
   __syncthreads();
   for (uint32_t l = 1; l < n; l <<= 1) {
@@ -565,6 +576,7 @@ __global__ void __launch_bounds__(1024) k_ntt_inv_small(NttGeom g, uint32_t logn
     }
     __syncthreads();
   }
+  pdl_trigger();
   for (uint32_t i = tid; i < n; i += nt) dst(jb, pr, i, inv_final_scale(g, pr, sm[i]));
 }
 
@@ -609,6 +621,7 @@ __device__ __forceinline__ void fwd_top_stages(uint64_t* x, const DevPrime& pr) 
 template <int S1, bool FOLD, class Src, class Dst>
 __global__ void __launch_bounds__(256) k_ntt_fwd_top(NttGeom g, uint32_t logb, uint32_t groups_per_limb,
                                                      uint64_t total, Src src, Dst dst) {
+  pdl_wait();
   const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= total) return;
   const uint32_t b = (uint32_t)gid & (groups_per_limb - 1);  // groups_per_limb = 2^logb
@@ -618,6 +631,7 @@ __global__ void __launch_bounds__(256) k_ntt_fwd_top(NttGeom g, uint32_t logb, u
 #pragma unroll
   for (int t = 0; t < (1 << S1); t++) x[t] = src_load<FOLD>(src, jb, pr, b + ((uint32_t)t << logb));
   fwd_top_stages<S1, FOLD>(x, pr);
+  pdl_trigger();
 #pragma unroll
   for (int t = 0; t < (1 << S1); t++) dst(jb, pr, b + ((uint32_t)t << logb), x[t]);
 }
@@ -698,6 +712,7 @@ __device__ __forceinline__ void inv_top_stages(uint64_t* x, const DevPrime& pr, 
 template <int S1, bool FOLD, class Src, class Dst>
 __global__ void __launch_bounds__(256) k_ntt_inv_top(NttGeom g, uint32_t logb, uint32_t groups_per_limb,
                                                      uint64_t total, Src src, Dst dst) {
+  pdl_wait();
   const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= total) return;
   const uint32_t b = (uint32_t)gid & (groups_per_limb - 1);  // groups_per_limb = 2^logb
@@ -707,6 +722,7 @@ __global__ void __launch_bounds__(256) k_ntt_inv_top(NttGeom g, uint32_t logb, u
 #pragma unroll
   for (int t = 0; t < (1 << S1); t++) x[t] = src(jb, pr, b + ((uint32_t)t << logb));
   inv_top_stages<S1, FOLD>(x, pr, 1u << (logb + S1), g.mont != 0);
+  pdl_trigger();
 #pragma unroll
   for (int t = 0; t < (1 << S1); t++) dst(jb, pr, b + ((uint32_t)t << logb), x[t]);
 }
@@ -782,8 +798,10 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, FOLD ? NttShape<LOGN>::FOLD
   extern __shared__ uint64_t sm[];
   const uint32_t tid = threadIdx.x;
   cluster_arrive_relaxed();
+  if (g.jobs) pdl_wait();
   const NttJob jb = cluster_job(g, blockIdx.x);  // beta = the CTA's rank in its cluster
   const DevPrime pr = g.primes[jb.limb];
+  pdl_wait();
   switch (g.s1) {
     case 1: fwd_cluster_top<LOGN, 1, FOLD>(src, jb, pr, sm, tid, jb.beta); break;
     case 2: fwd_cluster_top<LOGN, 2, FOLD>(src, jb, pr, sm, tid, jb.beta); break;
@@ -796,6 +814,7 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, FOLD ? NttShape<LOGN>::FOLD
 #pragma unroll
   for (int e = 0; e < E; e++) x[e] = sm_at(sm, sb ^ swz8(e * T));
   fwd_rounds<LOGN, 0, FOLD>(x, sm, tid, pr, (1u << g.s1) + jb.beta);
+  pdl_trigger();
   const uint32_t base = jb.beta << LOGN;
 #pragma unroll
   for (int e = 0; e < E; e++) {
@@ -838,8 +857,10 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, FOLD ? NttShape<LOGN>::FOLD
   constexpr int K0 = InvFirst<LOGN>::K;
   extern __shared__ uint64_t sm[];
   const uint32_t tid = threadIdx.x;
+  if (g.jobs) pdl_wait();
   const NttJob jb = cluster_job(g, blockIdx.x);
   const DevPrime pr = g.primes[jb.limb];
+  pdl_wait();
   const uint32_t base = jb.beta << LOGN;
   uint64_t x[E];
   const uint32_t sb = swz8(tid);
@@ -854,6 +875,7 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, FOLD ? NttShape<LOGN>::FOLD
   __syncthreads();
   inv_from_smem<LOGN, 0, K0>(x, sm, tid);
   inv_rounds<LOGN, 0, K0, FOLD>(x, sm, tid, pr, 1u << (LOGN + g.s1), g.s1, jb.beta);
+  pdl_trigger();
   // Every thread has read its last exchange: the block's results go to
   // shared memory for the cluster.
   __syncthreads();
@@ -953,7 +975,7 @@ void launch_fwd_block_as(NttGeom g, uint64_t polys, Src src, Dst dst, cudaStream
   g.pf_stride = ntt_prefetch_enabled() ? resident_ctas(kern, NttShape<LOGN>::T, smem, &resident) : 0;
   const uint64_t blocks = polys * g.limbs << g.s1;
   g.units = (uint32_t)polys;
-  kern<<<(unsigned)blocks, NttShape<LOGN>::T, smem, st>>>(g, src, dst);
+  launch_dependent<true>(kern, dim3((unsigned)blocks), NttShape<LOGN>::T, smem, st, g, src, dst);
   after_launch("k_ntt_fwd");
 }
 
@@ -977,7 +999,7 @@ void launch_inv_block_as(NttGeom g, uint64_t polys, Src src, Dst dst, cudaStream
   g.pf_stride = ntt_prefetch_enabled() ? resident_ctas(kern, NttShape<LOGN>::T, smem, &resident) : 0;
   const uint64_t blocks = polys * g.limbs << g.s1;
   g.units = (uint32_t)polys;
-  kern<<<(unsigned)blocks, NttShape<LOGN>::T, smem, st>>>(g, src, dst);
+  launch_dependent<true>(kern, dim3((unsigned)blocks), NttShape<LOGN>::T, smem, st, g, src, dst);
   after_launch("k_ntt_inv");
 }
 
@@ -989,7 +1011,7 @@ void launch_inv_block(NttGeom g, uint64_t polys, Src src, Dst dst, cudaStream_t 
   launch_inv_block_as<LOGN, FINAL, false>(g, polys, src, dst, st);
 }
 
-// Launch of a kernel on clusters of `csize` CTAs along x.
+// Launch of a kernel on clusters of `csize` CTAs along x, as launch_dependent.
 template <class K, class... Args>
 void launch_cluster(K kern, uint64_t blocks, unsigned threads, size_t smem, unsigned csize, cudaStream_t st,
                     Args... args) {
@@ -998,13 +1020,15 @@ void launch_cluster(K kern, uint64_t blocks, unsigned threads, size_t smem, unsi
   cfg.blockDim = dim3(threads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = csize;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
   check_cuda(cudaLaunchKernelEx(&cfg, kern, args...), "cudaLaunchKernelEx");
 }
 
@@ -1099,7 +1123,8 @@ void ntt_fwd_single(uint32_t logn, NttGeom g, uint64_t polys, Src src, Dst dst, 
       if (logn < 3 || logn > 11) throw Error(12, "unsupported NTT size");
       const uint32_t threads = logn >= 11 ? 1024 : (1u << (logn - 1));
       const uint64_t blocks = polys * g.limbs;
-      k_ntt_fwd_small<REDUCE><<<(unsigned)blocks, threads, (sizeof(uint64_t) << logn), st>>>(g, logn, src, dst);
+      launch_dependent<true>(k_ntt_fwd_small<REDUCE, Src, Dst>, dim3((unsigned)blocks), threads, sizeof(uint64_t) << logn, st, g,
+                       logn, src, dst);
       after_launch("k_ntt_fwd_small");
     }
   }
@@ -1115,7 +1140,8 @@ void ntt_inv_single(uint32_t logn, NttGeom g, uint64_t polys, Src src, Dst dst, 
       if (logn < 3 || logn > 11 || !FINAL) throw Error(12, "unsupported NTT size");
       const uint32_t threads = logn >= 11 ? 1024 : (1u << (logn - 1));
       const uint64_t blocks = polys * g.limbs;
-      k_ntt_inv_small<<<(unsigned)blocks, threads, (sizeof(uint64_t) << logn), st>>>(g, logn, src, dst);
+      launch_dependent<true>(k_ntt_inv_small<Src, Dst>, dim3((unsigned)blocks), threads, sizeof(uint64_t) << logn, st, g, logn, src,
+                       dst);
       after_launch("k_ntt_inv_small");
     }
   }
@@ -1131,10 +1157,10 @@ void launch_fwd_top_as(uint32_t s1, NttGeom g, uint32_t bl, uint64_t polys, Src 
   const unsigned blocks = (unsigned)((threads + 255) / 256);
   g.s1 = 0;
   switch (s1) {
-    case 1: k_ntt_fwd_top<1, FOLD><<<blocks, 256, 0, st>>>(g, bl, groups, threads, src, dst); break;
-    case 2: k_ntt_fwd_top<2, FOLD><<<blocks, 256, 0, st>>>(g, bl, groups, threads, src, dst); break;
-    case 3: k_ntt_fwd_top<3, FOLD><<<blocks, 256, 0, st>>>(g, bl, groups, threads, src, dst); break;
-    case 4: k_ntt_fwd_top<4, FOLD><<<blocks, 256, 0, st>>>(g, bl, groups, threads, src, dst); break;
+    case 1: launch_dependent<true>(k_ntt_fwd_top<1, FOLD, Src, Dst>, dim3(blocks), 256, 0, st, g, bl, groups, threads, src, dst); break;
+    case 2: launch_dependent<true>(k_ntt_fwd_top<2, FOLD, Src, Dst>, dim3(blocks), 256, 0, st, g, bl, groups, threads, src, dst); break;
+    case 3: launch_dependent<true>(k_ntt_fwd_top<3, FOLD, Src, Dst>, dim3(blocks), 256, 0, st, g, bl, groups, threads, src, dst); break;
+    case 4: launch_dependent<true>(k_ntt_fwd_top<4, FOLD, Src, Dst>, dim3(blocks), 256, 0, st, g, bl, groups, threads, src, dst); break;
     default: throw Error(12, "unsupported NTT plan");
   }
   after_launch("k_ntt_fwd_top");
@@ -1153,10 +1179,10 @@ void launch_inv_top_as(uint32_t s1, NttGeom g, uint32_t bl, uint64_t polys, Src 
   const unsigned blocks = (unsigned)((threads + 255) / 256);
   g.s1 = 0;
   switch (s1) {
-    case 1: k_ntt_inv_top<1, FOLD><<<blocks, 256, 0, st>>>(g, bl, groups, threads, src, dst); break;
-    case 2: k_ntt_inv_top<2, FOLD><<<blocks, 256, 0, st>>>(g, bl, groups, threads, src, dst); break;
-    case 3: k_ntt_inv_top<3, FOLD><<<blocks, 256, 0, st>>>(g, bl, groups, threads, src, dst); break;
-    case 4: k_ntt_inv_top<4, FOLD><<<blocks, 256, 0, st>>>(g, bl, groups, threads, src, dst); break;
+    case 1: launch_dependent<true>(k_ntt_inv_top<1, FOLD, Src, Dst>, dim3(blocks), 256, 0, st, g, bl, groups, threads, src, dst); break;
+    case 2: launch_dependent<true>(k_ntt_inv_top<2, FOLD, Src, Dst>, dim3(blocks), 256, 0, st, g, bl, groups, threads, src, dst); break;
+    case 3: launch_dependent<true>(k_ntt_inv_top<3, FOLD, Src, Dst>, dim3(blocks), 256, 0, st, g, bl, groups, threads, src, dst); break;
+    case 4: launch_dependent<true>(k_ntt_inv_top<4, FOLD, Src, Dst>, dim3(blocks), 256, 0, st, g, bl, groups, threads, src, dst); break;
     default: throw Error(12, "unsupported NTT plan");
   }
   after_launch("k_ntt_inv_top");

@@ -245,7 +245,8 @@ __global__ void __launch_bounds__(128) k_rns_hat(const __grid_constant__ HatLaun
   const uint32_t bar_b = smem_u32(&bars[0]), bar_mma = smem_u32(&bars[1]);  // bar_mma + 8 ch: chunk ch's
   const uint32_t a_addr = smem_u32(sa), b_addr = a_addr + s.b_offset;
   const uint32_t F = s.from_len;
-  // Operand B in flight and the tensor memory allocated while the sources load.
+  // Operand B in flight and the tensor memory allocated while the kernel
+  // before ends and the sources load.
   if (threadIdx.x == 0) {
     mbar_init(bar_b, 1);
     mbar_init(bar_mma, 1);
@@ -255,6 +256,7 @@ __global__ void __launch_bounds__(128) k_rns_hat(const __grid_constant__ HatLaun
     bulk_g2s(b_addr, mat, s.out_len * 16 * KP, bar_b);
   }
   if ((threadIdx.x >> 5) == 1) tc_alloc(smem_u32(&slot), s.cols);
+  pdl_wait();
 
   const uint32_t poly = blockIdx.x >> (logn - 7), part = blockIdx.x & ((1u << (logn - 7)) - 1);
   uint32_t i, b0 = 0, logb = logn, t = 0, gi = 0;
@@ -417,6 +419,7 @@ __global__ void __launch_bounds__(128) k_rns_hat(const __grid_constant__ HatLaun
   tc_fence_before();
   __syncthreads();
   if ((threadIdx.x >> 5) == 1) tc_dealloc(tmem, s.cols);
+  pdl_trigger();
   if constexpr (TOP > 0) {
     if (fwd_here || dig_here)
       scale_epilogue<TOP, true>(reinterpret_cast<uint64_t*>(sa), fwd_here, s.out_len, poly, b0, logb, out, fe);
@@ -512,9 +515,8 @@ void launch_hat_top(const RnsScalerD& sc, uint32_t logn, PolyRef in, PolyRef out
                                   std::max<size_t>(kA + 8 * MAXT * 2 * KP, 128 * kTcSmemPerColumn));
   s.b_offset = (uint32_t)kA;
   const size_t dyn = std::max<size_t>(kA + (size_t)s.b_rows * 2 * KP, s.cols * kTcSmemPerColumn - 1024 - stat);
-  kern<<<(unsigned)(total / 128), 128, dyn, st>>>(
-      s, logn, in, out, h.from_primes, h.zc, h.mat + (size_t)start * 8 * KP, static_cast<const HatExact*>(h.exact), start,
-      fe);
+  launch_dependent(kern, dim3((unsigned)(total / 128)), 128, dyn, st, s, logn, in, out, h.from_primes, h.zc,
+                   h.mat + (size_t)start * 8 * KP, static_cast<const HatExact*>(h.exact), start, fe);
   after_launch("k_rns_hat");
 }
 
