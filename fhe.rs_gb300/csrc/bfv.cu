@@ -314,6 +314,25 @@ struct DstKsF {
   }
 };
 
+// The block passes of F in one launch, after the scale-down applied the first
+// stages: the digit rows in place, c0 and c1 from where it left them (key and
+// ciphertext limbs are the same moduli). A launch of their own for c0 and c1 costs
+// a small batch 3-6 us (one multiplication at 2^14 x 6: 77 against 73 us); beyond
+// kMaxDependentCtas CTAs two launches are 0.3-0.6% faster.
+struct KsFBlocks {
+  PolyRef D;    // poly b*L + d
+  PolyRef c01;  // poly 2b + part
+  PolyRef out;  // poly 2b + part
+  uint32_t ndig_polys;
+  __device__ __forceinline__ void operator()(const NttJob& j, const DevPrime&, uint32_t i, uint64_t v) const {
+    if (j.poly < ndig_polys) D.at(j.poly, j.limb)[i] = v;
+    else out.at(j.poly - ndig_polys, j.limb)[i] = v;
+  }
+  __device__ __forceinline__ uint64_t reload(const NttJob& j, uint32_t i) const {
+    return j.poly < ndig_polys ? D.at(j.poly, j.limb)[i] : c01.at(j.poly - ndig_polys, j.limb)[i];
+  }
+};
+
 // Key inner product for relinearization, rotations and the multiplication:
 // out_part[j] = add_part[j] + sum_d D[d][j] * key_part[d][j] (mod q_j), with
 // D and the keys canonical, so each product is below 2^124 and up to 15
@@ -1342,6 +1361,9 @@ void Multiplicator::multiply(const uint64_t* lhs, const uint64_t* rhs, uint64_t*
       // mul.rs:196-210 with key_switching_key.rs:292-329: c0, c1 into Ntt;
       // G below adds the decomposed key switch of c2.
       ntt_forward_any<true>(logn, gb, 2 * count, SrcPoly{c01}, DstPoly{oref}, st, bf);
+    } else if (fuse_f && !ks_down && ((count * L * (Lk + 2)) << top_d) <= kMaxDependentCtas) {
+      const uint32_t ndp = (uint32_t)(count * L);
+      ntt_forward_after_top<true>(logn, gk, ndp + 2 * count, KsFBlocks{dref, c01, oref, ndp}, st, bf);
     } else if (fuse_f) {
       ntt_forward_after_top<true>(logn, gk, count * L, DstPoly{dref}, st, bf);
       ntt_forward_after_top<true>(logn, gb, 2 * count, DstPoly{c01}, DstPoly{oref}, st, bf);

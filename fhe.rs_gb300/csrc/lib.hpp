@@ -349,7 +349,8 @@ struct Multiplicator {
   // degree: a few ciphertexts do not fill the GPU with whole-limb CTAs, and
   // 2^12-residue blocks cut the one-pair latency by about 30% on GB300.
   uint64_t small_count = 8;
-  uint32_t small_plan[6] = {12, 12, 12, 12, 1, 0};
+  // A single-pass F runs its digits and c0 / c1 in one launch there.
+  uint32_t small_plan[6] = {12, 12, 12, 12, 0, 0};
   Workspace ws;
   DevBuf staging;  // device copies for the host entry point
   // `marks` (optional, 8 events) are recorded on `st` at the stage
