@@ -336,46 +336,43 @@ struct KsFBlocks {
 // Key inner product for relinearization, rotations and the multiplication:
 // out_part[j] = add_part[j] + sum_d D[d][j] * key_part[d][j] (mod q_j), with
 // D and the keys canonical, so each product is below 2^124 and up to 15
-// products are summed exactly before a Barrett reduction. A thread handles
-// one residue of limb j for KB ciphertexts of the batch (each key residue is
-// then read once per KB ciphertexts).
+// products are summed exactly before a reduction. A thread handles one residue of
+// limb j for one ciphertext (sharing the key loads among 4 ciphertexts a thread
+// measured 60% slower at 64 pairs: too few threads to cover the loads of D).
 // D is a plain array [batch * ndig][lk][N] (digit d of ciphertext b at row
 // b * ndig + d, dstride words apart), addressed directly: a PolyRef lookup
 // per digit would cost a division per residue.
-// MAXD > 0 (KB = 1, ndig <= MAXD): every digit and key residue is loaded
-// before the first product, so all of a thread's loads are in flight at once.
-template <int KB, int MAXD = 0>
+// MAXD > 0 (ndig <= MAXD): every digit and key residue is loaded before the first
+// product, so all of a thread's loads are in flight at once (groups of 4 to 6
+// digits in a loop were 14% slower at 6 digits and 3% at 12).
+template <int MAXD>
 __global__ void k_key_mac(const DevPrime* primes, const uint64_t* D, uint64_t dstride, const uint64_t* k0,
-                          const uint64_t* k1,
-                          const uint64_t* add0, uint64_t add0_stride, uint64_t add0_e, const uint64_t* add1,
-                          uint64_t add1_stride, uint64_t* out, uint64_t out_stride, uint32_t ndig, uint32_t lk,
-                          uint32_t logn, uint64_t batch, uint64_t total) {
+                          const uint64_t* k1, const uint64_t* add0, uint64_t add0_stride, uint64_t add0_e,
+                          const uint64_t* add1, uint64_t add1_stride, uint64_t* out, uint64_t out_stride, uint32_t ndig,
+                          uint32_t lk, uint32_t logn, uint64_t total) {
   pdl_wait();
   const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= total) return;
   const uint32_t i = gid & ((1u << logn) - 1);
   const uint32_t job = row_of(gid, logn);
   const uint32_t j = job % lk;
-  const uint64_t b0 = (uint64_t)(job / lk) * KB;
+  const uint64_t b = job / lk;
   const DevPrime pr = primes[j];
-  uint64_t lo0[KB], hi0[KB], lo1[KB], hi1[KB];
-  const uint32_t gi = add0_e ? gather_index(i, add0_e, logn) : i;
-#pragma unroll
-  for (int u = 0; u < KB; u++) {
-    const uint64_t b = b0 + u;
-    lo0[u] = hi0[u] = lo1[u] = hi1[u] = 0;
-    if (b < batch) {
-      if (add0) lo0[u] = add0[b * add0_stride + ((uint64_t)j << logn) + gi];
-      if (add1) lo1[u] = add1[b * add1_stride + ((uint64_t)j << logn) + i];
-    }
-  }
-  const uint64_t kstride = (uint64_t)lk << logn;
-  const uint64_t* kp0 = k0 + ((uint64_t)j << logn) + i;
-  const uint64_t* kp1 = k1 + ((uint64_t)j << logn) + i;
+  const uint64_t row = ((uint64_t)j << logn) + i, kstride = (uint64_t)lk << logn;
+  uint64_t lo0 = 0, hi0 = 0, lo1 = 0, hi1 = 0;
+  if (add0) lo0 = add0[b * add0_stride + (add0_e ? ((uint64_t)j << logn) + gather_index(i, add0_e, logn) : row)];
+  if (add1) lo1 = add1[b * add1_stride + row];
+  const uint64_t* kp0 = k0 + row;
+  const uint64_t* kp1 = k1 + row;
+  const uint64_t* dp = D + b * ndig * dstride + row;
+  auto flush = [&] {  // 15 products and a residue below 2^128
+    lo0 = reduce_sum(hi0, lo0, pr);
+    hi0 = 0;
+    lo1 = reduce_sum(hi1, lo1, pr);
+    hi1 = 0;
+  };
   if constexpr (MAXD > 0) {
-    static_assert(KB == 1, "digits up front take one ciphertext per thread");
     uint64_t x[MAXD], w0[MAXD], w1[MAXD];
-    const uint64_t* dp = D + b0 * ndig * dstride + ((uint64_t)j << logn) + i;
 #pragma unroll
     for (int d = 0; d < MAXD; d++) {
       if ((uint32_t)d < ndig) {
@@ -387,64 +384,35 @@ __global__ void k_key_mac(const DevPrime* primes, const uint64_t* D, uint64_t ds
 #pragma unroll
     for (int d = 0; d < MAXD; d++) {
       if ((uint32_t)d < ndig) {
-        mac128(hi0[0], lo0[0], x[d], w0[d]);
-        mac128(hi1[0], lo1[0], x[d], w1[d]);
-        if (d % 15 == 14) {
-          lo0[0] = reduce128(hi0[0], lo0[0], pr);
-          hi0[0] = 0;
-          lo1[0] = reduce128(hi1[0], lo1[0], pr);
-          hi1[0] = 0;
-        }
+        mac128(hi0, lo0, x[d], w0[d]);
+        mac128(hi1, lo1, x[d], w1[d]);
+        if (d % 15 == 14) flush();
       }
     }
-  }
-  // The digits of the generic form (MAXD 0): the other forms took theirs above.
-  if constexpr (MAXD == 0) {
+  } else {
     for (uint32_t d = 0; d < ndig; d++) {
-      const uint64_t w0 = __ldg(kp0 + d * kstride), w1 = __ldg(kp1 + d * kstride);
-#pragma unroll
-      for (int u = 0; u < KB; u++) {
-        const uint64_t b = b0 + u;
-        if (b < batch) {
-          const uint64_t x = D[(b * ndig + d) * dstride + ((uint64_t)j << logn) + i];
-          mac128(hi0[u], lo0[u], x, w0);
-          mac128(hi1[u], lo1[u], x, w1);
-        }
-      }
-      if (d % 15 == 14) {
-#pragma unroll
-        for (int u = 0; u < KB; u++) {
-          lo0[u] = reduce128(hi0[u], lo0[u], pr);
-          hi0[u] = 0;
-          lo1[u] = reduce128(hi1[u], lo1[u], pr);
-          hi1[u] = 0;
-        }
-      }
+      const uint64_t x = dp[d * dstride];
+      mac128(hi0, lo0, x, __ldg(kp0 + d * kstride));
+      mac128(hi1, lo1, x, __ldg(kp1 + d * kstride));
+      if (d % 15 == 14) flush();
     }
   }
-#pragma unroll
-  for (int u = 0; u < KB; u++) {
-    const uint64_t b = b0 + u;
-    if (b < batch) {
-      uint64_t* o = out + b * out_stride + ((uint64_t)j << logn) + i;
-      o[0] = reduce128(hi0[u], lo0[u], pr);
-      o[kstride] = reduce128(hi1[u], lo1[u], pr);
-    }
-  }
+  uint64_t* o = out + b * out_stride + row;
+  o[0] = reduce_sum(hi0, lo0, pr);
+  o[kstride] = reduce_sum(hi1, lo1, pr);
 }
 
-// Launches k_key_mac over `batch` ciphertexts, one per thread: sharing the
-// key loads among 4 ciphertexts per thread measured 60% slower on GB300 at 64
-// pairs (fewer threads left too little parallelism to cover the loads of D).
+// Launches k_key_mac over `batch` ciphertexts.
 void launch_key_mac(const DevPrime* primes, PolyRef D, const uint64_t* k0, const uint64_t* k1, const uint64_t* add0,
                     uint64_t add0_stride, uint64_t add0_e, const uint64_t* add1, uint64_t add1_stride, uint64_t* out,
                     uint64_t out_stride, uint32_t ndig, uint32_t lk, uint32_t logn, uint64_t batch, cudaStream_t st) {
   if (batch == 0) return;
   if (D.grp != 1) throw Error(FHEG_ERR_INTERNAL, "key inner product: digits must be a plain array");
   const uint64_t total = batch * lk << logn;
-  auto kern = ndig <= 8 ? k_key_mac<1, 8> : ndig <= 16 ? k_key_mac<1, 16> : k_key_mac<1>;
+  auto kern = ndig <= 4 ? k_key_mac<4> : ndig <= 6 ? k_key_mac<6> : ndig <= 8 ? k_key_mac<8> : ndig <= 12 ? k_key_mac<12>
+              : ndig <= 16 ? k_key_mac<16> : k_key_mac<0>;
   launch_dependent(kern, dim3(nblocks(total, 256)), 256, 0, st, primes, (const uint64_t*)D.base, D.grp_stride, k0, k1, add0,
-                   add0_stride, add0_e, add1, add1_stride, out, out_stride, ndig, lk, logn, batch, total);
+                   add0_stride, add0_e, add1, add1_stride, out, out_stride, ndig, lk, logn, total);
   after_launch("k_key_mac");
 }
 
@@ -836,14 +804,14 @@ __global__ void k_rot_mac(const DevPrime* primes, const RotDesc* d, const uint2*
     mac128(hi0, lo0, x, __ldg(r.k0 + off));
     mac128(hi1, lo1, x, __ldg(r.k1 + off));
     if (dd % 15 == 14) {
-      lo0 = reduce128(hi0, lo0, pr);
+      lo0 = reduce_sum(hi0, lo0, pr);
       hi0 = 0;
-      lo1 = reduce128(hi1, lo1, pr);
+      lo1 = reduce_sum(hi1, lo1, pr);
       hi1 = 0;
     }
   }
-  o[((uint64_t)j << logn) + i] = reduce128(hi0, lo0, pr);
-  o[plane + ((uint64_t)j << logn) + i] = reduce128(hi1, lo1, pr);
+  o[((uint64_t)j << logn) + i] = reduce_sum(hi0, lo0, pr);
+  o[plane + ((uint64_t)j << logn) + i] = reduce_sum(hi1, lo1, pr);
 }
 
 // Switch-down of the requests whose key lies below their level

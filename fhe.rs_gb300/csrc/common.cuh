@@ -486,6 +486,22 @@ __device__ __forceinline__ uint64_t fold_wide_product(uint64_t hi, uint64_t lo, 
   return fold_madu(n, c, pack64((uint32_t)u, (uint32_t)v & mask));
 }
 
+// (hi:lo) mod p, canonical, for a sum of up to 15 products of residues and one
+// residue (below 2^(2k + 4)): by folds where the prime has them (a branch all
+// threads of a limb take alike), else by Barrett. As fold_wide_product, with a
+// third word of at most 4 from bit k up: v stays below 2^62 + 2^60 at k = 62 and n
+// below 2^32.
+__device__ __forceinline__ uint64_t reduce_sum(uint64_t hi, uint64_t lo, const DevPrime& pr) {
+  if (!pr.f_c) return reduce128(hi, lo, pr);
+  const uint32_t mask = (1u << pr.f_sh) - 1, c = (uint32_t)pr.f_c;
+  const uint32_t l1 = (uint32_t)(lo >> 32), h0 = (uint32_t)hi, h1 = (uint32_t)(hi >> 32);
+  const uint32_t q0 = __funnelshift_r(l1, h0, pr.f_sh), q1 = __funnelshift_r(h0, h1, pr.f_sh);
+  const uint64_t u = fold_madu(q0, c, pack64((uint32_t)lo, l1 & mask));
+  const uint64_t v = fold_madu(q1, c, (u >> 32) + ((uint64_t)((h1 >> pr.f_sh) * c) << 32));
+  const uint32_t n = (uint32_t)(v >> pr.f_sh);
+  return fold_canon((int64_t)fold_madu(n, c, pack64((uint32_t)u, (uint32_t)v & mask)), pr);
+}
+
 // a * b mod p, canonical, for residues a, b: by folds where the prime has them
 // (a branch all threads of a limb take alike), else by Barrett.
 __device__ __forceinline__ uint64_t mul_residues(uint64_t a, uint64_t b, const DevPrime& pr) {
