@@ -81,8 +81,11 @@ inline NttGeom ntt_geom(const Context& c, const uint4* jobs) {
 }
 
 // Whether a reduced transform of 2^logn in blocks of 2^bl runs in fold
-// arithmetic: the default block size only (the others are for tuning runs).
-inline bool ntt_folds(const NttGeom& g, uint32_t logn, uint32_t bl) { return g.fold && logn >= 12 && bl == 12; }
+// arithmetic: the default block size only (the others are for tuning runs),
+// and, at 2^11, the whole transform.
+inline bool ntt_folds(const NttGeom& g, uint32_t logn, uint32_t bl) {
+  return g.fold && (logn >= 12 ? bl == 12 : logn == 11);
+}
 
 // Sources whose values come from other moduli or from callers' arrays declare
 // kAnyWord = true and provide word(job, prime, i), the value before any
@@ -249,7 +252,7 @@ __host__ __device__ __forceinline__ constexpr uint32_t swz8(uint32_t i) { return
 // rounds) 1,131.
 template <int LOGN>
 struct NttShape {
-  static constexpr int LOGE = LOGN < 5 ? LOGN : (LOGN >= 12 ? 4 : 5);
+  static constexpr int LOGE = LOGN < 5 ? LOGN : (LOGN >= 11 ? 4 : 5);
   static constexpr int E = 1 << LOGE;
   static constexpr int N = 1 << LOGN;
   static constexpr int T = N / E;
@@ -261,8 +264,8 @@ struct NttShape {
   // x 6 x 128 259 -> 238 and 282 -> 254, the tensor product's inverse 364 -> 356.
   // The plain FOLD block kernels lose 2-5% that way (2^12 x 6 x 512 forward 93
   // -> 97, inverse 109 -> 115).
-  static constexpr int FOLD_BLOCKS = LOGN == 12 ? 4 : 1;
-  static constexpr int MIN_BLOCKS = LOGN == 12 ? 3 : (T >= 512 ? 1 : (512 / T > 32 ? 32 : 512 / T));
+  static constexpr int MIN_BLOCKS = LOGN == 12 ? 3 : LOGN == 11 ? 6 : (T >= 512 ? 1 : (512 / T > 32 ? 32 : 512 / T));
+  static constexpr int FOLD_BLOCKS = LOGN == 12 ? 4 : MIN_BLOCKS;
 };
 
 // One forward round: global stages S0 .. S0+K-1 of a transform of size 2^LOGN
@@ -294,7 +297,7 @@ __device__ __forceinline__ void fwd_round(uint64_t* x, uint32_t tid, const DevPr
       for (int t = 0; t < (1 << K); t++) {
         if (t & half) continue;
         if constexpr (FOLD) {
-          const int4 z = __ldg(pr.ftw + tw0 + (t >> (K - r)) * (kLast ? T : 1));
+          const int4 z = __ldg(pr.ftw + tw0 + (t >> (K - r)) * (kLast ? 1 << S0 : 1));
           if ((LOGN - 1 - S0 - r) & 1) fold_fwd_bfly<false>(xx[t], xx[t + half], z, pr);
           else fold_fwd_bfly<true>(xx[t], xx[t + half], z, pr);
         } else {
@@ -425,7 +428,7 @@ __device__ __forceinline__ void inv_round(uint64_t* x, uint32_t tid, const DevPr
       for (int t = 0; t < (1 << K); t++) {
         if (t & span) continue;
         if constexpr (FOLD) {
-          const int4 z = __ldg(pr.fitw + tw0 + (t >> (r + 1)) * (kFirst ? T : 1));
+          const int4 z = __ldg(pr.fitw + tw0 + (t >> (r + 1)) * (kFirst ? 1 << (LOGN - K) : 1));
           if (U0 + r == 0) fold_inv_bfly<true>(xx[t], xx[t + span], z, pr);
           else fold_inv_bfly<false>(xx[t], xx[t + span], z, pr);
         } else {
@@ -983,7 +986,7 @@ void launch_fwd_block_as(NttGeom g, uint64_t polys, Src src, Dst dst, cudaStream
 // of a transform, and its callers that run one of them, come to the same choice.
 template <int LOGN, bool REDUCE, class Src, class Dst>
 void launch_fwd_block(NttGeom g, uint64_t polys, Src src, Dst dst, cudaStream_t st) {
-  if constexpr (REDUCE && LOGN == 12) {
+  if constexpr (REDUCE && LOGN <= 12) {
     if (g.fold) return launch_fwd_block_as<LOGN, REDUCE, true>(g, polys, src, dst, st);
   }
   launch_fwd_block_as<LOGN, REDUCE, false>(g, polys, src, dst, st);
@@ -1005,7 +1008,7 @@ void launch_inv_block_as(NttGeom g, uint64_t polys, Src src, Dst dst, cudaStream
 
 template <int LOGN, bool FINAL, class Src, class Dst>
 void launch_inv_block(NttGeom g, uint64_t polys, Src src, Dst dst, cudaStream_t st) {
-  if constexpr (LOGN == 12) {
+  if constexpr (LOGN <= 12) {
     if (g.fold) return launch_inv_block_as<LOGN, FINAL, true>(g, polys, src, dst, st);
   }
   launch_inv_block_as<LOGN, FINAL, false>(g, polys, src, dst, st);
@@ -1115,6 +1118,12 @@ constexpr uint32_t kMinUnrolledLogN = 12;
 
 template <bool REDUCE, class Src, class Dst>
 void ntt_fwd_single(uint32_t logn, NttGeom g, uint64_t polys, Src src, Dst dst, cudaStream_t st) {
+  // 2^11 in registers, as the blocks of 2^12, for folding primes (one polynomial
+  // of one limb forward and back, and 256 of 7 limbs: the figures beside
+  // k_ntt_fwd_small).
+  if constexpr (REDUCE) {
+    if (logn == 11 && g.fold) return launch_fwd_block_as<11, true, true>(g, polys, src, dst, st);
+  }
   switch (logn) {
     case 12: launch_fwd_block<12, REDUCE>(g, polys, src, dst, st); break;
     case 13: launch_fwd_block<13, REDUCE>(g, polys, src, dst, st); break;
@@ -1132,6 +1141,9 @@ void ntt_fwd_single(uint32_t logn, NttGeom g, uint64_t polys, Src src, Dst dst, 
 
 template <bool FINAL, class Src, class Dst>
 void ntt_inv_single(uint32_t logn, NttGeom g, uint64_t polys, Src src, Dst dst, cudaStream_t st) {
+  if constexpr (FINAL) {
+    if (logn == 11 && g.fold) return launch_inv_block_as<11, true, true>(g, polys, src, dst, st);
+  }
   switch (logn) {
     case 12: launch_inv_block<12, FINAL>(g, polys, src, dst, st); break;
     case 13: launch_inv_block<13, FINAL>(g, polys, src, dst, st); break;

@@ -132,14 +132,16 @@ int4 fold_constant(uint64_t w, const DevPrime& d) {
 }
 
 // Where the fold tables hold twiddle i of a stage with m chunks (i < m). The
-// stages with m >= N / 16, one round of a 2^12-block whose 256 threads take m'
-// = 16 m / N consecutive twiddles each, keep every 256 m' of them transposed:
-// the threads' first ones, then their second ones, and so on (16-byte loads of
-// a warp then cover four lines instead of up to 32: 59% of the L1's
-// throughput went into them). Other stages are in the tables' own order.
+// stages of a block's last forward round (first inverse one), whose 256 groups
+// take `per` consecutive twiddles each (blocks of 2^12: 16 m / N from m = N / 16;
+// 2^11: 8 m / N from N / 8), keep every 256 per of them transposed: the groups'
+// first ones, then their second ones, and so on (16-byte loads of a warp then
+// cover four lines instead of up to 32: 59% of the L1's throughput went into
+// them). Other stages are in the tables' own order.
 __device__ __forceinline__ uint32_t fold_table_index(uint32_t i, uint32_t m, uint32_t n) {
-  if (m < n / 16) return i;
-  const uint32_t per = 16 * m / n, group = i & ~(256 * per - 1), at = i & (256 * per - 1);
+  const uint32_t last = n >= 4096 ? 16 : 8;
+  if (m < n / last) return i;
+  const uint32_t per = last * m / n, group = i & ~(256 * per - 1), at = i & (256 * per - 1);
   return group + (at % per) * 256 + at / per;
 }
 
@@ -178,7 +180,7 @@ std::shared_ptr<PrimeTables> get_prime_tables(uint64_t p, size_t n, uint64_t roo
   t->host = make_ntt_tables(p, n, root);
   int32_t fc = 0, fk = 0;
   uint64_t fbias = 0;
-  const bool fold = n >= 4096 && fold_params(p, &fc, &fk, &fbias);
+  const bool fold = n >= 2048 && fold_params(p, &fc, &fk, &fbias);
   t->tables.alloc((fold ? 8 : 4) * n * sizeof(uint64_t));
   std::vector<uint64_t> inter(4 * n);
   for (size_t i = 0; i < n; i++) {

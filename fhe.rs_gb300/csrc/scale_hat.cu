@@ -583,13 +583,18 @@ std::unique_ptr<RnsHatD> make_rns_hat(const Context& from, const Context& to, co
     const BigUint hat = M / BigUint(m);
     hat_mod[k] = hat.mod_u64(m);
     hat_inv[k] = invmod(hat_mod[k], m);
+    if (host.is_one) {
+      phi_int[k] = hat;
+      continue;
+    }
     BigUint rem;
     BigUint::divmod(hat * num, den, &phi_int[k], &rem);
+    if (rem.is_zero()) continue;
     phi[k] = ((rem << 112) / den).low_u128();
-    if (!rem.is_zero()) h->frac = (uint32_t)k + 1;
+    h->frac = (uint32_t)k + 1;
   }
-  BigUint gamma_int, gamma_rem;
-  BigUint::divmod(M * num, den, &gamma_int, &gamma_rem);
+  BigUint gamma_int = M, gamma_rem;
+  if (!host.is_one) BigUint::divmod(M * num, den, &gamma_int, &gamma_rem);
   // 1 - gamma with gamma rounded up; without a fraction, Gamma itself and 0.
   uint64_t one_minus = 0;
   if (!gamma_rem.is_zero()) {

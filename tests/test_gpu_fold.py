@@ -22,7 +22,7 @@ SHAPES = [(39, 1 << 39), (40, 1 << 40), (41, 1 << 41), (43, 1 << 43), (50, 1 << 
 
 
 @pytest.mark.parametrize("bits,below", SHAPES)
-@pytest.mark.parametrize("logn", [12, 13, 14, 15, 16])
+@pytest.mark.parametrize("logn", [11, 12, 13, 14, 15, 16])
 def test_transforms(fg, ora, cuda, bits, below, logn):
     """Forward, lazy forward and inverse on random rows and on the rows that drive the lazy values to their bounds: all
     p - 1, alternating 0 and p - 1, a single p - 1, all p / 2."""
