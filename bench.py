@@ -49,10 +49,10 @@ STAGE_LIMBS = {
 }
 STAGE_KERNELS = {
     "A": "k_ntt_inv<12, SrcPair> (inverse NTT of the operands, block pass; its strided last stages run in B)",
-    "B": "k_rns_scale<6, 8> (A's strided last stages, extension 6 -> 7 new moduli, C's strided first stages)",
+    "B": "k_rns_hat<6, 8> (A's strided last stages, extension 6 -> 7 new moduli, C's strided first stages)",
     "C": "k_ntt_fwd<12> (forward NTT of the extension limbs, block pass)",
     "D": "k_ntt_inv<12, SrcTensor> (tensor product + inverse NTT, block pass; its strided last stages run in E)",
-    "E": "k_rns_scale<13, 8> (D's strided last stages, t/Q scale-down 13 -> 6, F's strided first stages and "
+    "E": "k_rns_hat<13, 8> (D's strided last stages, t/Q scale-down 13 -> 6, F's strided first stages and "
          "digit expansion)",
     "F": "k_ntt_fwd<12>, twice (digit NTTs in every key modulus, then c0/c1 NTTs; block passes)",
     "G": "k_key_mac (key inner product)",
@@ -64,18 +64,18 @@ STAGE_LAUNCHES = {"A": 1, "B": 1, "C": 1, "D": 1, "E": 1, "F": 2, "G": 1}
 # strided NTT stage applied inside the RNS scalers B and E; E's sums on the
 # tensor cores), from the ncu capture summarised in
 # profiles/stages_mul_relin_n16384_b64.md.
-STAGE_TRAFFIC_BYTES = {"A": 353.2e6, "B": 393.2e6, "C": 409.4e6, "D": 728.0e6, "E": 675.7e6, "F": 696.2e6,
-                       "G": 493.6e6}
+STAGE_TRAFFIC_BYTES = {"A": 352.6e6, "B": 397.2e6, "C": 408.6e6, "D": 747.3e6, "E": 682.3e6, "F": 694.1e6,
+                       "G": 494.0e6}
 # The ncu figures above and below hold for the library sources they were
 # captured on: library_source_hash() of that tree. A run on other sources
 # reports null for them instead of stale numbers.
-PROFILED_SOURCE_HASH = "e7052cef359c4eb3"
+PROFILED_SOURCE_HASH = "ba6313dd53e7415c"
 # Share of the elapsed cycles in which the integer multipliers (the FMA-heavy
 # pipe, which executes every IMAD) were busy, per stage, from the same ncu
 # capture of one 64-pair multiplication (F: time-weighted over its two
 # launches); the whole multiplication, time-weighted.
-STAGE_FMAHEAVY_PCT = {"A": 69.9, "B": 84.0, "C": 70.6, "D": 67.1, "E": 61.3, "F": 70.4, "G": 63.7}
-MULTIPLY_FMAHEAVY_PCT = 69.3
+STAGE_FMAHEAVY_PCT = {"A": 68.4, "B": 61.1, "C": 71.2, "D": 68.3, "E": 59.0, "F": 70.4, "G": 64.4}
+MULTIPLY_FMAHEAVY_PCT = 66.2
 
 
 def library_source_hash() -> str:
@@ -538,8 +538,9 @@ def run_ours(args, rank: int, world: int):
                     "fwd_frac_of_ceiling": bfly / (fwd_ms / 1000.0) / probes[4]["ops_per_s"],
                     "inv_frac_of_ceiling": bfly / (inv_ms / 1000.0) / probes[5]["ops_per_s"],
                     "butterflies_per_s_for_60pct_hbm": need_60,
-                    "note": "the butterfly ceiling is fheg_intpeak's register-resident Harvey butterfly: an NTT "
-                            "at 60% of HBM needs more butterflies per second than the integer pipes issue"},
+                    "note": "the butterfly ceiling is fheg_intpeak's register-resident Harvey butterfly (the "
+                            "transforms of primes just below powers of two run a cheaper one): an NTT at 60% "
+                            "of HBM needs more butterflies per second than the integer pipes issue"},
             "gpu_launches": int(launches),
             "clocks": clocks.summary(),
             "cpu_baseline": cpu,

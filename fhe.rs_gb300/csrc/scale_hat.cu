@@ -28,9 +28,10 @@
 // Stage times, events, against the CUDA-core extension and the two- and
 // four-pass tensor-core scale-down (scale.cu) in the same multiplication: 64
 // pairs at N = 2^14, L = 6: extension 0.326 -> 0.216 ms, scale-down 0.490 -> 0.330;
-// 16 pairs at N = 2^15, L = 12: 0.379 -> 0.283 and 0.764 -> 0.508 (both with the
+// 16 pairs at N = 2^15, L = 12: 0.379 -> 0.283 and 0.764 -> 0.510 (both with the
 // transforms' stages on either side in fold arithmetic as well). Bound by
-// latency: 24-28 warps an SM, the multiplier 45-54% busy.
+// latency at 24-28 warps an SM beside the multiplier (59-61% busy, the tensor
+// pipe 5-7%).
 
 #include <algorithm>
 #include <cstring>
