@@ -275,8 +275,10 @@ def _dp(t) -> int:
 
 
 def _stream() -> int:
+    # The raw handle of torch.cuda.current_stream() without its Stream object: 0.3
+    # against 2.8 us a call, where the smallest transforms take 6 us on the device.
     torch = _torch()
-    return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def empty(shape, device="cuda"):
