@@ -1120,8 +1120,8 @@ template <bool REDUCE, class Src, class Dst>
 void ntt_fwd_single(uint32_t logn, NttGeom g, uint64_t polys, Src src, Dst dst, cudaStream_t st) {
   // 2^11 in registers, as the blocks of 2^12, for folding primes: the kernels for
   // any size up to 2^14 go to shared memory and a barrier in every stage
-  // (forward / inverse: one polynomial of one limb 11.3 / 11.3 -> 8.1 / 8.0 us, 175
-  // of 7 limbs 69.7 / 69.9 -> 19.8 / 22.3, 1024 of 6 limbs 334 / 337 -> 86 / 95).
+  // (forward and inverse: one polynomial of one limb 20.5 -> 11.2 us, 175 of 7 limbs
+  // 140 -> 42, 1024 of 6 limbs 670 -> 181).
   if constexpr (REDUCE) {
     if (logn == 11 && g.fold) return launch_fwd_block_as<11, true, true>(g, polys, src, dst, st);
   }
