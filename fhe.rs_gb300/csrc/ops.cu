@@ -73,6 +73,9 @@ void set_ntt_block_logn(uint32_t logn, uint32_t block_logn) {
 
 void upload(void* dst, const void* src, size_t bytes) {
   check_cuda(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice), "cudaMemcpy H2D");
+  // A copy from pageable memory may return with its last part on the way, and
+  // non-blocking streams do not wait for the default stream.
+  check_cuda(cudaStreamSynchronize(nullptr), "cudaStreamSynchronize");
 }
 
 // ---------------------------------------------------------------------------
@@ -219,9 +222,10 @@ std::shared_ptr<PrimeTables> get_prime_tables(uint64_t p, size_t n, uint64_t roo
     const uint64_t r32 = (1ull << 32) % p;
     k_fold_tables<<<(unsigned)((2 * n + 255) / 256), 256>>>(dp.tw, ft, p, r32, shoup(r32, p), fc, fk,
                                                             (uint32_t)n);
-    // Complete before any use: every context uploads its primes after this,
-    // on the same stream.
     after_launch("k_fold_tables");
+    // Complete before the registry hands the tables out: a non-blocking stream
+    // (or another thread's) does not wait for this launch on the default one.
+    check_cuda(cudaStreamSynchronize(nullptr), "cudaStreamSynchronize");
     dp.ftw = ft;
     dp.fitw = ft + n;
     dp.f_bias = fbias;
