@@ -412,15 +412,23 @@ def ntt_prefetch_set(on: bool):
     check(lib().fheg_ntt_prefetch_set(int(on)))
 
 
+class _ClusterByPrimes(int):
+    """The cluster setting of a size left to its default, where that depends on
+    a context's primes: reads as off, and set again leaves the default in place."""
+
+    def __repr__(self):
+        return "by primes"
+
+
 def ntt_cluster_set(logn: int, on: bool):
     """Single-pass cluster mode of the 2^12-block plan for 2^logn (see fheg.h)."""
-    check(lib().fheg_ntt_cluster_set(logn, int(on)))
+    check(lib().fheg_ntt_cluster_set(logn, -1 if isinstance(on, _ClusterByPrimes) else int(on)))
 
 
 def ntt_cluster_get(logn: int) -> bool:
     out = ctypes.c_int(0)
     check(lib().fheg_ntt_cluster_get(logn, ctypes.byref(out)))
-    return bool(out.value)
+    return _ClusterByPrimes(0) if out.value < 0 else bool(out.value)
 
 
 def rns_tensor_set(on: bool):

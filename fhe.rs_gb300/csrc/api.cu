@@ -165,13 +165,14 @@ FHEG_API int fheg_ntt_prefetch_set(int on) {
 }
 
 FHEG_API int fheg_ntt_cluster_set(uint32_t logn, int on) {
-  return abi_call([&] { set_ntt_cluster(logn, on != 0); });
+  return abi_call([&] { set_ntt_cluster(logn, on < 0 ? -1 : on != 0); });
 }
 
 FHEG_API int fheg_ntt_cluster_get(uint32_t logn, int* on) {
   return abi_call([&] {
     abi_need(on && logn <= 16, "bad size or null output");
-    *on = ntt_cluster_enabled(logn, false) ? 1 : 0;
+    const bool off_fold = ntt_cluster_enabled(logn, false);
+    *on = off_fold == ntt_cluster_enabled(logn, true) ? (off_fold ? 1 : 0) : -1;
   });
 }
 
@@ -222,7 +223,7 @@ uint32_t autotune_plans(uint32_t logn, cudaStream_t st, F run) {
   try {
     for (const auto& plan : plans) {
       set_ntt_block_logn(logn, plan.first);
-      set_ntt_cluster(logn, plan.second);
+      set_ntt_cluster(logn, plan.second ? 1 : 0);
       for (int rep = 0; rep < 2; rep++) {
         check_cuda(cudaEventRecord(e0, st), "cudaEventRecord");
         run();
@@ -238,7 +239,7 @@ uint32_t autotune_plans(uint32_t logn, cudaStream_t st, F run) {
     }
   } catch (...) {
     set_ntt_block_logn(logn, before);
-    restore_ntt_cluster(logn, before_cluster);
+    set_ntt_cluster(logn, before_cluster);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     throw;
@@ -246,7 +247,7 @@ uint32_t autotune_plans(uint32_t logn, cudaStream_t st, F run) {
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   set_ntt_block_logn(logn, best.first);
-  set_ntt_cluster(logn, best.second);
+  set_ntt_cluster(logn, best.second ? 1 : 0);
   return best.first;
 }
 

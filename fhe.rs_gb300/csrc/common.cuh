@@ -74,10 +74,9 @@ std::vector<uint32_t> ntt_plans(uint32_t logn);
 // memory (fheg_ntt_cluster_set).
 // `fold`: the transform runs in fold arithmetic.
 bool ntt_cluster_enabled(uint32_t logn, bool fold);
-void set_ntt_cluster(uint32_t logn, bool on);
-// The setting itself (-1: never set), and putting it back.
+// The setting itself: 1 on, 0 off, -1 the default.
 int ntt_cluster_state(uint32_t logn);
-void restore_ntt_cluster(uint32_t logn, int state);
+void set_ntt_cluster(uint32_t logn, int state);
 
 inline void check_cuda(cudaError_t e, const char* what) {
   if (e != cudaSuccess) throw Error(10 /*FHEG_ERR_CUDA*/, std::string(what) + ": " + cudaGetErrorString(e));

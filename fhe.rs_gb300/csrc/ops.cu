@@ -58,12 +58,9 @@ bool ntt_cluster_enabled(uint32_t logn, bool fold) {
   return v >= 0 ? v != 0 : logn == 13 || logn == 14 || (logn == 15 && fold);
 }
 int ntt_cluster_state(uint32_t logn) { return logn <= 16 ? g_ntt_cluster[logn].load(std::memory_order_relaxed) : -1; }
-void restore_ntt_cluster(uint32_t logn, int state) {
-  if (logn <= 16) g_ntt_cluster[logn].store(state, std::memory_order_relaxed);
-}
-void set_ntt_cluster(uint32_t logn, bool on) {
+void set_ntt_cluster(uint32_t logn, int state) {
   if (logn > 16) throw Error(FHEG_ERR_INVALID_ARGUMENT, "unsupported NTT size");
-  g_ntt_cluster[logn].store(on ? 1 : 0, std::memory_order_relaxed);
+  g_ntt_cluster[logn].store(state, std::memory_order_relaxed);
 }
 
 void set_ntt_block_logn(uint32_t logn, uint32_t block_logn) {

@@ -165,8 +165,10 @@ FHEG_API int fheg_ntt_prefetch_set(int on);
  * the strided stages through distributed shared memory instead of a second
  * pass over device memory (GPUs that cannot run the cluster size fall back
  * to two passes). Schedules only; process-wide per logn. On by default at 2^13
- * and 2^14, and at 2^15 for contexts whose primes lie just below powers of two;
- * the setting reads as off at 2^15 until it is set. */
+ * and 2^14, and at 2^15 for contexts whose primes lie just below powers of two:
+ * there the setting reads as -1, "by the context's primes", until it is set.
+ * Setting -1 gives a size its default back, so that setting what was read
+ * changes nothing. */
 FHEG_API int fheg_ntt_cluster_set(uint32_t logn, int on);
 FHEG_API int fheg_ntt_cluster_get(uint32_t logn, int* on);
 /* Tensor-core form of the exact RNS scalings (rns/scaler.rs:249-352 through
