@@ -1103,7 +1103,7 @@ class Multiplicator:
 
     def set_small_plan(self, max_count: int, plan=None):
         """Plan of batches of at most max_count pairs (0 turns it off)."""
-        arr = (ctypes.c_uint32 * 6)(*(list(plan or [12, 12, 12, 12, 1, 0]) + [0] * 6)[:6])
+        arr = (ctypes.c_uint32 * 6)(*(list(plan or [12, 12, 12, 12, 0, 0]) + [0] * 6)[:6])
         check(lib().fheg_multiplicator_set_small_plan(self._h, max_count, arr))
 
     @property
