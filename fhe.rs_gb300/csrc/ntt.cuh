@@ -9,18 +9,19 @@
 // and are reduced at the end, so outputs are bit-identical to the reference.
 //
 // Layout: one CTA transforms one block of 2^bl residues of one limb (bl <= 14,
-// resident in shared memory). Each thread keeps 16 residues in registers
-// (32 in blocks below 2^12) and runs up to four (five) butterfly stages on
+// resident in shared memory). From 2^12 on (2^11 in fold arithmetic) each
+// thread keeps 16 residues in registers and runs up to four butterfly stages on
 // them per round; rounds exchange data through shared memory with an XOR
-// swizzle that keeps 64-bit
-// accesses free of bank conflicts. A transform of 2^logn is either one block
+// swizzle that keeps 64-bit accesses free of bank conflicts. Smaller transforms
+// stay in shared memory. A transform of 2^logn is either one block
 // (bl = logn) or, following the plan of ntt_block_logn(), a strided pass over
 // groups of 2^(logn - bl) elements for the first (forward) or last (inverse)
 // stages plus the block kernel for the others.
 //
 // Two arithmetics. Any prime below 2^62 takes Harvey's butterflies with Shoup
 // twiddles; where every prime of a launch lies just below a power of two
-// (DevPrime::f_c, NttGeom::fold) and the blocks hold 2^12 residues, reduced
+// (DevPrime::f_c, NttGeom::fold) and the blocks hold 2^12 residues or the whole
+// transform 2^11, reduced
 // transforms take the FOLD form of the same stages (common.cuh), with signed
 // lazy values between the passes and the same canonical outputs. Lazy forward
 // outputs ([0, 4p), a value callers see) stay with Harvey's butterflies.
@@ -241,9 +242,8 @@ __device__ __forceinline__ uint64_t& sm_at(uint64_t* sm, uint32_t off8) {
 // Byte offset of the swizzled word index i.
 __host__ __device__ __forceinline__ constexpr uint32_t swz8(uint32_t i) { return swz(i) << 3; }
 
-// Residues per thread: 16 (radix-16 rounds) in blocks of 2^12 to 2^14, 32
-// (radix-32 rounds) in smaller blocks. With 32 residues the 2^12-2^14 kernels
-// spilled 100-470 bytes per thread at their 128-register budget; with 16 they
+// Residues per thread: 16 (radix-16 rounds) in blocks of 2^11 to 2^14. With 32
+// residues (radix-32 rounds) the 2^12-2^14 kernels spilled 100-470 bytes per thread at their 128-register budget; with 16 they
 // spill nothing at 128. Blocks of 2^12 (256 threads) run three CTAs per SM
 // under an 80-register cap (24 warps, a few words spilled). On GB300 the
 // forward + inverse NTT at N = 2^14 with 2^12 blocks went from 1,064 GB/s
@@ -1114,12 +1114,11 @@ bool launch_inv_cluster(NttGeom g, uint32_t s1, uint64_t polys, Src src, Dst dst
 }
 
 // Dispatch over log2(N) for a single-pass transform (3 <= logn <= 14).
-constexpr uint32_t kMinUnrolledLogN = 12;
 
 template <bool REDUCE, class Src, class Dst>
 void ntt_fwd_single(uint32_t logn, NttGeom g, uint64_t polys, Src src, Dst dst, cudaStream_t st) {
-  // 2^11 in registers, as the blocks of 2^12, for folding primes: the kernels for
-  // any size up to 2^14 go to shared memory and a barrier in every stage
+  // 2^11 in registers, as the blocks of 2^12, for folding primes: the kernels of
+  // the sizes up to 2^11 go to shared memory and a barrier in every stage
   // (forward and inverse: one polynomial of one limb 20.5 -> 11.2 us, 175 of 7 limbs
   // 140 -> 42, 1024 of 6 limbs 670 -> 181).
   if constexpr (REDUCE) {
@@ -1221,7 +1220,7 @@ void ntt_forward_any(uint32_t logn, NttGeom g, uint64_t polys, Src src, Dst dst,
     return;
   }
   const uint32_t s1 = logn - bl;
-  if (bl == 12 && ntt_cluster_enabled(logn, g.fold) && launch_fwd_cluster<12, REDUCE>(g, s1, polys, src, dst, st)) return;
+  if (bl == 12 && ntt_cluster_enabled(logn, REDUCE && g.fold) && launch_fwd_cluster<12, REDUCE>(g, s1, polys, src, dst, st)) return;
   launch_fwd_top<REDUCE>(s1, g, bl, polys, src, dst, st);
   g.s1 = s1;
   switch (bl) {

@@ -34,3 +34,18 @@ def test_small_plan_goes_back_to_its_default(fg, ora, cuda, n):
     mult.set_small_plan(8)
     assert _launches(fg, lambda: mult.multiply(x, y)) == default
     assert np.array_equal(fg.to_host(mult.multiply(x, y)), want)
+
+
+@pytest.mark.parametrize("logn,lazy,launches", [(13, False, 1), (13, True, 1), (14, True, 1), (15, False, 1),
+                                                (15, True, 2), (16, False, 2), (16, True, 2)])
+def test_lazy_transforms_of_folding_primes(fg, ora, cuda, logn, lazy, launches):
+    """2^15 runs in clusters by default where the transform folds; a lazy one does not, and takes two passes."""
+    n = 1 << logn
+    p = ora.generate_prime(62, 2 * n, 1 << 62)
+    ctx = fg.Context([p], n)
+    row = np.random.default_rng(logn).integers(0, p, n, dtype=np.uint64)
+    want = row.copy()
+    ora.ntt_operator(p, n).forward(want)
+    t = fg.to_device(row[None, None])
+    assert _launches(fg, lambda: fg.ntt_forward(ctx, t, lazy=lazy)) == launches
+    assert np.array_equal(fg.to_host(t)[0, 0] % np.uint64(p), want)
