@@ -993,7 +993,11 @@ RnsScalerD::RnsScalerD(const Context& from, const Context& to, const BigUint& nu
       to_pinv[j] = 0 - inv;
     }
     hat = make_rns_hat(from, to, host, gamma_neg, gamma_neg_hi, num, den);
-    if (!hat) build_tc_matrix();
+    // k_rns_scale's tensor-core forms are those of 12, 13 and 25 sources. With
+    // scale_hat.cu they take the transforms that do not fold (blocks other than
+    // 2^12, or a key whose moduli do not fold): 12 pairs at N = 2^15, L = 12 in blocks
+    // of 2^13 were 2.79 ms without them and are 2.66 with them.
+    if (!hat || F == 12 || F == 13 || F == 25) build_tc_matrix();
   }
 }
 
