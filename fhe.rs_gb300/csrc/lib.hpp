@@ -105,7 +105,7 @@ int4 fold_constant(uint64_t w, const DevPrime& d);
 // Constants of the scaler between primes just below a power of two
 // (scale_hat.cu): what its launches copy, and its device tables.
 struct RnsHatD {
-  uint32_t maxf, maxt, kp, frac;  // kernel class, matrix width, sources with a fraction
+  uint32_t maxf, maxt, maxs, kp, frac;  // kernel class, matrix width, sources with a fraction
   std::vector<uint32_t> inv, zsh, th, c, sh;
   std::vector<uint64_t> gneg;
   uint32_t g1, g2;

@@ -58,8 +58,8 @@ namespace {
 // Count of waits of this kernel that ran out (hat_wait_failures).
 __device__ uint32_t g_hat_wait_failures;
 
-// Constants of one launch, read from the parameter bank. MS: sources with a
-// nonzero phi_k come first (k < frac).
+// Constants of one launch, read from the parameter bank. The sources with a
+// nonzero phi_k come first (k < frac <= MS).
 template <int MAXF, int MAXT, int MS>
 struct HatLaunch {
   uint32_t from_len, out_len, frac;
@@ -231,12 +231,12 @@ __device__ __forceinline__ void hat_mma(uint32_t bar_b, uint32_t phase, uint32_t
 // CTA owns 128 >> TOP groups), and the outputs may leave through the first
 // TOP stages of a forward one. zc: per source the digits (fold_mul) of
 // hat_k^-1, N^-1 hat_k^-1 and zetas_inv[N - 2] N^-1 hat_k^-1.
-template <int MAXF, int MAXT, int TOP, bool ONE>
-__global__ void __launch_bounds__(128) k_rns_hat(const __grid_constant__ HatLaunch<MAXF, MAXT, MAXF / 2 + 1> s,
+template <int MAXF, int MAXT, int MS, int TOP, bool ONE>
+__global__ void __launch_bounds__(128) k_rns_hat(const __grid_constant__ HatLaunch<MAXF, MAXT, MS> s,
                                                  uint32_t logn, PolyRef in, PolyRef out, const DevPrime* src_primes,
                                                  const int4* zc, const uint16_t* mat, const HatExact* ex,
                                                  uint32_t start, const FwdEpilogue fe) {
-  constexpr int G = 128 >> TOP, MS = MAXF / 2 + 1;
+  constexpr int G = 128 >> TOP;
   using K = HatShape<MAXF>;
   constexpr bool BIASED = K::kBiased;
   constexpr uint32_t KP = K::kKp;
@@ -427,13 +427,19 @@ __global__ void __launch_bounds__(128) k_rns_hat(const __grid_constant__ HatLaun
   }
 }
 
-// Source and output counts of the kernels. Factor one: F <= 3, 6, 8, 12, 16;
-// others: F <= 7, 13, 16, 25, 32 with a fraction at up to F / 2 + 1 sources.
+// Sources, outputs and sources with a fraction of the kernels. A scaler takes
+// the first one that holds all three. Scale-downs of multiplications have a
+// fraction at up to F / 2 + 1 sources, decryption's at every one: up to 16 sources
+// the kernels come with both (one with them all is 0.5% slower for the former,
+// whose unrolled sums it skips one by one; the next larger class was 20-45% slower
+// for the latter: 13 sources to 1 output 27.4 -> 18.7 us, 12 to 12 with
+// six fractions 43.2 on k_rns_scale's tensor cores -> 35.1).
 struct HatClass {
-  uint32_t maxf, maxt;
+  uint32_t maxf, maxt, maxs;
 };
-constexpr HatClass kHatOne[] = {{3, 8}, {6, 8}, {8, 16}, {12, 16}, {16, 16}};
-constexpr HatClass kHatDown[] = {{7, 8}, {13, 8}, {16, 16}, {25, 16}, {32, 16}};
+constexpr HatClass kHatOne[] = {{3, 8, 1}, {6, 8, 1}, {8, 16, 1}, {12, 16, 1}, {16, 16, 1}};
+constexpr HatClass kHatDown[] = {{7, 8, 4},   {7, 8, 7},    {13, 8, 7},   {13, 8, 13},
+                                 {16, 16, 9}, {16, 16, 16}, {25, 16, 13}, {32, 16, 16}};
 
 // HatShape at run time.
 constexpr uint32_t hat_chunks(uint32_t maxf) { return maxf > 12 ? 2 : 1; }
@@ -470,11 +476,10 @@ size_t hat_prepare(const void* kern, size_t most) {
   return a.sharedSizeBytes;
 }
 
-template <int MAXF, int MAXT, int TOP, bool ONE>
+template <int MAXF, int MAXT, int MS, int TOP, bool ONE>
 void launch_hat_top(const RnsScalerD& sc, uint32_t logn, PolyRef in, PolyRef out, uint32_t start, uint32_t out_len,
                     uint64_t total, cudaStream_t st, const FwdEpilogue& fe) {
   constexpr uint32_t KP = HatShape<MAXF>::kKp;
-  constexpr int MS = MAXF / 2 + 1;
   const RnsHatD& h = *sc.hat;
   if (h.kp != KP) throw Error(FHEG_ERR_INTERNAL, "tensor-core scaler matrix of another width");
   HatLaunch<MAXF, MAXT, MS> s;
@@ -506,7 +511,7 @@ void launch_hat_top(const RnsScalerD& sc, uint32_t logn, PolyRef in, PolyRef out
   }
   s.b_rows = (8 * out_len + 15) / 16 * 16;
   s.cols = s.b_rows <= 32 ? 32 : s.b_rows <= 64 ? 64 : 128;
-  auto kern = k_rns_hat<MAXF, MAXT, TOP, ONE>;
+  auto kern = k_rns_hat<MAXF, MAXT, MS, TOP, ONE>;
   // The stage buffer (TOP > 0) overlaid by A, then B; at least 456 bytes per
   // tensor-memory column (with the 1 KB the SM reserves per CTA), so that the
   // CTAs an SM holds never ask for more than its 512 columns.
@@ -521,14 +526,14 @@ void launch_hat_top(const RnsScalerD& sc, uint32_t logn, PolyRef in, PolyRef out
   after_launch("k_rns_hat");
 }
 
-template <int MAXF, int MAXT, bool ONE>
+template <int MAXF, int MAXT, int MS, bool ONE>
 void launch_hat(const RnsScalerD& sc, uint32_t logn, PolyRef in, PolyRef out, uint32_t start, uint32_t out_len,
                 uint64_t total, cudaStream_t st, uint32_t top, const FwdEpilogue& fe) {
   switch (top) {
-    case 0: launch_hat_top<MAXF, MAXT, 0, ONE>(sc, logn, in, out, start, out_len, total, st, fe); break;
-    case 1: launch_hat_top<MAXF, MAXT, 1, ONE>(sc, logn, in, out, start, out_len, total, st, fe); break;
-    case 2: launch_hat_top<MAXF, MAXT, 2, ONE>(sc, logn, in, out, start, out_len, total, st, fe); break;
-    case 3: launch_hat_top<MAXF, MAXT, 3, ONE>(sc, logn, in, out, start, out_len, total, st, fe); break;
+    case 0: launch_hat_top<MAXF, MAXT, MS, 0, ONE>(sc, logn, in, out, start, out_len, total, st, fe); break;
+    case 1: launch_hat_top<MAXF, MAXT, MS, 1, ONE>(sc, logn, in, out, start, out_len, total, st, fe); break;
+    case 2: launch_hat_top<MAXF, MAXT, MS, 2, ONE>(sc, logn, in, out, start, out_len, total, st, fe); break;
+    case 3: launch_hat_top<MAXF, MAXT, MS, 3, ONE>(sc, logn, in, out, start, out_len, total, st, fe); break;
     default: throw Error(FHEG_ERR_INTERNAL, "unsupported strided stage count");
   }
 }
@@ -549,20 +554,23 @@ void rns_scale_hat(const RnsScalerD& sc, uint32_t logn, PolyRef in, PolyRef out,
   const uint64_t total = polys << logn;
   const uint32_t s1 = top ? top->s1 : 0;
   const bool one = sc.host.is_one;
-  const uint32_t cls = sc.hat->maxf;
-#define HAT(F_, T_, ONE_) launch_hat<F_, T_, ONE_>(sc, logn, in, out, start, out_len, total, st, s1, fe)
+  const uint32_t cls = sc.hat->maxf, fr = sc.hat->maxs;
+#define HAT(F_, T_, S_, ONE_) launch_hat<F_, T_, S_, ONE_>(sc, logn, in, out, start, out_len, total, st, s1, fe)
   if (one) {
-    if (cls == 3) HAT(3, 8, true);
-    else if (cls == 6) HAT(6, 8, true);
-    else if (cls == 8) HAT(8, 16, true);
-    else if (cls == 12) HAT(12, 16, true);
-    else HAT(16, 16, true);
+    if (cls == 3) HAT(3, 8, 1, true);
+    else if (cls == 6) HAT(6, 8, 1, true);
+    else if (cls == 8) HAT(8, 16, 1, true);
+    else if (cls == 12) HAT(12, 16, 1, true);
+    else HAT(16, 16, 1, true);
   } else {
-    if (cls == 7) HAT(7, 8, false);
-    else if (cls == 13) HAT(13, 8, false);
-    else if (cls == 16) HAT(16, 16, false);
-    else if (cls == 25) HAT(25, 16, false);
-    else HAT(32, 16, false);
+    if (cls == 7 && fr == 4) HAT(7, 8, 4, false);
+    else if (cls == 7) HAT(7, 8, 7, false);
+    else if (cls == 13 && fr == 7) HAT(13, 8, 7, false);
+    else if (cls == 13) HAT(13, 8, 13, false);
+    else if (cls == 16 && fr == 9) HAT(16, 16, 9, false);
+    else if (cls == 16) HAT(16, 16, 16, false);
+    else if (cls == 25) HAT(25, 16, 13, false);
+    else HAT(32, 16, 16, false);
   }
 #undef HAT
 }
@@ -604,14 +612,21 @@ std::unique_ptr<RnsHatD> make_rns_hat(const Context& from, const Context& to, co
   }
   h->g1 = (uint32_t)(one_minus >> 28);
   h->g2 = (uint32_t)(one_minus & ((1u << 28) - 1));
-  // The kernel class.
-  h->maxf = h->maxt = 0;
-  if (host.is_one) {
-    for (const HatClass& c : kHatOne)
-      if (!h->maxf && F <= c.maxf) h->maxf = c.maxf, h->maxt = c.maxt;
-  } else {
-    for (const HatClass& c : kHatDown)
-      if (!h->maxf && F <= c.maxf && h->frac <= std::min<uint32_t>(c.maxf / 2 + 1, 16)) h->maxf = c.maxf, h->maxt = c.maxt;
+  // The kernel class, by the outputs a scaling writes (with factor one, without
+  // the leading moduli both sides share); where none holds them all, for calls
+  // that ask for fewer.
+  size_t outs = T;
+  if (host.is_one)
+    for (size_t k = 0; k < F && k < T && from.moduli[k] == to.moduli[k]; k++) outs--;
+  h->maxf = h->maxt = h->maxs = 0;
+  auto pick = [&](const HatClass& c, size_t least) {
+    if (!h->maxf && F <= c.maxf && h->frac <= c.maxs && least <= c.maxt) h->maxf = c.maxf, h->maxt = c.maxt, h->maxs = c.maxs;
+  };
+  for (const size_t least : {outs, (size_t)0}) {
+    if (host.is_one)
+      for (const HatClass& c : kHatOne) pick(c, least);
+    else
+      for (const HatClass& c : kHatDown) pick(c, least);
   }
   if (!h->maxf) return nullptr;
   h->kp = hat_kp(h->maxf);

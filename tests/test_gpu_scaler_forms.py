@@ -99,3 +99,23 @@ def test_scalers(fg, ora, cuda, F, T, factor, folding):
     finally:
         fg.rns_tensor_set(default)
     assert fg.rns_tensor_wait_failures() == 0
+
+
+@pytest.mark.parametrize("n,L", [(4096, 3), (8192, 6), (16384, 3), (16384, 6), (16384, 7), (32768, 4)])
+def test_products_with_a_fraction_at_every_source(fg, ora, cuda, n, L):
+    """Scaled down by 3 / 1001, which no modulus divides out of, with none to three strided stages on either side."""
+    moduli = _primes(ora, n, L, True)
+    rng = np.random.default_rng(n + L)
+    par_o = ora.BfvParameters(n, 65537, moduli=moduli)
+    sk = ora.SecretKey.random(par_o, rng)
+    values = rng.integers(0, 65537, (2, n), dtype=np.uint64)
+    ct = [sk.encrypt(ora.Plaintext.encode(v, "simd", par_o), rng) for v in values]
+    extended = ora.Multiplicator.default_extended_basis(par_o, 0)
+    want = ora.Multiplicator(ora.ScalingFactor.one(), ora.ScalingFactor.one(), extended, ora.ScalingFactor(3, 1001), 0,
+                             par_o).multiply(*ct).to_array()
+    par = fg.BfvParameters(n, moduli, 65537)
+    mult = fg.Multiplicator.new_leveled(fg.ScalingFactor.one(), fg.ScalingFactor.one(), extended,
+                                        fg.ScalingFactor(3, 1001), 0, par)
+    got = fg.to_host(mult.multiply(*(fg.to_device(c.to_array()[None]) for c in ct)))[0]
+    assert np.array_equal(got, want)
+    assert fg.rns_tensor_wait_failures() == 0
