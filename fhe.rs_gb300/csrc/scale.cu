@@ -909,6 +909,33 @@ static bool uses_hat(const RnsScalerD& s, uint32_t logn, uint32_t out_len) {
   return s.hat && rns_tc_enabled() && out_len <= s.hat->maxt && logn >= 7;
 }
 
+// Whether it is the faster one where no strided stages come along. What it does
+// once a coefficient (operands, tensor memory, v and w) few outputs do not pay for:
+// k_rns_scale's products are as many as sources times outputs, and cheapest where
+// it has a kernel of the very count of sources (3, 6, 7) or a tensor-core form (12,
+// 13). The lines are the most outputs with which k_rns_scale was no slower at 2^19 or
+// 2^21 coefficients (k_rns_scale against k_rns_hat at 2^21, factor one: 3 sources to
+// 1 output 33 and 64 us, to 6 outputs 72 and 69; 6 to 1 43 and 70, to 5 90 and 78; 10
+// to 1 88 and 101, to 2 109 and 104; 12 to 6 129 and 156; 13 to 7 146 and 148; with
+// fractions 3 to 1 54 and 72, to 3 82 and 73; 12 to 1 108 and 115, to 3 134 and 124). Grids up to
+// kMaxDependentCtas start k_rns_hat behind the kernel before, which makes up for it
+// but at 12 and 13 sources (2^18 coefficients: 3 to 1 14 and 10 us, 10 to 1 14.7 and
+// 15.3, 13 to 4 18.5 and 19.5, 12 to 7 18.9 and 19.7, to 8 23.8 and 22.0).
+static bool hat_pays(const RnsScalerD& s, uint32_t out_len, uint64_t total) {
+  static constexpr uint8_t kOne[17] = {0, 3, 3, 5, 2, 2, 4, 3, 1, 1, 1, 1, 11, 7, 1, 1, 1};
+  static constexpr uint8_t kFractions[17] = {0, 1, 1, 2, 0, 0, 1, 0, 0, 0, 0, 0, 1, 1, 0, 0, 0};
+  const size_t F = s.host.from_len;
+  if (F > 16) return true;
+  const bool one = s.host.is_one;
+  if (total <= 128 * kMaxDependentCtas) {
+    const uint32_t few = !one || F < 9 ? 0 : F == 12 ? 7 : F == 13 ? 4 : 1;
+    return out_len > few;
+  }
+  if (one && F == 12 && out_len > 14) return false;  // tensor memory halves the CTAs of an SM
+  if (!one && F == 12 && s.hat->frac > 7) return out_len > 2;  // the kernel of twice the terms of w
+  return out_len > (one ? kOne : kFractions)[F];
+}
+
 bool rns_scale_takes_top(const RnsScalerD& s, uint32_t logn, uint32_t out_len, uint32_t s1, bool fold) {
   if (fold && uses_hat(s, logn, out_len)) return s1 >= 1 && s1 <= 3;
   const size_t F = s.host.from_len;
@@ -923,7 +950,7 @@ void rns_scale(const RnsScalerD& s, uint32_t logn, PolyRef in, PolyRef out, uint
   const size_t F = s.host.from_len;
   if (fwd && (!top || fwd->s1 != top->s1))
     throw Error(FHEG_ERR_INTERNAL, "forward strided stages need the same count of inverse ones");
-  if (uses_hat(s, logn, out_len) && (!top || top->fold)) {
+  if (uses_hat(s, logn, out_len) && (top ? top->fold : hat_pays(s, out_len, total))) {
     rns_scale_hat(s, logn, in, out, start, out_len, polys, st, top, fwd);
     return;
   }

@@ -119,3 +119,41 @@ def test_products_with_a_fraction_at_every_source(fg, ora, cuda, n, L):
     got = fg.to_host(mult.multiply(*(fg.to_device(c.to_array()[None]) for c in ct)))[0]
     assert np.array_equal(got, want)
     assert fg.rns_tensor_wait_failures() == 0
+
+
+# Sources and outputs on either side of the lines between the two kernels of large launches.
+LINES = [(1, 3, "one"), (1, 4, "one"), (3, 5, "one"), (3, 6, "one"), (6, 4, "one"), (6, 5, "one"), (7, 3, "one"),
+         (7, 4, "one"), (8, 1, "one"), (8, 2, "one"), (12, 11, "one"), (12, 12, "one"), (12, 14, "one"), (12, 15, "one"),
+         (13, 7, "one"), (13, 8, "one"), (16, 1, "one"), (16, 2, "one"), (1, 1, "t_over_q"), (1, 2, "t_over_q"),
+         (3, 2, "t_over_q"), (3, 3, "t_over_q"), (6, 1, "t_over_q"), (6, 2, "t_over_q"), (12, 1, "t_over_half"),
+         (12, 2, "t_over_half"), (12, 2, "t_over_q"), (12, 3, "t_over_q"), (13, 1, "t_over_q"), (13, 2, "t_over_q")]
+
+
+@pytest.mark.parametrize("F,T,factor", LINES)
+def test_large_scalings(fg, ora, cuda, F, T, factor):
+    """20 polynomials at 2^14, more than a dependent launch takes, against the same ones scaled singly and with the
+    tensor cores off, the first one (rounding boundaries) against the oracle."""
+    n, count = 16384, 20
+    rng = np.random.default_rng(F * 64 + T)
+    pool = _primes(ora, n, F + T, True)
+    frm, to = pool[:F], pool[F:]
+    full, half = ora.RnsContext(frm).modulus(), ora.RnsContext(frm[:(F + 1) // 2]).modulus()
+    num, den = {"one": (1, 1), "t_over_half": (65537, half), "t_over_q": (65537, full)}[factor]
+    frm_o, to_o = ora.Context(frm, n), ora.Context(to, n)
+    sc_o = ora.Scaler(frm_o, to_o, ora.ScalingFactor(num, den) if num != den else ora.ScalingFactor.one())
+    sc = fg.Scaler(fg.Context(frm, n), fg.Context(to, n),
+                   fg.ScalingFactor(num, den) if num != den else fg.ScalingFactor.one())
+    x = rng.integers(0, 1 << 62, (count, F, n), dtype=np.uint64) % np.array(frm, dtype=np.uint64)[:, None]
+    pb = ora.Poly.from_biguints(frm_o, _coefficients(full, num, den, n, rng))
+    x[0] = pb.coefficients
+    t = fg.to_device(x)
+    got = fg.to_host(sc.scale(t, 0))
+    assert np.array_equal(got[0], sc_o.scale(pb).coefficients)
+    assert np.array_equal(got, np.concatenate([fg.to_host(sc.scale(t[i:i + 1], 0)) for i in range(count)]))
+    default = fg.rns_tensor_get()
+    fg.rns_tensor_set(False)
+    try:
+        assert np.array_equal(got, fg.to_host(sc.scale(t, 0)))
+    finally:
+        fg.rns_tensor_set(default)
+    assert fg.rns_tensor_wait_failures() == 0
