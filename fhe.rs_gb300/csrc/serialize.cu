@@ -61,15 +61,18 @@ __device__ __forceinline__ uint64_t pack_word(const uint64_t* row, uint32_t n, u
   return word;
 }
 
-// Packed payloads of whole limbs: row blockIdx.y (polynomial * limbs + limb),
-// two words of its stream per thread, stored together when the destination
-// is aligned to 16 bytes, as one word each when to 8, else byte by byte (a limb's
-// last word may be short). A grid over rows leaves no 64-bit divisions: the kernel
-// over flat indexes spent its time on them (128 polynomials of 2^14 x 6: 100 us).
+// Packed payloads of whole limbs: blockDim.y rows (polynomial * limbs + limb) a
+// CTA, two words of a row's stream per thread, stored together when the
+// destination is aligned to 16 bytes, else by 8, 4 or 2 bytes as it is aligned to, or
+// byte by byte (a limb's last word may be short). A grid over rows leaves no 64-bit divisions:
+// the kernel over flat indexes spent its time on them (128 polynomials of 2^14 x 6:
+// 100 us). Rows below 512 words share a CTA: with one each, 65536 polynomials of
+// 2^4 x 2 took 99 us against 25 over flat indexes, and take 21 so.
 __global__ void __launch_bounds__(256) k_pack(const __grid_constant__ PackLayout lay, const PolyRef in, uint8_t* out,
-                                              uint32_t row0) {
-  const uint32_t r = row0 + blockIdx.y, poly = r / lay.limbs, j = r - poly * lay.limbs;
-  const uint32_t c = 2 * (blockIdx.x * 256 + threadIdx.x);
+                                              uint32_t row0, uint32_t rows) {
+  const uint32_t r = row0 + blockIdx.y * blockDim.y + threadIdx.y, poly = r / lay.limbs, j = r - poly * lay.limbs;
+  if (r >= rows) return;
+  const uint32_t c = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
   const uint32_t bytes = (uint32_t)(lay.offset[j + 1] - lay.offset[j]);
   if (c * 8 >= bytes) return;
   const uint32_t n = 1u << lay.logn, nb = lay.nbits[j];
@@ -83,6 +86,20 @@ __global__ void __launch_bounds__(256) k_pack(const __grid_constant__ PackLayout
   if (c * 8 + 16 <= bytes && ((uintptr_t)dst & 7) == 0) {
     reinterpret_cast<uint64_t*>(dst)[0] = w0;
     reinterpret_cast<uint64_t*>(dst)[1] = w1;
+    return;
+  }
+  if (c * 8 + 16 <= bytes && ((uintptr_t)dst & 1) == 0) {
+    const uint32_t v[4] = {(uint32_t)w0, (uint32_t)(w0 >> 32), (uint32_t)w1, (uint32_t)(w1 >> 32)};
+    const bool four = ((uintptr_t)dst & 3) == 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      if (four) {
+        reinterpret_cast<uint32_t*>(dst)[q] = v[q];
+      } else {
+        reinterpret_cast<uint16_t*>(dst)[2 * q] = (uint16_t)v[q];
+        reinterpret_cast<uint16_t*>(dst)[2 * q + 1] = (uint16_t)(v[q] >> 16);
+      }
+    }
     return;
   }
   const uint32_t left = bytes - c * 8 < 16 ? bytes - c * 8 : 16;
@@ -167,9 +184,13 @@ void pack_polys(const Context& c, int representation, PolyRef in, uint8_t* bytes
   uint64_t longest = 0;
   for (uint32_t j = 0; j < lay.limbs; j++) longest = std::max(longest, lay.offset[j + 1] - lay.offset[j]);
   const uint64_t rows = count * lay.limbs;
-  for (uint64_t r = 0; r < rows; r += 65535) {  // the grid's limit along y
-    k_pack<<<dim3(nblk((longest + 15) / 16, 256), (unsigned)std::min<uint64_t>(65535, rows - r)), 256, 0, st>>>(
-        lay, src, bytes, (uint32_t)r);
+  const unsigned pairs = nblk(longest, 16);
+  unsigned tx = 256;
+  while (tx > 4 && tx / 2 >= pairs) tx /= 2;
+  const unsigned ty = 256 / tx;
+  for (uint64_t r = 0; r < rows; r += 65535ull * ty) {  // the grid's limit along y
+    const unsigned gy = (unsigned)std::min<uint64_t>(65535, (rows - r + ty - 1) / ty);
+    k_pack<<<dim3(nblk(pairs, tx), gy), dim3(tx, ty), 0, st>>>(lay, src, bytes, (uint32_t)r, (uint32_t)rows);
     after_launch("k_pack");
   }
 }
