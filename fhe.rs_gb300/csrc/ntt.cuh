@@ -530,6 +530,9 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, FOLD && src_is_montgomery<S
 // Small transforms (N <= 2^11, used by small parameter sets and tests): one
 // CTA per limb, radix-2 stages in shared memory, the size a runtime value.
 // Same butterflies and twiddle indices as above, so the same outputs.
+// Large grids leave the next kernel's start to the ends of their CTAs: a trigger
+// takes about a nanosecond a CTA, whatever its size (131072 limbs of 2^3 forward: 134
+// us with it, 72 without; 2^9 and up no difference).
 
 template <bool REDUCE, class Src, class Dst>
 __global__ void __launch_bounds__(1024) k_ntt_fwd_small(NttGeom g, uint32_t logn, Src src, Dst dst) {
@@ -553,7 +556,7 @@ __global__ void __launch_bounds__(1024) k_ntt_fwd_small(NttGeom g, uint32_t logn
     }
     __syncthreads();
   }
-  pdl_trigger();
+  if (gridDim.x <= kMaxDependentCtas) pdl_trigger();
   for (uint32_t i = tid; i < n; i += nt) dst(jb, pr, i, REDUCE ? reduce4(sm[i], pr.p, pr.p2) : sm[i]);
 }
 
@@ -579,7 +582,7 @@ __global__ void __launch_bounds__(1024) k_ntt_inv_small(NttGeom g, uint32_t logn
     }
     __syncthreads();
   }
-  pdl_trigger();
+  if (gridDim.x <= kMaxDependentCtas) pdl_trigger();
   for (uint32_t i = tid; i < n; i += nt) dst(jb, pr, i, inv_final_scale(g, pr, sm[i]));
 }
 

@@ -29,3 +29,25 @@ def test_context_is_complete_on_return(fg, ora, cuda, logn):
         want = row.copy()
         ora.ntt_operator(below, n).forward(want)
         assert np.array_equal(got[0, 0], want)
+
+
+@pytest.mark.parametrize("logn,count", [(3, 1), (3, 1216), (3, 1217), (3, 5000), (6, 1216), (6, 3000), (9, 1217), (11, 1300)])
+def test_chains_of_small_transforms(fg, ora, cuda, logn, count):
+    """Launches that each wait for the one before, on either side of the grid size up to which they start early."""
+    n = 1 << logn
+    moduli = [ora.generate_prime(bits, 2 * n, 1 << bits) for bits in (39, 61)]
+    ctx = fg.Context(moduli, n)
+    x = np.random.default_rng(logn).integers(0, 1 << 38, (count, 2, n), dtype=np.uint64)
+    want = x.copy()
+    for b in {0, count // 2, count - 1}:
+        for j, p in enumerate(moduli):
+            ora.ntt_operator(p, n).forward(want[b, j])
+    t = fg.to_device(x)
+    for _ in range(20):
+        fg.ntt_forward(ctx, t)
+        fg.ntt_backward(ctx, t)
+    assert np.array_equal(fg.to_host(t), x)
+    fg.ntt_forward(ctx, t)
+    got = fg.to_host(t)
+    for b in {0, count // 2, count - 1}:
+        assert np.array_equal(got[b], want[b])
