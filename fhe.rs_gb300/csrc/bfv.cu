@@ -1244,6 +1244,8 @@ void Multiplicator::multiply(const uint64_t* lhs, const uint64_t* rhs, uint64_t*
   };
   const uint32_t bl_a = plan_a ? plan_a : ntt_block_logn(logn), bl_d = plan_d ? plan_d : ntt_block_logn(logn);
 
+  // The scalers' switch, which another thread may turn meanwhile.
+  const bool tc = rns_tc_enabled();
   // Strided last stages of a two-pass inverse NTT that the RNS scaler after
   // it can apply while loading (its only consumer): 0 when the plan is single
   // pass or the scaler cannot.
@@ -1252,8 +1254,8 @@ void Multiplicator::multiply(const uint64_t* lhs, const uint64_t* rhs, uint64_t*
     if (bl >= logn || logn < 13) return 0;
     const uint32_t s1 = logn - bl;
     const bool folds = fold && bl == 12;
-    if (!rns_scale_takes_top(*s1c.rns, logn, out_len, s1, folds)) return 0;
-    if (s2c && !rns_scale_takes_top(*s2c->rns, logn, out_len, s1, folds)) return 0;
+    if (!rns_scale_takes_top(*s1c.rns, logn, out_len, s1, folds, tc)) return 0;
+    if (s2c && !rns_scale_takes_top(*s2c->rns, logn, out_len, s1, folds, tc)) return 0;
     return s1;
   };
 
@@ -1266,7 +1268,7 @@ void Multiplicator::multiply(const uint64_t* lhs, const uint64_t* rhs, uint64_t*
     if (top_a) ntt_inverse_blocks(logn, g, 4 * count, SrcPair{lref, rref}, DstPoly{pbref}, st, plan_a);
     else ntt_inverse_any(logn, g, 4 * count, SrcPair{lref, rref}, DstPoly{pbref}, st, plan_a);
   }
-  const InverseTop top_a_args{top_a, 0u, bc.primes_dev(), fold && bl_a == 12};
+  const InverseTop top_a_args{top_a, 0u, bc.primes_dev(), fold && bl_a == 12, tc};
   mark(1);
   // B + C: extension of each operand and forward NTT of the new limbs.
   const bool same_ext = ncm_l == ncm_r && ext_lhs->num == ext_rhs->num && ext_lhs->den == ext_rhs->den;
@@ -1320,7 +1322,7 @@ void Multiplicator::multiply(const uint64_t* lhs, const uint64_t* rhs, uint64_t*
   // E: scale down by t/Q into the base context (power basis), applying the
   // strided last stages of D's inverse NTT (Montgomery products) on the way.
   PolyRef dnref = plain_ref(dn, L, logn);
-  const InverseTop top_d_args{top_d, 1u, mc.primes_dev(), fold && bl_d == 12};
+  const InverseTop top_d_args{top_d, 1u, mc.primes_dev(), fold && bl_d == 12, tc};
   // F's strided first stages run in E's epilogue when F's plan has as many as
   // D's: c0 and c1 get them over their own limbs (left in dn for F's block
   // pass), and c2 is expanded there into the digit rows of every key modulus

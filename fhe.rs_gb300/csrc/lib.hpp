@@ -181,6 +181,7 @@ struct InverseTop {
   uint32_t mont;
   const DevPrime* primes;
   bool fold = false;
+  bool tc = false;  // the tensor-core switch as rns_scale_takes_top was asked with
 };
 // The strided first stages of two-pass forward NTTs applied by their
 // producer, the RNS scaler: `s1` stages. Polynomials with poly % period <
@@ -208,7 +209,7 @@ void rns_scale(const RnsScalerD& s, uint32_t logn, PolyRef in, PolyRef out, uint
 bool rns_tc_enabled();
 void set_rns_tc(bool on);
 uint64_t rns_tc_wait_failures();
-bool rns_scale_takes_top(const RnsScalerD& s, uint32_t logn, uint32_t out_len, uint32_t s1, bool fold);
+bool rns_scale_takes_top(const RnsScalerD& s, uint32_t logn, uint32_t out_len, uint32_t s1, bool fold, bool tc);
 // The scaler of scale_hat.cu (s.hat set, out_len <= s.hat->maxt, logn >= 7) and
 // its construction (null where it does not apply).
 void rns_scale_hat(const RnsScalerD& s, uint32_t logn, PolyRef in, PolyRef out, uint32_t start, uint32_t out_len,

@@ -905,8 +905,8 @@ static void launch_rns_scale_top(const RnsScalerD& s, uint32_t logn, PolyRef in,
 }
 
 // Whether scale_hat.cu takes the call.
-static bool uses_hat(const RnsScalerD& s, uint32_t logn, uint32_t out_len) {
-  return s.hat && rns_tc_enabled() && out_len <= s.hat->maxt && logn >= 7;
+static bool uses_hat(const RnsScalerD& s, uint32_t logn, uint32_t out_len, bool tc) {
+  return s.hat && tc && out_len <= s.hat->maxt && logn >= 7;
 }
 
 // Whether it is the faster one where no strided stages come along. What it does
@@ -936,8 +936,8 @@ static bool hat_pays(const RnsScalerD& s, uint32_t out_len, uint64_t total) {
   return out_len > (one ? kOne : kFractions)[F];
 }
 
-bool rns_scale_takes_top(const RnsScalerD& s, uint32_t logn, uint32_t out_len, uint32_t s1, bool fold) {
-  if (fold && uses_hat(s, logn, out_len)) return s1 >= 1 && s1 <= 3;
+bool rns_scale_takes_top(const RnsScalerD& s, uint32_t logn, uint32_t out_len, uint32_t s1, bool fold, bool tc) {
+  if (fold && uses_hat(s, logn, out_len, tc)) return s1 >= 1 && s1 <= 3;
   const size_t F = s.host.from_len;
   const bool exact = (F == 6 || F == 13 || F == 3 || F == 7) ? out_len <= 8 : (F == 12 || F == 25) && out_len <= 16;
   return exact && s.mont && s1 >= 1 && s1 <= 3 && logn >= 7;
@@ -950,12 +950,14 @@ void rns_scale(const RnsScalerD& s, uint32_t logn, PolyRef in, PolyRef out, uint
   const size_t F = s.host.from_len;
   if (fwd && (!top || fwd->s1 != top->s1))
     throw Error(FHEG_ERR_INTERNAL, "forward strided stages need the same count of inverse ones");
-  if (uses_hat(s, logn, out_len) && (top ? top->fold : hat_pays(s, out_len, total))) {
+  // Read once: with strided stages, the value their layout was chosen by.
+  const bool tc = top ? top->tc : rns_tc_enabled();
+  if (uses_hat(s, logn, out_len, tc) && (top ? top->fold : hat_pays(s, out_len, total))) {
     rns_scale_hat(s, logn, in, out, start, out_len, polys, st, top, fwd);
     return;
   }
   if (top) {
-    if (!rns_scale_takes_top(s, logn, out_len, top->s1, top->fold))
+    if (!rns_scale_takes_top(s, logn, out_len, top->s1, top->fold, tc))
       throw Error(FHEG_ERR_INTERNAL, "RNS scaling cannot apply these strided stages");
     if (F == 6) launch_rns_scale_top<6, 8>(s, logn, in, out, start, out_len, total, st, *top, fwd);
     else if (F == 13) launch_rns_scale_top<13, 8>(s, logn, in, out, start, out_len, total, st, *top, fwd);

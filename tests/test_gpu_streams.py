@@ -51,3 +51,41 @@ def test_chains_of_small_transforms(fg, ora, cuda, logn, count):
     got = fg.to_host(t)
     for b in {0, count // 2, count - 1}:
         assert np.array_equal(got[b], want[b])
+
+
+def test_tensor_switch_turned_during_products(fg, ora, cuda):
+    """The scalers' switch is process-wide: a thread that turns it on and off while another multiplies changes neither
+    the products nor whether they are accepted (five moduli: the strided stages run in the scalers with it, and in passes of
+    their own without)."""
+    import threading
+
+    n = 16384
+    moduli, ub = [], 1 << 62
+    for _ in range(5):
+        ub = ora.generate_prime(62, 2 * n, ub)
+        moduli.append(ub)
+    rng = np.random.default_rng(5)
+    q = np.array(moduli, dtype=np.uint64)[:, None]
+    rows = rng.integers(0, 1 << 62, (2, 5, 5, n), dtype=np.uint64) % q
+    x, y = (fg.to_device(rng.integers(0, 1 << 62, (1, 2, 5, n), dtype=np.uint64) % q) for _ in range(2))
+    mult = fg.Multiplicator.default(fg.RelinearizationKey(fg.BfvParameters(n, moduli, 65537), rows[0], rows[1]))
+    default, done = fg.rns_tensor_get(), threading.Event()
+    want = fg.to_host(mult.multiply(x, y))
+
+    def turn():
+        while not done.is_set():
+            fg.rns_tensor_set(False)
+            fg.rns_tensor_set(True)
+
+    thread = threading.Thread(target=turn)
+    thread.start()
+    try:
+        for _ in range(2000):
+            out = mult.multiply(x, y)
+        for _ in range(50):
+            assert np.array_equal(fg.to_host(mult.multiply(x, y)), want)
+    finally:
+        done.set()
+        thread.join()
+        fg.rns_tensor_set(default)
+    assert np.array_equal(fg.to_host(out), want)
