@@ -277,8 +277,11 @@ def _dp(t) -> int:
 def _stream() -> int:
     # The raw handle of torch.cuda.current_stream() without its Stream object: 0.3
     # against 2.8 us a call, where the smallest transforms take 6 us on the device.
+    # The function is torch's own (its compiled code calls it), so a torch without
+    # it gets the handle from the object.
     torch = _torch()
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return raw(torch.cuda.current_device()) if raw else torch.cuda.current_stream().cuda_stream
 
 
 def empty(shape, device="cuda"):
