@@ -89,3 +89,73 @@ def test_tensor_switch_turned_during_products(fg, ora, cuda):
         thread.join()
         fg.rns_tensor_set(default)
     assert np.array_equal(fg.to_host(out), want)
+
+
+@pytest.mark.parametrize("n,L", [(4096, 2), (16384, 3), (32768, 4)])
+def test_two_streams_with_copies_and_waits(fg, ora, cuda, n, L):
+    """Products on one stream feed rotations on another and back, with copies and event waits in between and transforms
+    on both: the same words as one call after the other."""
+    torch = cuda
+    moduli, ub = [], 1 << 62
+    for _ in range(L):
+        ub = ora.generate_prime(62, 2 * n, ub)
+        moduli.append(ub)
+    rng = np.random.default_rng(n)
+    q = np.array(moduli, dtype=np.uint64)[:, None]
+
+    def residues(*lead):
+        return rng.integers(0, 1 << 62, (*lead, L, n), dtype=np.uint64) % q
+
+    par, ctx = fg.BfvParameters(n, moduli, 65537), fg.Context(moduli, n)
+    rk, gk = residues(2, L), residues(2, L)
+    mult = fg.Multiplicator.default(fg.RelinearizationKey(par, rk[0], rk[1]))
+    gk = fg.GaloisKey(par, 3, gk[0], gk[1])
+    first, other = residues(2, 2), residues(2, 2)
+    pinned = torch.from_numpy(other.view(np.int64)).pin_memory()
+    torch.cuda.synchronize()
+
+    def run(a, b, serial):
+        def after():
+            if serial:
+                torch.cuda.synchronize()
+
+        with torch.cuda.stream(a):
+            x, w = fg.to_device(first), fg.to_device(first[:, 0])
+        with torch.cuda.stream(b):
+            v = fg.to_device(first[:, 1])
+        torch.cuda.synchronize()
+        for _ in range(12):
+            with torch.cuda.stream(a):
+                y = torch.empty_like(x)
+                y.copy_(pinned, non_blocking=True)
+                after()
+                product = mult.multiply(x, y)
+                after()
+                ready = a.record_event()
+                fg.ntt_forward(ctx, w)
+                fg.ntt_backward(ctx, w)
+                after()
+            with torch.cuda.stream(b):
+                fg.ntt_backward(ctx, v)
+                after()
+                b.wait_event(ready)
+                turned = gk.relinearize(product)
+                after()
+                fg.ntt_forward(ctx, v)
+                done = b.record_event()
+                after()
+            product.record_stream(b)
+            with torch.cuda.stream(a):
+                a.wait_event(done)
+                x.copy_(turned)
+                after()
+            turned.record_stream(a)
+        torch.cuda.synchronize()
+        return [fg.to_host(t) for t in (x, v, w)]
+
+    default = torch.cuda.default_stream()
+    want = run(default, default, True)
+    assert np.array_equal(want[1], first[:, 1]) and np.array_equal(want[2], first[:, 0])
+    for _ in range(3):
+        got = run(torch.cuda.Stream(), torch.cuda.Stream(), False)
+        assert all(np.array_equal(g, e) for g, e in zip(got, want))
