@@ -802,8 +802,14 @@ struct DstRotD {
 
 // G: out0 = substitute(ct0) + sum_d D[d] * k0[d], out1 = sum_d D[d] * k1[d]
 // for row (poly, limb) = rows[blockIdx.y]; exact sums reduced once. Requests
-// whose key switches down write the bare sums (key context) to ks instead.
+// whose key switches down write the bare sums (key context) to ks instead. With
+// both reductions in one kernel it took 44 us at 2^14 x 6 x 32 of primes that do not
+// fold, and 41 with Barrett's alone.
+template <bool FOLD>
 __global__ void k_rot_mac(const DevPrime* primes, const RotDesc* d, const uint2* rows, uint32_t logn) {
+  const auto reduce = [](uint64_t hi, uint64_t lo, const DevPrime& pr) {
+    return FOLD ? reduce_sum(hi, lo, pr) : reduce128(hi, lo, pr);
+  };
   pdl_wait();
   const uint2 row = rows[blockIdx.y];
   const RotDesc& r = d[row.x];
@@ -820,14 +826,14 @@ __global__ void k_rot_mac(const DevPrime* primes, const RotDesc* d, const uint2*
     mac128(hi0, lo0, x, __ldg(r.k0 + off));
     mac128(hi1, lo1, x, __ldg(r.k1 + off));
     if (dd % 15 == 14) {
-      lo0 = reduce_sum(hi0, lo0, pr);
+      lo0 = reduce(hi0, lo0, pr);
       hi0 = 0;
-      lo1 = reduce_sum(hi1, lo1, pr);
+      lo1 = reduce(hi1, lo1, pr);
       hi1 = 0;
     }
   }
-  o[((uint64_t)j << logn) + i] = reduce_sum(hi0, lo0, pr);
-  o[plane + ((uint64_t)j << logn) + i] = reduce_sum(hi1, lo1, pr);
+  o[((uint64_t)j << logn) + i] = reduce(hi0, lo0, pr);
+  o[plane + ((uint64_t)j << logn) + i] = reduce(hi1, lo1, pr);
 }
 
 // Switch-down of the requests whose key lies below their level
@@ -1016,15 +1022,25 @@ static RotBatchPlan prepare_rot_batch(const Params& par, const RotRequest* req, 
     Dpos += (size_t)r.nd * Lk * N;
     max_l = std::max(max_l, std::max(L, Lk));
   }
-  // The jobs of the two large launches by limb: CTAs that run together then
-  // share the limb's twiddles.
-  for (uint32_t i = 0; i < max_l; i++)
+  // The jobs of the two large launches: by limb where the transforms fold, so that
+  // CTAs that run together share the limb's twiddles; else by ciphertext, whose
+  // digits then come from L2 (32 rotations at 2^15 x 6 of primes that do not fold:
+  // 762 us by limb, 756 so).
+  if (par.ctx(0)->fold) {
+    for (uint32_t i = 0; i < max_l; i++)
+      for (size_t b = 0; b < count; b++)
+        if (i < desc[b].L) jobs.push_back(make_uint4((uint32_t)b, i, 0, 0));
+    for (uint32_t j = 0; j < max_l; j++)
+      for (size_t b = 0; b < count; b++)
+        if (j < desc[b].Lk)
+          for (uint32_t dd = 0; dd < desc[b].nd; dd++) jobs.push_back(make_uint4((uint32_t)b, j, dd, 0));
+  } else {
     for (size_t b = 0; b < count; b++)
-      if (i < desc[b].L) jobs.push_back(make_uint4((uint32_t)b, i, 0, 0));
-  for (uint32_t j = 0; j < max_l; j++)
+      for (uint32_t i = 0; i < desc[b].L; i++) jobs.push_back(make_uint4((uint32_t)b, i, 0, 0));
     for (size_t b = 0; b < count; b++)
-      if (j < desc[b].Lk)
-        for (uint32_t dd = 0; dd < desc[b].nd; dd++) jobs.push_back(make_uint4((uint32_t)b, j, dd, 0));
+      for (uint32_t dd = 0; dd < desc[b].nd; dd++)
+        for (uint32_t j = 0; j < desc[b].Lk; j++) jobs.push_back(make_uint4((uint32_t)b, j, dd, 0));
+  }
   for (size_t b = 0; b < count; b++)
     if (desc[b].ks)
       for (uint32_t part = 0; part < 2; part++)
@@ -1081,7 +1097,8 @@ static void launch_rot_batch(const RotBatchPlan& pl, cudaStream_t st) {
   ntt_forward_any<true>(logn, g2, cnt.n_f, SrcRotDigit{d_desc, logn}, DstRotD{d_desc, logn}, st);
   // G: inner products and the substituted c0.
   const unsigned gx = (unsigned)((N + 255) / 256);
-  launch_dependent(k_rot_mac, dim3(gx, (unsigned)cnt.n_rows), 256, 0, st, top.primes_dev(), d_desc, d_rows, logn);
+  launch_dependent(top.fold ? k_rot_mac<true> : k_rot_mac<false>, dim3(gx, (unsigned)cnt.n_rows), 256, 0, st,
+                   top.primes_dev(), d_desc, d_rows, logn);
   after_launch("k_rot_mac");
   if (cnt.n_chain == 0) return;
   // Requests with keys below their level: the sums into the power basis, down

@@ -624,8 +624,11 @@ __device__ __forceinline__ void fwd_top_stages(uint64_t* x, const DevPrime& pr) 
   }
 }
 
+// At most 64 registers up to eight residues: the rotations' source came out with 66
+// in Harvey's arithmetic, three CTAs an SM instead of four (2^15 x 6 x 32: 88 us
+// instead of 84).
 template <int S1, bool FOLD, class Src, class Dst>
-__global__ void __launch_bounds__(256) k_ntt_fwd_top(NttGeom g, uint32_t logb, uint32_t groups_per_limb,
+__global__ void __launch_bounds__(256, S1 <= 3 ? 4 : 0) k_ntt_fwd_top(NttGeom g, uint32_t logb, uint32_t groups_per_limb,
                                                      uint64_t total, Src src, Dst dst) {
   pdl_wait();
   const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
