@@ -266,6 +266,10 @@ struct NttShape {
   // -> 97, inverse 109 -> 115).
   static constexpr int MIN_BLOCKS = LOGN == 12 ? 3 : LOGN == 11 ? 6 : (T >= 512 ? 1 : (512 / T > 32 ? 32 : 512 / T));
   static constexpr int FOLD_BLOCKS = LOGN == 12 ? 4 : MIN_BLOCKS;
+  // Whether the next kernel starts early. Blocks of 2^13, one CTA an SM, lose 2-4% by
+  // the trigger (inverse of 32 pairs at 2^14 x 6: 166 us with it, 160 without); those of
+  // 2^14 gain 0.7%.
+  static constexpr bool EARLY = LOGN != 13;
 };
 
 // One forward round: global stages S0 .. S0+K-1 of a transform of size 2^LOGN
@@ -380,7 +384,7 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, NttShape<LOGN>::MIN_BLOCKS)
 #pragma unroll
   for (int e = 0; e < E; e++) x[e] = src_load<FOLD>(src, jb, pr, base + tid + e * T);
   fwd_rounds<LOGN, 0, FOLD>(x, sm, tid, pr, (1u << g.s1) + jb.beta);
-  pdl_trigger();
+  if constexpr (NttShape<LOGN>::EARLY) pdl_trigger();
   const uint32_t sb = swz8(tid);
 #pragma unroll
   for (int e = 0; e < E; e++) {
@@ -516,7 +520,7 @@ __global__ void __launch_bounds__(NttShape<LOGN>::T, FOLD && src_is_montgomery<S
   __syncthreads();
   inv_from_smem<LOGN, 0, K0>(x, sm, tid);
   inv_rounds<LOGN, 0, K0, FOLD>(x, sm, tid, pr, 1u << (LOGN + g.s1), g.s1, jb.beta);
-  pdl_trigger();
+  if constexpr (NttShape<LOGN>::EARLY) pdl_trigger();
   // The last round holds elements tid + e*T (b = tid, c = 0): coalesced stores.
 #pragma unroll
   for (int e = 0; e < E; e++) {
@@ -984,7 +988,7 @@ void launch_fwd_block_as(NttGeom g, uint64_t polys, Src src, Dst dst, cudaStream
   g.pf_stride = ntt_prefetch_enabled() ? resident_ctas(kern, NttShape<LOGN>::T, smem, &resident) : 0;
   const uint64_t blocks = polys * g.limbs << g.s1;
   g.units = (uint32_t)polys;
-  launch_dependent<true>(kern, dim3((unsigned)blocks), NttShape<LOGN>::T, smem, st, g, src, dst);
+  launch_dependent<NttShape<LOGN>::EARLY>(kern, dim3((unsigned)blocks), NttShape<LOGN>::T, smem, st, g, src, dst);
   after_launch("k_ntt_fwd");
 }
 
@@ -1008,7 +1012,7 @@ void launch_inv_block_as(NttGeom g, uint64_t polys, Src src, Dst dst, cudaStream
   g.pf_stride = ntt_prefetch_enabled() ? resident_ctas(kern, NttShape<LOGN>::T, smem, &resident) : 0;
   const uint64_t blocks = polys * g.limbs << g.s1;
   g.units = (uint32_t)polys;
-  launch_dependent<true>(kern, dim3((unsigned)blocks), NttShape<LOGN>::T, smem, st, g, src, dst);
+  launch_dependent<NttShape<LOGN>::EARLY>(kern, dim3((unsigned)blocks), NttShape<LOGN>::T, smem, st, g, src, dst);
   after_launch("k_ntt_inv");
 }
 
