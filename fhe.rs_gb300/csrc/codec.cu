@@ -346,7 +346,8 @@ void decrypt(const SecretKeyDev& sk, size_t level, size_t parts, const uint64_t*
                   DstPoly{plain_ref(pb, c.L(), logn)}, st);
   // t/Q scaling; only the first plaintext-context limb is read afterwards.
   const Scaler& sc = *ps.dec[level];
-  rns_scale(*sc.rns, logn, plain_ref(pb, c.L(), logn), plain_ref(d0, 1, logn), 0, 1, count, st);
+  rns_scale(*sc.rns, logn, plain_ref(pb, c.L(), logn), plain_ref(d0, 1, logn), 0, 1, count, st, nullptr, nullptr,
+            true);
   const SrcFinish fin{d0, par.plaintext, par.moduli[0], par.plaintext ? ~0ull / par.plaintext : 0, logn};
   if (!simd) {
     const uint64_t total = count << logn;

@@ -202,8 +202,11 @@ struct ForwardTop {
 // applies its last stages while loading (only where rns_scale_takes_top).
 // fwd != nullptr (with top, the same s1 and arithmetic): the outputs are written after the
 // first stages of the forward NTT that consumes them.
+// integers: the scaled values lie next to integers before they are rounded, as
+// decryption's do (schedules only).
 void rns_scale(const RnsScalerD& s, uint32_t logn, PolyRef in, PolyRef out, uint32_t start, uint32_t out_len,
-               uint64_t polys, cudaStream_t st, const InverseTop* top = nullptr, const ForwardTop* fwd = nullptr);
+               uint64_t polys, cudaStream_t st, const InverseTop* top = nullptr, const ForwardTop* fwd = nullptr,
+               bool integers = false);
 // Whether exact RNS scalings run on the tensor cores (default on), and the
 // count of that form's bounded waits that ran out since the process started.
 bool rns_tc_enabled();

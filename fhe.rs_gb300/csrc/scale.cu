@@ -956,11 +956,14 @@ static bool uses_hat(const RnsScalerD& s, uint32_t logn, uint32_t out_len, bool 
 // kMaxDependentCtas start k_rns_hat behind the kernel before, which makes up for it
 // but at 12 and 13 sources (2^18 coefficients: 3 to 1 14 and 10 us, 10 to 1 14.7 and
 // 15.3, 13 to 4 18.5 and 19.5, 12 to 7 18.9 and 19.7, to 8 23.8 and 22.0).
-static bool hat_pays(const RnsScalerD& s, uint32_t out_len, uint64_t total) {
+// Next to integers the kernels of 3 and 6 sources, which sum high words alone, take
+// the exact sums for every coefficient (decryption of 64 at 2^14 x 6: 207 us so, 189
+// with k_rns_hat; of random words 182 and 189).
+static bool hat_pays(const RnsScalerD& s, uint32_t out_len, uint64_t total, bool integers) {
   static constexpr uint8_t kOne[17] = {0, 3, 3, 5, 2, 2, 4, 3, 1, 1, 1, 1, 11, 7, 1, 1, 1};
   static constexpr uint8_t kFractions[17] = {0, 1, 1, 2, 0, 0, 1, 0, 0, 0, 0, 0, 1, 1, 0, 0, 0};
   const size_t F = s.host.from_len;
-  if (F > 16) return true;
+  if (F > 16 || (integers && (F == 3 || F == 6))) return true;
   const bool one = s.host.is_one;
   if (total <= 128 * kMaxDependentCtas) {
     const uint32_t few = !one || F < 9 ? 0 : F == 12 ? 7 : F == 13 ? 4 : 1;
@@ -979,7 +982,7 @@ bool rns_scale_takes_top(const RnsScalerD& s, uint32_t logn, uint32_t out_len, u
 }
 
 void rns_scale(const RnsScalerD& s, uint32_t logn, PolyRef in, PolyRef out, uint32_t start, uint32_t out_len,
-               uint64_t polys, cudaStream_t st, const InverseTop* top, const ForwardTop* fwd) {
+               uint64_t polys, cudaStream_t st, const InverseTop* top, const ForwardTop* fwd, bool integers) {
   const uint64_t total = polys << logn;
   if (total == 0 || out_len == 0) return;
   const size_t F = s.host.from_len;
@@ -987,7 +990,7 @@ void rns_scale(const RnsScalerD& s, uint32_t logn, PolyRef in, PolyRef out, uint
     throw Error(FHEG_ERR_INTERNAL, "forward strided stages need the same count of inverse ones");
   // Read once: with strided stages, the value their layout was chosen by.
   const bool tc = top ? top->tc : rns_tc_enabled();
-  if (uses_hat(s, logn, out_len, tc) && (top ? top->fold : hat_pays(s, out_len, total))) {
+  if (uses_hat(s, logn, out_len, tc) && (top ? top->fold : hat_pays(s, out_len, total, integers))) {
     rns_scale_hat(s, logn, in, out, start, out_len, polys, st, top, fwd);
     return;
   }

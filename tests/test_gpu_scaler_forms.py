@@ -157,3 +157,26 @@ def test_large_scalings(fg, ora, cuda, F, T, factor):
     finally:
         fg.rns_tensor_set(default)
     assert fg.rns_tensor_wait_failures() == 0
+
+
+@pytest.mark.parametrize("L", [1, 3, 6, 12, 13])
+@pytest.mark.parametrize("count", [1, 40])
+def test_decryption_of_encryptions(fg, ora, cuda, L, count):
+    """Phases next to integers, in small and large launches: the values that went in, and the same with the tensor cores
+    off."""
+    n = 16384
+    moduli = _primes(ora, n, L, True)
+    rng = np.random.default_rng(L)
+    par = fg.BfvParameters(n, moduli, 65537)
+    sk = fg.SecretKey(par, rng.integers(-1, 2, n))
+    values = rng.integers(0, 65537, (count, n), dtype=np.uint64)
+    a = rng.integers(0, 1 << 62, (count, L, n), dtype=np.uint64) % np.array(moduli, dtype=np.uint64)[:, None]
+    errors = cuda.from_numpy(rng.integers(-9, 10, (count, n), dtype=np.int64)).cuda()
+    ct = sk.encrypt(fg.to_device(values), fg.to_device(a), errors)
+    assert np.array_equal(fg.to_host(sk.decrypt(ct)), values)
+    default = fg.rns_tensor_get()
+    fg.rns_tensor_set(False)
+    try:
+        assert np.array_equal(fg.to_host(sk.decrypt(ct)), values)
+    finally:
+        fg.rns_tensor_set(default)
