@@ -64,18 +64,18 @@ STAGE_LAUNCHES = {"A": 1, "B": 1, "C": 1, "D": 1, "E": 1, "F": 2, "G": 1}
 # strided NTT stage applied inside the RNS scalers B and E; E's sums on the
 # tensor cores), from the ncu capture summarised in
 # profiles/stages_mul_relin_n16384_b64.md.
-STAGE_TRAFFIC_BYTES = {"A": 352.5e6, "B": 397.1e6, "C": 408.4e6, "D": 747.5e6, "E": 682.5e6, "F": 694.1e6,
-                       "G": 494.1e6}
+STAGE_TRAFFIC_BYTES = {"A": 352.7e6, "B": 396.8e6, "C": 408.5e6, "D": 747.4e6, "E": 682.0e6, "F": 694.3e6,
+                       "G": 494.0e6}
 # The ncu figures above and below hold for the library sources they were
 # captured on: library_source_hash() of that tree. A run on other sources
 # reports null for them instead of stale numbers.
-PROFILED_SOURCE_HASH = "6f5666bf458147df"
+PROFILED_SOURCE_HASH = "bcf5169b2dcd3cd9"
 # Share of the elapsed cycles in which the integer multipliers (the FMA-heavy
 # pipe, which executes every IMAD) were busy, per stage, from the same ncu
 # capture of one 64-pair multiplication (F: time-weighted over its two
 # launches); the whole multiplication, time-weighted.
-STAGE_FMAHEAVY_PCT = {"A": 68.6, "B": 61.0, "C": 71.5, "D": 68.5, "E": 58.9, "F": 70.8, "G": 64.6}
-MULTIPLY_FMAHEAVY_PCT = 66.4
+STAGE_FMAHEAVY_PCT = {"A": 68.5, "B": 61.1, "C": 71.4, "D": 68.5, "E": 59.0, "F": 70.5, "G": 64.6}
+MULTIPLY_FMAHEAVY_PCT = 66.3
 
 
 def library_source_hash() -> str:

@@ -15,13 +15,14 @@ namespace fheg {
 std::atomic<uint64_t> g_launches{0};
 
 // Default NTT plan: single pass up to 2^12 (the whole limb in shared memory);
-// 2^13 to 2^16 in 2^12-residue blocks, which run three CTAs per SM. At 2^13
-// and 2^14 the blocks of a limb form one cluster that exchanges the strided
-// stages through distributed shared memory (GB300, 256 x 6 limbs, forward /
+// 2^13 to 2^16 in 2^12-residue blocks, which run three CTAs per SM (four where
+// they fold in clusters). At 2^13 and 2^14, and at 2^15 in fold arithmetic, the
+// blocks of a limb form one cluster that exchanges the strided stages through
+// distributed shared memory (GB300, 256 x 6 limbs, Harvey's butterflies, forward /
 // inverse GB/s: 2^13 1,435 / 1,400 against 1,223 / 1,211 in two passes and
-// about 1,141 single-pass; 2^14 1,370 / 1,343 against 1,318 / 1,286); at 2^15
-// (equal) and 2^16 (1,050 / 958 against 1,166 / 1,135) they run as a strided
-// pass plus blocks.
+// about 1,141 single-pass; 2^14 1,370 / 1,343 against 1,318 / 1,286); else at 2^15
+// and at 2^16 (1,050 / 958 against 1,166 / 1,135) they run as a strided pass plus
+// blocks.
 static std::atomic<uint32_t> g_ntt_block[17] = {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 12, 12, 12, 12};
 
 uint32_t ntt_block_logn(uint32_t logn) { return logn <= 16 ? g_ntt_block[logn].load(std::memory_order_relaxed) : 14; }
