@@ -58,7 +58,8 @@ struct StreamScratch {
   uint64_t* u64() const { return static_cast<uint64_t*>(ptr); }
 };
 
-// Host memory to the device; complete on return, for every stream.
+// Host memory to a new allocation on the device; complete on return, for every
+// stream. (It does not wait for earlier work on any.)
 void upload(void* dst, const void* src, size_t bytes);
 // Sets the message returned by fheg_last_error() on this thread.
 void set_last_error(const std::string& msg);

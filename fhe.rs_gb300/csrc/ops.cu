@@ -69,11 +69,27 @@ void set_ntt_block_logn(uint32_t logn, uint32_t block_logn) {
   g_ntt_block[logn].store(block_logn, std::memory_order_relaxed);
 }
 
+// The current device's stream for set-up work: waiting for it waits for that work
+// alone, not for what callers have queued on the default stream (never destroyed:
+// a context may outlive every static object).
+static cudaStream_t setup_stream() {
+  static std::mutex mu;
+  static auto* streams = new std::map<int, cudaStream_t>();
+  int dev = 0;
+  check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
+  std::lock_guard<std::mutex> lock(mu);
+  auto it = streams->find(dev);
+  if (it != streams->end()) return it->second;
+  cudaStream_t s = nullptr;
+  check_cuda(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "cudaStreamCreateWithFlags");
+  (*streams)[dev] = s;
+  return s;
+}
+
 void upload(void* dst, const void* src, size_t bytes) {
-  check_cuda(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice), "cudaMemcpy H2D");
-  // A copy from pageable memory may return with its last part on the way, and
-  // non-blocking streams do not wait for the default stream.
-  check_cuda(cudaStreamSynchronize(nullptr), "cudaStreamSynchronize");
+  const cudaStream_t s = setup_stream();
+  check_cuda(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync H2D");
+  check_cuda(cudaStreamSynchronize(s), "cudaStreamSynchronize");
 }
 
 // ---------------------------------------------------------------------------
@@ -218,12 +234,12 @@ std::shared_ptr<PrimeTables> get_prime_tables(uint64_t p, size_t n, uint64_t roo
   if (fold) {
     int4* ft = reinterpret_cast<int4*>(d + 4 * n);
     const uint64_t r32 = (1ull << 32) % p;
-    k_fold_tables<<<(unsigned)((2 * n + 255) / 256), 256>>>(dp.tw, ft, p, r32, shoup(r32, p), fc, fk,
-                                                            (uint32_t)n);
+    const cudaStream_t s = setup_stream();
+    k_fold_tables<<<(unsigned)((2 * n + 255) / 256), 256, 0, s>>>(dp.tw, ft, p, r32, shoup(r32, p), fc, fk,
+                                                                  (uint32_t)n);
     after_launch("k_fold_tables");
-    // Complete before the registry hands the tables out: a non-blocking stream
-    // (or another thread's) does not wait for this launch on the default one.
-    check_cuda(cudaStreamSynchronize(nullptr), "cudaStreamSynchronize");
+    // Complete before the registry hands the tables out: no other stream waits for it.
+    check_cuda(cudaStreamSynchronize(s), "cudaStreamSynchronize");
     dp.ftw = ft;
     dp.fitw = ft + n;
     dp.f_bias = fbias;
