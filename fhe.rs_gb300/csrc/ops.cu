@@ -92,6 +92,39 @@ void upload(void* dst, const void* src, size_t bytes) {
   check_cuda(cudaStreamSynchronize(s), "cudaStreamSynchronize");
 }
 
+namespace {
+// Pools by device, and the contexts that live there (never destroyed, as
+// setup_stream's streams).
+struct ScratchPools {
+  std::mutex mu;
+  std::map<int, cudaMemPool_t> pools;
+  std::map<int, int> contexts;
+};
+ScratchPools& scratch_pools() {
+  static auto* sp = new ScratchPools();
+  return *sp;
+}
+}  // namespace
+
+cudaMemPool_t scratch_pool() {
+  ScratchPools& sp = scratch_pools();
+  int dev = 0;
+  check_cuda(cudaGetDevice(&dev), "cudaGetDevice");
+  std::lock_guard<std::mutex> lock(sp.mu);
+  auto it = sp.pools.find(dev);
+  if (it != sp.pools.end()) return it->second;
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  cudaMemPool_t pool = nullptr;
+  check_cuda(cudaMemPoolCreate(&pool, &props), "cudaMemPoolCreate");
+  uint64_t keep = 128ull << 20;
+  check_cuda(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep), "cudaMemPoolSetAttribute");
+  sp.pools[dev] = pool;
+  return pool;
+}
+
 // ---------------------------------------------------------------------------
 // Prime table registry.
 
@@ -287,6 +320,17 @@ Context::Context(const std::vector<uint64_t>& m, size_t n, const uint64_t* roots
   }
   d_switch.alloc(sw.size() * 8);
   upload(d_switch.ptr, sw.data(), sw.size() * 8);
+  ScratchPools& sp = scratch_pools();
+  std::lock_guard<std::mutex> lock(sp.mu);
+  sp.contexts[device]++;
+}
+
+Context::~Context() {
+  ScratchPools& sp = scratch_pools();
+  std::lock_guard<std::mutex> lock(sp.mu);
+  if (--sp.contexts[device] > 0) return;
+  auto it = sp.pools.find(device);
+  if (it != sp.pools.end() && cudaMemPoolTrimTo(it->second, 0) != cudaSuccess) cudaGetLastError();
 }
 
 std::vector<uint64_t> Context::roots() const {

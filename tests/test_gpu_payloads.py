@@ -62,3 +62,45 @@ def test_payloads_at_any_alignment(fg, ora, cuda, logn, offset):
         assert np.array_equal(view.cpu().numpy(), want)
         assert not buf[:offset].any() and not buf[offset + count * size:].any()
         assert np.array_equal(fg.to_host(fg.deserialize(ctx, view, representation)), fg.to_host(t))
+
+
+def test_scratch_is_kept_bounded_and_given_back(fg, ora, cuda):
+    """Packing from Ntt takes scratch: calls that are waited for one by one keep at most 128 MB of it, threads with
+    streams of their own do not share it, and it goes back with the last context."""
+    import gc
+    import threading
+
+    torch, n = cuda, 1 << 14
+    gc.collect()
+    torch.cuda.synchronize()
+    ctx, moduli = _context(fg, ora, n, (62, 61, 59, 50))
+    q = np.array(moduli, dtype=np.uint64)[:, None]
+    x = np.random.default_rng(1).integers(0, 1 << 62, (8, 4, n), dtype=np.uint64) % q
+    want = _packed(x, moduli)
+    ntt = fg.to_device(x)
+    fg.ntt_forward(ctx, ntt)
+    torch.cuda.synchronize()
+    got = {}
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(20):
+                got[i] = fg.serialize(ctx, ntt, 1)
+            torch.cuda.current_stream().synchronize()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert all(np.array_equal(got[i].cpu().numpy(), want) for i in range(4))
+    big = ntt.repeat(64, 1, 1)  # 268 MB of scratch
+    fg.serialize(ctx, big, 1)
+    torch.cuda.synchronize()
+    del big
+    torch.cuda.empty_cache()
+    before = torch.cuda.mem_get_info()[0]
+    fg.serialize(ctx, ntt, 1)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    assert before - torch.cuda.mem_get_info()[0] <= 160 << 20
