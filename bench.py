@@ -64,18 +64,18 @@ STAGE_LAUNCHES = {"A": 1, "B": 1, "C": 1, "D": 1, "E": 1, "F": 2, "G": 1}
 # strided NTT stage applied inside the RNS scalers B and E; E's sums on the
 # tensor cores), from the ncu capture summarised in
 # profiles/stages_mul_relin_n16384_b64.md.
-STAGE_TRAFFIC_BYTES = {"A": 352.7e6, "B": 396.8e6, "C": 408.5e6, "D": 747.4e6, "E": 682.0e6, "F": 694.3e6,
+STAGE_TRAFFIC_BYTES = {"A": 352.6e6, "B": 397.2e6, "C": 408.5e6, "D": 746.9e6, "E": 682.3e6, "F": 694.1e6,
                        "G": 494.0e6}
 # The ncu figures above and below hold for the library sources they were
 # captured on: library_source_hash() of that tree. A run on other sources
 # reports null for them instead of stale numbers.
-PROFILED_SOURCE_HASH = "bcf5169b2dcd3cd9"
+PROFILED_SOURCE_HASH = "2a2a9b528f2d1400"
 # Share of the elapsed cycles in which the integer multipliers (the FMA-heavy
 # pipe, which executes every IMAD) were busy, per stage, from the same ncu
 # capture of one 64-pair multiplication (F: time-weighted over its two
 # launches); the whole multiplication, time-weighted.
-STAGE_FMAHEAVY_PCT = {"A": 68.5, "B": 61.1, "C": 71.4, "D": 68.5, "E": 59.0, "F": 70.5, "G": 64.6}
-MULTIPLY_FMAHEAVY_PCT = 66.3
+STAGE_FMAHEAVY_PCT = {"A": 68.6, "B": 60.8, "C": 71.0, "D": 68.4, "E": 58.9, "F": 70.4, "G": 64.5}
+MULTIPLY_FMAHEAVY_PCT = 66.2
 
 
 def library_source_hash() -> str:
